@@ -103,3 +103,36 @@ def test_rotations_need_fourteen_terms_at_half_width_1():
     ref = _chains([h1, h2], 64)
     r14 = _chains([h1, h2], 14)
     assert all(np.array_equal(r14[p][i], ref[p][i]) for p in (0, 1) for i in (0, 1))
+
+
+def _plain_chain(h, K):
+    """taylor_fixed: K terms, no stop."""
+    t, c, s = h, np.ones_like(h), h.copy()
+    for k in range(2, K + 1):
+        t = (t * h) * INV[k]
+        if k % 4 == 1:
+            s = s + t
+        elif k % 4 == 2:
+            c = c - t
+        elif k % 4 == 3:
+            s = s - t
+        else:
+            c = c + t
+    return c, s
+
+
+def test_chains_without_the_stop_have_the_reference_bits():
+    # terms past the 1e-18 stop are below half an ulp of both sums, also for
+    # the smallest half width a sweep admits and for lambda8's pair, whose
+    # reference stops on the larger of two terms
+    for a, K in ((0.3, 11), (0.3, 14), (1.0, 14), (1e-8, 11), (1e-3, 14)):
+        theta = _grid_thetas(a, 500_000, 7)
+        ref = _chains([0.5 * theta], 64)
+        c, s = _plain_chain(0.5 * theta, K)
+        assert np.array_equal(c, ref[0][0]) and np.array_equal(s, ref[1][0])
+        d1, d2 = (0.5 * INV_SQRT3) * theta, (-INV_SQRT3) * theta
+        sc = np.where(np.maximum(np.abs(d1), np.abs(d2)) > 0.5, 0.5, 1.0)
+        ref = _chains([d1 * sc, d2 * sc], 64)
+        for i, d in enumerate((d1, d2)):
+            c, s = _plain_chain(d * sc, K)
+            assert np.array_equal(c, ref[0][i]) and np.array_equal(s, ref[1][i])

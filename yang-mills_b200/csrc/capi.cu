@@ -516,9 +516,9 @@ int32_t ym_ensemble_create(const ym_ensemble_desc *desc, ym_ensemble **out) {
     if (err == cudaSuccess) err = dalloc(&e->d_error, 1);
     if (err == cudaSuccess) err = cudaMemset(e->d_error, 0, sizeof(unsigned));
     // plaquette shares of a measured sweep: three arrays of the 128-site
-    // layouts' CTA count (binary64 SU(3))
+    // layouts' warp count (binary64 SU(3))
     if (err == cudaSuccess && e->group == YM_GROUP_SU3 && e->precision == YM_PREC_F64)
-        err = dalloc(&e->d_tr_partial, 3 * (size_t)e->layouts[0].ctas);
+        err = dalloc(&e->d_tr_partial, 3 * ym::kSweepWarps * (size_t)e->layouts[0].ctas);
     if (err == cudaSuccess)
         err = cudaMemcpy(e->d_chains, e->chains.data(), e->chains.size() * sizeof(ChainInfo), cudaMemcpyHostToDevice);
     if (err == cudaSuccess && !half.empty())
@@ -801,7 +801,7 @@ static bool fused_plaquette(const ym_ensemble *e, int mode) {
 }
 
 // One sweep of the cadence (measure: sub-sweeps (1, mu), mu = 1..3, also
-// write their plaquette shares to d_tr_partial, one array of CTAs each).
+// write their plaquette shares to d_tr_partial, one array of warps each).
 static cudaError_t cadence_sweep(ym_ensemble *e, double angle, int mode, bool measure) {
     const int64_t ctas = e->layouts[e->sweep_layout].ctas;
     for (int parity = 0; parity < 2; ++parity)
@@ -809,7 +809,7 @@ static cudaError_t cadence_sweep(ym_ensemble *e, double angle, int mode, bool me
             cudaError_t err;
             if (f32(e)) err = ym::launch_f32_metropolis(e, parity, mu, angle, mode);
             else if (measure && parity == 1 && mu >= 1)
-                err = ym::launch_su3_metropolis_measure(e, mu, angle, e->d_tr_partial + (mu - 1) * ctas);
+                err = ym::launch_su3_metropolis_measure(e, mu, angle, e->d_tr_partial + (mu - 1) * ctas * ym::kSweepWarps);
             else err = ym::launch_su3_metropolis(e, parity, mu, angle, mode);
             if (err != cudaSuccess) return err;
         }

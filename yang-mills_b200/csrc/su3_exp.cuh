@@ -23,6 +23,9 @@ static __constant__ double c_inv[68] = {
     YM_INV4(44), YM_INV4(48), YM_INV4(52), YM_INV4(56), YM_INV4(60), YM_INV4(64)};
 #undef YM_INV4
 
+// fl(1/k) as a compile-time constant (c_inv's entries).
+__host__ __device__ constexpr double inv_int(int k) { return 1.0 / k; }
+
 constexpr double kTermCutoff = 1.0e-18;           // EXP_TERM_CUTOFF su3.rs:25
 constexpr double kInvSqrt3 = 0.5773502691896258;  // su3.rs:22
 

@@ -90,16 +90,16 @@ __device__ __forceinline__ double site_plaquette_sum_staged(const double2 *links
 
 // One 1024-thread block per chain: the plaquette shares the last three
 // sub-sweeps of a sweep wrote for the chain's CTAs (planes (0,1); (0,2),
-// (1,2); (0,3), (1,3), (2,3)), summed CTA by CTA in a fixed order, then the
+// (1,2); (0,3), (1,3), (2,3)), summed warp by warp in a fixed order, then the
 // average plaquette sum / (6 V).
-__global__ void k_chain_reduce_sweep(const double *__restrict__ tr_partial, int64_t ctas,
+__global__ void k_chain_reduce_sweep(const double *__restrict__ tr_partial, int64_t warps,
                                      const int32_t *__restrict__ cta_range, const ChainInfo *__restrict__ chains,
                                      double *__restrict__ out) {
     const int chain = blockIdx.x;
-    const int b = cta_range[2 * chain], e = cta_range[2 * chain + 1];
+    const int b = cta_range[2 * chain] * kSweepWarps, e = cta_range[2 * chain + 1] * kSweepWarps;
     double v = 0.0;
     for (int i = b + threadIdx.x; i < e; i += blockDim.x) {
-        const double p = (tr_partial[i] + tr_partial[ctas + i]) + tr_partial[2 * ctas + i];
+        const double p = (tr_partial[i] + tr_partial[warps + i]) + tr_partial[2 * warps + i];
         v = (i == b + (int)threadIdx.x) ? p : v + p;
     }
     v = block_reduce<false>(v);
@@ -451,7 +451,7 @@ cudaError_t launch_su3_plaquette(ym_ensemble *e) {
 cudaError_t launch_su3_plaquette_from_sweep(ym_ensemble *e, const double *tr_partial) {
     const SweepLayout &L = e->layouts[e->sweep_layout];
     if (!L.d_chain_ctas) return cudaErrorInvalidValue;
-    k_chain_reduce_sweep<<<(unsigned)e->n_chains, 1024, 0, e->stream>>>(tr_partial, L.ctas, L.d_chain_ctas,
+    k_chain_reduce_sweep<<<(unsigned)e->n_chains, 1024, 0, e->stream>>>(tr_partial, L.ctas * kSweepWarps, L.d_chain_ctas,
                                                                          e->d_chains, e->d_result);
     return cudaGetLastError();
 }

@@ -23,8 +23,8 @@
 //
 // Layout: every factor of the six staple terms is copied global -> shared by
 // cp.async ahead of its use.  Ordered hits (k_su3_metropolis_ring) keep the
-// staple accumulator in registers and stage two terms ahead, two 128-thread
-// blocks per SM; drawn generators (k_su3_metropolis) keep it in shared
+// staple accumulator in registers and stage two terms ahead, two persistent
+// 128-thread blocks per SM; drawn generators (k_su3_metropolis) keep it in shared
 // memory (nine double2 per thread, conflict-free column layout) and stage
 // one term ahead, three blocks per SM.
 #pragma once
@@ -410,71 +410,78 @@ __device__ __forceinline__ unsigned visit(m3 &u, const double2 (*sa)[T], double 
 
 // ---- the reference's ordered hits, software-pipelined ---------------------
 // A hit has a link-independent half (its two stream words, the angle, the
-// rotation entries from the Taylor chain, the uniform) and a link-dependent
-// half (candidate rows, Re Tr against the staple, the decision).  visit()
-// runs them back to back, and the Taylor chain's early exits split the code
-// into many small blocks; here every hit's link-independent half is computed
-// while the previous hit's link-dependent half runs, both branch-free in one
-// straight-line block, so each link carries two independent dependency
+// rotation entries from the Taylor chain, the accept threshold) and a
+// link-dependent half (candidate rows, Re Tr against the staple, the
+// decision).  visit() runs them back to back, and the Taylor chain's early
+// exits split the code into many small blocks; here every hit's
+// link-independent half is computed next to the previous hit's
+// link-dependent half, so each link carries two independent dependency
 // chains instead of one.  The values are visit()'s, bit for bit:
-//   * taylor_fixed<K> evaluates K terms of taylor_chain's recurrence and adds
-//     term k only while no earlier term was at or below the 1e-18 cutoff.
-//     K is taken from the proposal half width a so that every admissible
-//     angle stops within K terms: |t_k| <= |h|^k / k! with |h| <= a/2 for
-//     generators 1..7 and |h| <= 0.5774 a (at most 0.5 after lambda8's
-//     halving) for generator 8.  Terms the reference still adds past K
-//     must be too small to move their sum (below half an ulp of it): for
-//     a <= 0.3, K = 11 (t_12 <= 0.1732^12/12! = 1.5e-18 against sums near
-//     0.985, t_13 / s <= 0.1732^12/13! = 1.2e-19); for a <= 1, K = 14
-//     (t_15 / s <= 0.5^14/15! = 4.7e-17 < 2^-54, t_16 <= 7.3e-19), so the
-//     sums are the reference's bit for bit (checked on the CPU against
-//     the loop run to the cutoff over millions of grid angles).
-//   * the decision is accept_step's u < exp(-max(dS, 0)) (for m = 0,
-//     exp(-0) = 1 > u, as its explicit branch gives); the accepted rows are
-//     selected, not branched to.
+//   * taylor_fixed<K> adds K terms of taylor_chain's recurrence, without its
+//     1e-18 stop.  A term past the stop is below 1e-18 |h| / 2, less than
+//     half an ulp of both sums (c >= 0.87; s >= 0.95 |h|), so adding it
+//     changes no bit, and leaving the test out saves a comparison and a
+//     select per term.  K is taken from the proposal half width a: |t_k| <=
+//     |h|^k / k! with |h| <= a/2 for generators 1..7 and |h| <= 0.5774 a (at
+//     most 0.5 after lambda8's halving) for generator 8, and terms past K
+//     must be below half an ulp too: for a <= 0.3, K = 11 (t_12 <=
+//     0.1732^12/12! = 1.5e-18 against sums near 0.985, t_13 / s <=
+//     0.1732^12/13! = 1.2e-19); for a <= 1, K = 14 (t_15 / s <= 0.5^14/15!
+//     = 4.7e-17 < 2^-54, t_16 <= 7.3e-19), so the sums are the reference's
+//     bit for bit (checked on the CPU against the loop run to the cutoff
+//     over millions of grid angles).
+//   * the decision is accept_step's u < exp(-max(dS, 0)) through accept_log;
+//     the accepted rows are selected, not branched to.
 template <int K>
 __device__ __forceinline__ void taylor_fixed(double h, double &c, double &s) {
-    double t = 1.0;
+    double t = h;      // k = 1: t = (1 h) 1, s = 0 + t
     c = 1.0;
-    s = 0.0;
-    bool done = false;
+    s = h;
 #pragma unroll
-    for (int k = 1; k <= K; ++k) {
-        t = (t * h) * c_inv[k];
-        if ((k & 3) == 1) { const double v = s + t; s = done ? s : v; }
-        else if ((k & 3) == 2) { const double v = c - t; c = done ? c : v; }
-        else if ((k & 3) == 3) { const double v = s - t; s = done ? s : v; }
-        else { const double v = c + t; c = done ? c : v; }
-        done = done || fabs(t) <= kTermCutoff;
+    for (int k = 2; k <= K; ++k) {
+        t = (t * h) * inv_int(k);
+        if ((k & 3) == 1) s = s + t;
+        else if ((k & 3) == 2) c = c - t;
+        else if ((k & 3) == 3) s = s - t;
+        else c = c + t;
     }
 }
 
-// lambda8_rotation with taylor_chain2's lockstep chains (stopping on the
-// larger term) evaluated for K terms; |theta| <= 1 needs at most one halving.
+// lambda8_rotation with taylor_chain2's two chains evaluated for K terms;
+// |theta| <= 1 needs at most one halving.
 template <int K>
 __device__ __forceinline__ void lambda8_fixed(double theta, cplx &e1, cplx &e2) {
     const double d1 = (0.5 * kInvSqrt3) * theta;
     const double d2 = (-kInvSqrt3) * theta;
     const bool sq = fmax(fabs(d1), fabs(d2)) > 0.5;
     const double sc = sq ? 0.5 : 1.0;
-    const double h1 = d1 * sc, h2 = d2 * sc;
-    double t1 = 1.0, t2 = 1.0, c1 = 1.0, s1 = 0.0, c2 = 1.0, s2 = 0.0;
-    bool done = false;
-#pragma unroll
-    for (int k = 1; k <= K; ++k) {
-        t1 = (t1 * h1) * c_inv[k];
-        t2 = (t2 * h2) * c_inv[k];
-        if ((k & 3) == 1) { const double a = s1 + t1, b = s2 + t2; s1 = done ? s1 : a; s2 = done ? s2 : b; }
-        else if ((k & 3) == 2) { const double a = c1 - t1, b = c2 - t2; c1 = done ? c1 : a; c2 = done ? c2 : b; }
-        else if ((k & 3) == 3) { const double a = s1 - t1, b = s2 - t2; s1 = done ? s1 : a; s2 = done ? s2 : b; }
-        else { const double a = c1 + t1, b = c2 + t2; c1 = done ? c1 : a; c2 = done ? c2 : b; }
-        done = done || fmax(fabs(t1), fabs(t2)) <= kTermCutoff;
-    }
-    e1 = cmake(c1, s1);
-    e2 = cmake(c2, s2);
+    taylor_fixed<K>(d1 * sc, e1.re, e1.im);
+    taylor_fixed<K>(d2 * sc, e2.re, e2.im);
     const cplx q1 = cmul(e1, e1), q2 = cmul(e2, e2);
     e1 = sq ? q1 : e1;
     e2 = sq ? q2 : e2;
+}
+
+// The decision u < exp(-m), m = max(dS, 0), taken as m < -log u in binary32
+// away from equality.  neg_log_unit's error: the word's 32 high bits give u
+// to 2^-32, so log u to 2^-16 = 1.53e-5 for u >= 2^-16 (smaller u, one in
+// 65,536, return NaN: never sure); __logf adds at most 3.6e-7 on [0.5, 2] and
+// 3 ulp, 2.9e-6, down to log 2^-16 = -11.1; rounding m to binary32 7e-7.
+// Together below kLogBand, so every decision outside the band is
+// accept_step's; one inside (one in a few thousand) evaluates that test.
+constexpr float kLogBand = 2.5e-5f;
+
+__device__ __forceinline__ float neg_log_unit(uint64_t w) {
+    const uint32_t hi = (uint32_t)(w >> 32);
+    const float l = -__logf((float)hi * 0x1p-32f);
+    return hi < 65536u ? __int_as_float(0x7fffffff) : l;
+}
+
+__device__ __forceinline__ bool accept_log(double ds, float logu, uint64_t key, int h) {
+    const float d = fmaxf((float)ds, 0.0f) - logu;
+    bool acc = d < 0.0f;
+    if (!(fabsf(d) > kLogBand)) acc = unit_from(splitmix_at(key, (uint64_t)(2 * h + 1))) < exp(-fmax(ds, 0.0));
+    return acc;
 }
 
 // Rotation entries of a hit: the reference's bits (taylor_fixed,
@@ -503,39 +510,47 @@ __device__ __forceinline__ void diag_rotation(double theta, cplx &e1, cplx &e2) 
 }
 
 struct BlockPre {
-    double c, s, unif;
+    double c, s;
+    float logu;        // neg_log_unit of the accept word
 };
 struct DiagPre {
     cplx e1, e2;
-    double unif;
+    float logu;
 };
 
+// The stream's next word (state starts at the link's key).
+__device__ __forceinline__ uint64_t next_word(uint64_t &state) { return mix64(state += kGolden); }
+
 template <int K>
-__device__ __forceinline__ BlockPre pre_block(uint64_t key, int h, double angle) {
+__device__ __forceinline__ BlockPre pre_block(uint64_t &state, double angle) {
     BlockPre p;
-    block_rotation<K>(0.5 * grid_angle(splitmix_at(key, (uint64_t)(2 * h)), angle), p.c, p.s);
-    p.unif = unit_from(splitmix_at(key, (uint64_t)(2 * h + 1)));
+    block_rotation<K>(0.5 * grid_angle(next_word(state), angle), p.c, p.s);
+    p.logu = neg_log_unit(next_word(state));
     return p;
 }
 
 template <int K>
-__device__ __forceinline__ DiagPre pre_diag(uint64_t key, int h, double angle) {
+__device__ __forceinline__ DiagPre pre_diag(uint64_t &state, double angle) {
     DiagPre p;
-    diag_rotation<K>(grid_angle(splitmix_at(key, (uint64_t)(2 * h)), angle), p.e1, p.e2);
-    p.unif = unit_from(splitmix_at(key, (uint64_t)(2 * h + 1)));
+    diag_rotation<K>(grid_angle(next_word(state), angle), p.e1, p.e2);
+    p.logu = neg_log_unit(next_word(state));
     return p;
 }
 
-// hit_block for a compile-time generator, decision by selects.
-template <int I0, int I1, int KIND>
-__device__ __forceinline__ void hit_block_sel(m3 &u, const double2 (*sa)[T], double rr[3], double &old_tr,
-                                              const BlockPre &p, double beta3, unsigned &accepted) {
-    const double c = p.c, s = p.s;
-    cplx n0[3], n1[3];
+// One row of a link and its Re Tr share.
+struct Row {
+    cplx e[3];
+    double rr;
+};
+
+// Candidate entries of an SU(2)-subgroup hit on rows x, y (hit_block's).
+template <int KIND>
+__device__ __forceinline__ void block_candidate(const Row &x, const Row &y, double c, double s, cplx n0[3],
+                                                cplx n1[3]) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const double x0 = u.e[I0][k].re, y0 = u.e[I0][k].im;
-        const double x1 = u.e[I1][k].re, y1 = u.e[I1][k].im;
+        const double x0 = x.e[k].re, y0 = x.e[k].im;
+        const double x1 = y.e[k].re, y1 = y.e[k].im;
         if (KIND == 0) {
             n0[k] = cmake(c * x0 - s * y1, c * y0 + s * x1);
             n1[k] = cmake(c * x1 - s * y0, s * x0 + c * y1);
@@ -547,83 +562,107 @@ __device__ __forceinline__ void hit_block_sel(m3 &u, const double2 (*sa)[T], dou
             n1[k] = cmake(c * x1 + s * y1, c * y1 - s * x1);
         }
     }
-    cplx col0[3], col1[3];
-    sa_col(sa, I0, col0);
-    sa_col(sa, I1, col1);
-    double q[3] = {rr[0], rr[1], rr[2]};
-    q[I0] = retr_row_fma(n0, col0);
-    q[I1] = retr_row_fma(n1, col1);
-    const double new_tr = (q[0] + q[1]) + q[2];
-    const double m = fmax(beta3 * (old_tr - new_tr), 0.0);
-    const bool acc = p.unif < exp(-m);
+}
+
+__device__ __forceinline__ void take_row(Row &r, bool acc, const cplx n[3], double q) {
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        u.e[I0][k] = acc ? n0[k] : u.e[I0][k];
-        u.e[I1][k] = acc ? n1[k] : u.e[I1][k];
-    }
-    rr[I0] = acc ? q[I0] : rr[I0];
-    rr[I1] = acc ? q[I1] : rr[I1];
+    for (int k = 0; k < 3; ++k) r.e[k] = acc ? n[k] : r.e[k];
+    r.rr = acc ? q : r.rr;
+}
+
+// An SU(2)-subgroup hit on rows x and y, whose A columns are ca and cb; z is
+// the third row.  first: the subgroup is (0, 1), so the trace sums as
+// (x + y) + z; else z lies between or before them: (x + z) + y.
+template <int KIND>
+__device__ __forceinline__ void hit_rows(Row &x, Row &y, const Row &z, const double2 (*ca)[T],
+                                         const double2 (*cb)[T], bool first, double &old_tr, const BlockPre &p,
+                                         double beta3, unsigned &accepted, uint64_t key, int h) {
+    cplx n0[3], n1[3], col[3];
+    block_candidate<KIND>(x, y, p.c, p.s, n0, n1);
+    sa_col(ca, 0, col);
+    const double q0 = retr_row_fma(n0, col);
+    sa_col(cb, 0, col);
+    const double q1 = retr_row_fma(n1, col);
+    const double mid = first ? q1 : z.rr, end = first ? z.rr : q1;
+    const double new_tr = (q0 + mid) + end;
+    const bool acc = accept_log(beta3 * (old_tr - new_tr), p.logu, key, h);
+    take_row(x, acc, n0, q0);
+    take_row(y, acc, n1, q1);
     old_tr = acc ? new_tr : old_tr;
     accepted += acc ? 1u : 0u;
 }
 
-__device__ __forceinline__ void hit_diag_sel(m3 &u, const double2 (*sa)[T], double rr[3], double &old_tr,
-                                             const DiagPre &p, double beta3, unsigned &accepted) {
-    cplx n[3][3];
-    double q[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const cplx e = i < 2 ? p.e1 : p.e2;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) n[i][k] = cmul(e, u.e[i][k]);
-        cplx col[3];
-        sa_col(sa, i, col);
-        q[i] = retr_row_fma(n[i], col);
-    }
-    const double new_tr = (q[0] + q[1]) + q[2];
-    const double m = fmax(beta3 * (old_tr - new_tr), 0.0);
-    const bool acc = p.unif < exp(-m);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) u.e[i][k] = acc ? n[i][k] : u.e[i][k];
-        rr[i] = acc ? q[i] : rr[i];
-    }
-    old_tr = acc ? new_tr : old_tr;
-    accepted += acc ? 1u : 0u;
+__device__ __forceinline__ void swap_rows(Row &x, Row &y) {
+    const Row t = x;
+    x = y;
+    y = t;
 }
 
-// The eight ordered hits (generators 1..8, su3_ensemble.rs:361): hit h+1's
-// link-independent half is written next to hit h.
+// The eight ordered hits (generators 1..8, su3_ensemble.rs:361) in a loop
+// over the three SU(2) subgroups (rows (0,1), (0,2), (1,2)): the rows trade
+// places between its passes, so one copy of the code serves all three.  Hit
+// h+1's link-independent half is written next to hit h.
 // tr receives Re Tr(U' A) of the final link, the sum of its six plaquettes.
 template <int K>
 __device__ __forceinline__ unsigned visit_ordered(m3 &u, const double2 (*sa)[T], double beta3,
                                                   double angle, uint64_t key, double &tr) {
-    double rr[3];
+    Row r[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         cplx col[3];
         sa_col(sa, i, col);
-        rr[i] = retr_row_fma(u.e[i], col);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) r[i].e[k] = u.e[i][k];
+        r[i].rr = retr_row_fma(u.e[i], col);
     }
-    double old_tr = (rr[0] + rr[1]) + rr[2];
+    double old_tr = (r[0].rr + r[1].rr) + r[2].rr;
     unsigned accepted = 0;
-    const BlockPre p0 = pre_block<K>(key, 0, angle);
-    const BlockPre p1 = pre_block<K>(key, 1, angle);
-    hit_block_sel<0, 1, 0>(u, sa, rr, old_tr, p0, beta3, accepted);
-    const BlockPre p2 = pre_block<K>(key, 2, angle);
-    hit_block_sel<0, 1, 1>(u, sa, rr, old_tr, p1, beta3, accepted);
-    const BlockPre p3 = pre_block<K>(key, 3, angle);
-    hit_block_sel<0, 1, 2>(u, sa, rr, old_tr, p2, beta3, accepted);
-    const BlockPre p4 = pre_block<K>(key, 4, angle);
-    hit_block_sel<0, 2, 0>(u, sa, rr, old_tr, p3, beta3, accepted);
-    const BlockPre p5 = pre_block<K>(key, 5, angle);
-    hit_block_sel<0, 2, 1>(u, sa, rr, old_tr, p4, beta3, accepted);
-    const BlockPre p6 = pre_block<K>(key, 6, angle);
-    hit_block_sel<1, 2, 0>(u, sa, rr, old_tr, p5, beta3, accepted);
-    const DiagPre p7 = pre_diag<K>(key, 7, angle);
-    hit_block_sel<1, 2, 1>(u, sa, rr, old_tr, p6, beta3, accepted);
-    hit_diag_sel(u, sa, rr, old_tr, p7, beta3, accepted);
+    Row x = r[0], y = r[1], z = r[2];
+    uint64_t state = key;
+    BlockPre p = pre_block<K>(state, angle);
+#pragma unroll 1
+    for (int it = 0; it < 3; ++it) {
+        const double2 (*ca)[T] = sa + (it == 2 ? 1 : 0);
+        const double2 (*cb)[T] = sa + (it == 0 ? 1 : 2);
+        const int h0 = it == 0 ? 0 : 2 * it + 1;   // the pass's first hit
+        BlockPre q = pre_block<K>(state, angle);
+        hit_rows<0>(x, y, z, ca, cb, it == 0, old_tr, p, beta3, accepted, key, h0);
+        if (it < 2) p = pre_block<K>(state, angle);
+        hit_rows<1>(x, y, z, ca, cb, it == 0, old_tr, q, beta3, accepted, key, h0 + 1);
+        if (it == 0) {
+            q = pre_block<K>(state, angle);
+            hit_rows<2>(x, y, z, ca, cb, true, old_tr, p, beta3, accepted, key, 2);
+            p = q;
+            swap_rows(y, z);
+        } else if (it == 1) {
+            swap_rows(x, z);
+        }
+    }
+    // now x is row 1, y row 2, z row 0
+    const DiagPre d = pre_diag<K>(state, angle);
+    cplx n0[3], n1[3], n2[3], col[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        n0[k] = cmul(d.e1, z.e[k]);
+        n1[k] = cmul(d.e1, x.e[k]);
+        n2[k] = cmul(d.e2, y.e[k]);
+    }
+    sa_col(sa, 0, col);
+    const double q0 = retr_row_fma(n0, col);
+    sa_col(sa, 1, col);
+    const double q1 = retr_row_fma(n1, col);
+    sa_col(sa, 2, col);
+    const double q2 = retr_row_fma(n2, col);
+    const double new_tr = (q0 + q1) + q2;
+    const bool acc = accept_log(beta3 * (old_tr - new_tr), d.logu, key, 7);
+    old_tr = acc ? new_tr : old_tr;
+    accepted += acc ? 1u : 0u;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        u.e[0][k] = acc ? n0[k] : z.e[k];
+        u.e[1][k] = acc ? n1[k] : x.e[k];
+        u.e[2][k] = acc ? n2[k] : y.e[k];
+    }
     tr = old_tr;
     return accepted;
 }
@@ -675,24 +714,81 @@ k_su3_metropolis(const ChainInfo *__restrict__ chains, const Tile *__restrict__ 
 // 128-thread CTAs per SM fit (registers and 108 KB of staging each); after
 // the staple the accumulator is written once to the second set's memory for
 // the hits.  The products and their order are staple_pipelined's, so A has
-// the same bits.  On a 32^4 lattice this is 1.4 % faster than the
-// three-CTA form with the ordered visit, and 20 % slower with the drawn
-// generators' visit, whose loop-carried hits need the third CTA's warps.
+// the same bits.
+//
+// What bounds it: latency, at two warps per scheduler.  Two things cut it.
+// (1) The CTAs are persistent, and the next item's first term loads into the
+// first set while this item's hits run, so no item starts on an empty
+// pipeline (chain table, then links: three dependent trips to L2).  (2) The
+// code is small: directions and subgroups are loops, not copies.  Unrolled
+// (66 KB, four directions of it) the warps, which drift apart once they are
+// persistent, waited for instructions as long as for data.  Per issued
+// instruction on a 32^4 lattice, half width 0.3: unrolled and one tile per
+// CTA 1.57 cycles on loads + 0.40 on instruction fetch (168 us per launch
+// under the profiler), persistent unrolled 0.85-1.13 + 0.52-0.91 (169 us),
+// persistent loops 0.76 + 0.12 (161 us; 10 % more integer instructions).
+// Three CTAs per SM (one term ahead, 168 registers with 150 bytes spilled):
+// 1.52 + 0.62, 180 us.  Sweep of 32^4 live, same box: 1438 -> 1300 us at
+// half width 0.3, 1439 -> 1289 us at 0.35 (of which the shorter rotations
+// and accept_log 6 %); 8^4 94 -> 73 us, 16^4 102 -> 97 us.
 struct TermSet {
     double2 (*f[3])[T];
 };
 
-template <int MU, int NU>
-__device__ __forceinline__ void stage_term3(const TermSet &b, const double2 *links, const ChainInfo &c,
-                                            const TermSites &t) {
-    const double2 *p1 = links + c.offset + (int64_t)(NU * 9) * c.volume + t.s1;
-    const double2 *p2 = links + c.offset + (int64_t)(MU * 9) * c.volume + t.s2;
-    const double2 *p3 = links + c.offset + (int64_t)(NU * 9) * c.volume + t.s3;
+// A link's site within its chain and the steps to its neighbours, in
+// lexicographic positions.  Sweeps need even extents, so every step changes
+// the parity; 32 bits hold any site (a lattice of 2^31 sites takes 1.2 TB).
+struct Site {
+    int32_t lex, half;
+    int32_t fwd[4], bwd[4];
+};
+
+__device__ __forceinline__ Site site_of(const ChainInfo &c, const Coord &x) {
+    Site k;
+    k.lex = (int32_t)x.lex;
+    k.half = (int32_t)c.half;
+    int32_t st = 1;
+#pragma unroll
+    for (int d = 3; d >= 0; --d) {
+        const int32_t span = c.n[d] * st;
+        k.fwd[d] = x.x[d] == c.n[d] - 1 ? st - span : st;
+        k.bwd[d] = x.x[d] == 0 ? span - st : -st;
+        st = span;
+    }
+    return k;
+}
+
+__device__ __forceinline__ int32_t pick(const int32_t *v, int d) {
+    return d == 0 ? v[0] : (d == 1 ? v[1] : (d == 2 ? v[2] : v[3]));
+}
+
+// The three factors of staple term (nu, BWD) of link (x, mu):
+//   forward  U_nu(x+mu), U_mu(x+nu), U_nu(x)
+//   backward U_nu(x-nu+mu), U_mu(x-nu), U_nu(x-nu)
+// mu and nu are run-time values (uniform over the launch), so one copy of
+// the code serves every direction.
+template <bool BWD>
+__device__ __forceinline__ void stage_term3(const TermSet &b, const double2 *base, int64_t v, const Site &x, int par,
+                                            int mu, int nu) {
+    const int32_t same = par ? x.half : 0, other = par ? 0 : x.half;
+    const int32_t up = pick(x.fwd, mu);
+    int32_t i1, i2, i3;
+    if (!BWD) {
+        i1 = other + ((x.lex + up) >> 1);
+        i2 = other + ((x.lex + pick(x.fwd, nu)) >> 1);
+        i3 = same + (x.lex >> 1);
+    } else {
+        const int32_t o = x.lex + pick(x.bwd, nu);
+        i1 = same + ((o + up) >> 1);
+        i2 = i3 = other + (o >> 1);
+    }
+    const double2 *pn = base + (int64_t)(nu * 9) * v, *pm = base + (int64_t)(mu * 9) * v;
+    const double2 *p1 = pn + i1, *p2 = pm + i2, *p3 = pn + i3;
 #pragma unroll
     for (int e = 0; e < 9; ++e) {
-        cp_async16(&b.f[0][e][threadIdx.x], p1 + (int64_t)e * c.volume);
-        cp_async16(&b.f[1][e][threadIdx.x], p2 + (int64_t)e * c.volume);
-        cp_async16(&b.f[2][e][threadIdx.x], p3 + (int64_t)e * c.volume);
+        cp_async16(&b.f[0][e][threadIdx.x], p1 + (int64_t)e * v);
+        cp_async16(&b.f[1][e][threadIdx.x], p2 + (int64_t)e * v);
+        cp_async16(&b.f[2][e][threadIdx.x], p3 + (int64_t)e * v);
     }
     cp_async_commit();
 }
@@ -727,103 +823,130 @@ __device__ __forceinline__ void term_accumulate(const TermSet &b, m3 &a) {
             }
 }
 
-// SAVE = 2 or 4: a_part receives the accumulator after the first SAVE terms
-// (the terms of the first one or two directions other than MU).
-template <int MU, int SAVE = 0>
-__device__ __forceinline__ m3 staple_ring(const double2 *links, const ChainInfo &c, const Coord &x, int par,
-                                          const Nb &pm, const TermSet &s0, const TermSet &s1, int64_t s_self,
-                                          m3 *a_part = nullptr) {
-    constexpr int N0 = Nu<MU, 0>::v, N1 = Nu<MU, 1>::v, N2 = Nu<MU, 2>::v;
-    stage_term3<MU, N0>(s0, links, c, term_sites<MU, N0, false>(c, x, par, pm));
-    stage_term3<MU, N0>(s1, links, c, term_sites<MU, N0, true>(c, x, par, pm));
+// The staple of link (x, mu); term 0 has been staged into s0.  SAVE (mu = 1
+// or 2): `part` receives the accumulator after the directions below mu.
+template <bool SAVE>
+__device__ __forceinline__ m3 staple_ring(const double2 *base, int64_t v, const Site &x, int par, int mu,
+                                          const TermSet &s0, const TermSet &s1, m3 &part) {
     m3 a;
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
         for (int k = 0; k < 3; ++k) a.e[r][k] = cmake(0.0, 0.0);
-    cp_async_wait_one();
-    term_accumulate<false>(s0, a);
-    stage_term3<MU, N1>(s0, links, c, term_sites<MU, N1, false>(c, x, par, pm));
-    cp_async_wait_one();
-    term_accumulate<true>(s1, a);
-    if (SAVE == 2) *a_part = a;
-    stage_term3<MU, N1>(s1, links, c, term_sites<MU, N1, true>(c, x, par, pm));
-    cp_async_wait_one();
-    term_accumulate<false>(s0, a);
-    stage_term3<MU, N2>(s0, links, c, term_sites<MU, N2, false>(c, x, par, pm));
-    cp_async_wait_one();
-    term_accumulate<true>(s1, a);
-    if (SAVE == 4) *a_part = a;
-    stage_term3<MU, N2>(s1, links, c, term_sites<MU, N2, true>(c, x, par, pm));
-    cp_async_wait_one();
-    term_accumulate<false>(s0, a);
-    stage_link(s0.f[0], links, c, s_self, MU);   // the updated link itself
-    cp_async_wait_one();
-    term_accumulate<true>(s1, a);
+#pragma unroll 1
+    for (int i = 0; i < 3; ++i) {
+        const int nu = i + (i >= mu ? 1 : 0), nn = i + 1 + (i + 1 >= mu ? 1 : 0);
+        stage_term3<true>(s1, base, v, x, par, mu, nu);
+        cp_async_wait_one();
+        term_accumulate<false>(s0, a);
+        if (i < 2) {
+            stage_term3<false>(s0, base, v, x, par, mu, nn);
+        } else {   // the updated link itself
+            const double2 *p = base + (int64_t)(mu * 9) * v + (par ? x.half : 0) + (x.lex >> 1);
+#pragma unroll
+            for (int e = 0; e < 9; ++e) cp_async16(&s0.f[0][e][threadIdx.x], p + (int64_t)e * v);
+            cp_async_commit();
+        }
+        cp_async_wait_one();
+        term_accumulate<true>(s1, a);
+        if (SAVE && i + 1 == mu) part = a;
+    }
     return a;
 }
 
 constexpr int kRingBuffers = 6;   // two sets of three factors
 
 // MEASURE (parity 1, MU = 1, 2 or 3: the last three sub-sweeps of a sweep,
-// one chain per CTA): each CTA also writes tr_partial[cta], the sum over its
-// links of (1/3) Re Tr(U' A_p) with A_p the staple terms of the directions
+// one chain per CTA): each warp also writes its slot of tr_partial (work
+// item b, warp w: b * kSweepWarps + w), the sum over its links of (1/3) Re Tr(U' A_p) with A_p the staple terms of the directions
 // nu < MU (MU = 1: nu = 0; MU = 2: nu = 0, 1; MU = 3: all of A).  Once this
 // sub-sweep has run, every link of those terms is final (directions below
 // MU are done, direction MU's even links were done in parity 0, its odd
 // links here), and each plaquette of plane (nu, MU) holds exactly one
 // odd-site MU-link, so the three launches' sums are the plaquettes of
 // planes (0,1); (0,2), (1,2); (0,3), (1,3), (2,3): all six planes.
-template <int MU, int K, bool MEASURE = false>
+template <int K, bool MEASURE>
 __global__ void __launch_bounds__(T, 2)
-k_su3_metropolis_ring(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles,
-                      double2 *__restrict__ links, int parity, double angle,
+k_su3_metropolis_ring(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles, int n_ctas,
+                      double2 *__restrict__ links, int parity, int mu, double angle,
                       const uint64_t *__restrict__ sweep_ptr, unsigned long long *__restrict__ accepts,
                       int log2_item, int reverse, double *__restrict__ tr_partial = nullptr) {
     extern __shared__ __align__(16) double2 ring_mem[];
     auto buf = [&](int i) { return reinterpret_cast<double2 (*)[T]>(ring_mem + (size_t)i * 9 * T); };
     const TermSet s0{{buf(0), buf(1), buf(2)}}, s1{{buf(3), buf(4), buf(5)}};
-    const int64_t cta = reverse ? (int64_t)gridDim.x - 1 - blockIdx.x : (int64_t)blockIdx.x;
-    const Tile tile = tiles[cta * (T >> log2_item) + (threadIdx.x >> log2_item)];
-    const bool live = tile.chain >= 0;
-    const ChainInfo c = chains[live ? tile.chain : 0];
-    const int64_t t = tile.start + (threadIdx.x & ((1u << log2_item) - 1u));
+    auto tile_of = [&](int b) {
+        return tiles[(int64_t)(reverse ? n_ctas - 1 - b : b) * (T >> log2_item) + (threadIdx.x >> log2_item)];
+    };
+    const int64_t lane = threadIdx.x & ((1u << log2_item) - 1u);
     const uint64_t sweep = *sweep_ptr;
-    unsigned accepted = 0;
-    double tr = 0.0;
-    if (live && t < c.half) {
-        const int64_t s = (int64_t)parity * c.half + t;
-        const Coord x = decode_storage(c, s);
-        const Nb pm = step(c, x.x, x.lex, parity, MU, +1);
-        constexpr int kSave = (MEASURE && MU == 1) ? 2 : ((MEASURE && MU == 2) ? 4 : 0);
-        m3 a_part;
-        const m3 a = staple_ring<MU, kSave>(links, c, x, parity, pm, s0, s1, s, &a_part);
-        cp_async_wait_all();
-        m3 u = staged_link(s0.f[0]);
-        // the accumulator, for the hits, in the second set's (now free) memory
+    int32_t chain;        // of the item in hand
+    bool live;
+    Site x;
+    const double2 *base;  // the chain's links
+    int64_t volume;
+    double beta;
+    uint64_t seed;
+    auto take_item = [&](int b) {
+        const Tile tile = tile_of(b);
+        const ChainInfo c = chains[tile.chain >= 0 ? tile.chain : 0];
+        chain = tile.chain;
+        live = tile.chain >= 0 && tile.start + lane < c.half;
+        x = site_of(c, decode_storage(c, (int64_t)parity * c.half + (live ? tile.start + lane : 0)));
+        base = links + c.offset;
+        volume = c.volume;
+        beta = c.beta;
+        seed = c.seed;
+        if (live) stage_term3<false>(s0, base, volume, x, parity, mu, mu == 0 ? 1 : 0);
+    };
+    take_item(blockIdx.x);
+    for (int b = blockIdx.x; b < n_ctas; b += gridDim.x) {
+        unsigned accepted = 0;
+        double tr = 0.0;
+        const int32_t this_chain = chain;
+        const bool this_live = live;
+        m3 u, part;
         double2 (*sa)[T] = s1.f[0];
+        double beta3 = 0.0;
+        uint64_t key = 0;
+        double2 *dst = links;
+        const int64_t this_volume = volume;
+        if (live) {
+            const m3 a = staple_ring<MEASURE>(base, volume, x, parity, mu, s0, s1, part);
+            cp_async_wait_all();
+            u = staged_link(s0.f[0]);
+            // the accumulator, for the hits, in the second set's (now free) memory
 #pragma unroll
-        for (int e = 0; e < 9; ++e) sa[e][threadIdx.x] = make_double2(a.e[e / 3][e % 3].re, a.e[e / 3][e % 3].im);
-        const uint64_t key = link_key(c.seed, sweep, x.lex, MU);
-        accepted = visit_ordered<K>(u, sa, c.beta / 3.0, angle, key, tr);
-        store_su3(links, c, s, MU, u);
-        if (kSave) {   // Re Tr(U' A_p)
-            double q = 0.0;
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                const cplx col[3] = {a_part.e[0][i], a_part.e[1][i], a_part.e[2][i]};
-                q = q + retr_row_fma(u.e[i], col);
-            }
-            tr = q;
+            for (int e = 0; e < 9; ++e) sa[e][threadIdx.x] = make_double2(a.e[e / 3][e % 3].re, a.e[e / 3][e % 3].im);
+            key = link_key(seed, sweep, x.lex, mu);
+            beta3 = beta / 3.0;
+            dst = const_cast<double2 *>(base) + (int64_t)(mu * 9) * volume + (parity ? x.half : 0) + (x.lex >> 1);
         }
-    }
-    const unsigned warp_sum = __reduce_add_sync(0xffffffffu, accepted);
-    if ((threadIdx.x & 31) == 0 && warp_sum)
-        atomicAdd(accepts + tile.chain, (unsigned long long)warp_sum);
-    if (MEASURE) {
-        double v = (live && t < c.half) ? tr / 3.0 : 0.0;
-        v = block_reduce<false>(v);
-        if (threadIdx.x == 0) tr_partial[cta] = v;
+        // the next item's first staple term loads while this link's hits run
+        if (b + (int)gridDim.x < n_ctas) take_item(b + gridDim.x);
+        if (this_live) {
+            accepted = visit_ordered<K>(u, sa, beta3, angle, key, tr);
+#pragma unroll
+            for (int e = 0; e < 9; ++e)
+                dst[(int64_t)e * this_volume] = make_double2(u.e[e / 3][e % 3].re, u.e[e / 3][e % 3].im);
+            if (MEASURE && mu < 3) {   // Re Tr(U' A_p)
+                double q = 0.0;
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const cplx col[3] = {part.e[0][i], part.e[1][i], part.e[2][i]};
+                    q = q + retr_row_fma(u.e[i], col);
+                }
+                tr = q;
+            }
+        }
+        const unsigned warp_sum = __reduce_add_sync(0xffffffffu, accepted);
+        if ((threadIdx.x & 31) == 0 && warp_sum) atomicAdd(accepts + this_chain, (unsigned long long)warp_sum);
+        if (MEASURE) {
+            double v = this_live ? tr / 3.0 : 0.0;
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+            if ((threadIdx.x & 31) == 0)
+                tr_partial[(int64_t)(reverse ? n_ctas - 1 - b : b) * kSweepWarps + (threadIdx.x >> 5)] = v;
+        }
     }
 }
 
@@ -832,20 +955,29 @@ constexpr size_t kStageBytes = 27 * T * sizeof(double2);   // three staged facto
 
 constexpr size_t kRingBytes = (size_t)kRingBuffers * 9 * T * sizeof(double2);
 
+// Two resident CTAs per SM walk all work items.
+unsigned ring_grid(int64_t ctas) {
+    static thread_local int sms = 0, dev_seen = -1;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev != dev_seen) {
+        sms = 148;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        dev_seen = dev;
+    }
+    return (unsigned)(ctas < 2 * sms ? ctas : 2 * sms);
+}
+
 // Both launchers take the handle's sweep layout: work items of 2^log2
 // sites, chain order or by descending chain volume (all layouts give the
 // same bits).
 template <int K>
 void metro_launch_ordered(ym_ensemble *e, int parity, int mu, double angle, int reverse) {
     const SweepLayout &L = e->layouts[e->sweep_layout];
-    const dim3 grid((unsigned)L.ctas), block(T);
-    const Tile *items = L.d_items;
-    switch (mu) {
-    case 0: k_su3_metropolis_ring<0, K><<<grid, block, kRingBytes, e->stream>>>(e->d_chains, items, e->d_links, parity, angle, e->d_sweep, e->d_accepts, L.log2_item, reverse); break;
-    case 1: k_su3_metropolis_ring<1, K><<<grid, block, kRingBytes, e->stream>>>(e->d_chains, items, e->d_links, parity, angle, e->d_sweep, e->d_accepts, L.log2_item, reverse); break;
-    case 2: k_su3_metropolis_ring<2, K><<<grid, block, kRingBytes, e->stream>>>(e->d_chains, items, e->d_links, parity, angle, e->d_sweep, e->d_accepts, L.log2_item, reverse); break;
-    default: k_su3_metropolis_ring<3, K><<<grid, block, kRingBytes, e->stream>>>(e->d_chains, items, e->d_links, parity, angle, e->d_sweep, e->d_accepts, L.log2_item, reverse); break;
-    }
+    const dim3 grid(ring_grid(L.ctas)), block(T);
+    k_su3_metropolis_ring<K, false><<<grid, block, kRingBytes, e->stream>>>(
+        e->d_chains, L.d_items, (int)L.ctas, e->d_links, parity, mu, angle, e->d_sweep, e->d_accepts, L.log2_item,
+        reverse, nullptr);
 }
 
 void metro_launch_drawn(ym_ensemble *e, int parity, int mu, double angle, int reverse) {
@@ -866,14 +998,11 @@ void metro_launch_drawn(ym_ensemble *e, int parity, int mu, double angle, int re
 template <int K>
 void metro_launch_measure(ym_ensemble *e, int mu, double angle, double *tr_partial) {
     const SweepLayout &L = e->layouts[e->sweep_layout];
-    const dim3 g((unsigned)L.ctas), b(T);
+    const dim3 g(ring_grid(L.ctas)), b(T);
     const int rev = (1 * 4 + mu) & 1;   // the tile order tiled_launch gives (parity 1, mu)
-    if (mu == 1)
-        k_su3_metropolis_ring<1, K, true><<<g, b, kRingBytes, e->stream>>>(e->d_chains, L.d_items, e->d_links, 1, angle, e->d_sweep, e->d_accepts, L.log2_item, rev, tr_partial);
-    else if (mu == 2)
-        k_su3_metropolis_ring<2, K, true><<<g, b, kRingBytes, e->stream>>>(e->d_chains, L.d_items, e->d_links, 1, angle, e->d_sweep, e->d_accepts, L.log2_item, rev, tr_partial);
-    else
-        k_su3_metropolis_ring<3, K, true><<<g, b, kRingBytes, e->stream>>>(e->d_chains, L.d_items, e->d_links, 1, angle, e->d_sweep, e->d_accepts, L.log2_item, rev, tr_partial);
+    k_su3_metropolis_ring<K, true><<<g, b, kRingBytes, e->stream>>>(
+        e->d_chains, L.d_items, (int)L.ctas, e->d_links, 1, mu, angle, e->d_sweep, e->d_accepts, L.log2_item, rev,
+        tr_partial);
 }
 
 cudaError_t set_smem(const void *f, size_t bytes) {
@@ -892,16 +1021,8 @@ cudaError_t configure_kernels() {
     if (configured_device != dev) {
         const void *drawn[4] = {(const void *)k_su3_metropolis<0>, (const void *)k_su3_metropolis<1>,
                                 (const void *)k_su3_metropolis<2>, (const void *)k_su3_metropolis<3>};
-        const void *ordered[14] = {(const void *)k_su3_metropolis_ring<0, 11>, (const void *)k_su3_metropolis_ring<1, 11>,
-                                   (const void *)k_su3_metropolis_ring<2, 11>, (const void *)k_su3_metropolis_ring<3, 11>,
-                                   (const void *)k_su3_metropolis_ring<0, 14>, (const void *)k_su3_metropolis_ring<1, 14>,
-                                   (const void *)k_su3_metropolis_ring<2, 14>, (const void *)k_su3_metropolis_ring<3, 14>,
-                                   (const void *)k_su3_metropolis_ring<1, 11, true>,
-                                   (const void *)k_su3_metropolis_ring<2, 11, true>,
-                                   (const void *)k_su3_metropolis_ring<3, 11, true>,
-                                   (const void *)k_su3_metropolis_ring<1, 14, true>,
-                                   (const void *)k_su3_metropolis_ring<2, 14, true>,
-                                   (const void *)k_su3_metropolis_ring<3, 14, true>};
+        const void *ordered[4] = {(const void *)k_su3_metropolis_ring<11, false>, (const void *)k_su3_metropolis_ring<14, false>,
+                                  (const void *)k_su3_metropolis_ring<11, true>, (const void *)k_su3_metropolis_ring<14, true>};
         for (const void *f : drawn)
             if ((err = set_smem(f, kStageBytes)) != cudaSuccess) return err;
         for (const void *f : ordered)

@@ -226,12 +226,15 @@ __device__ __forceinline__ uint64_t link_key(uint64_t chain_seed, uint64_t sweep
                                              int mu) {
     return splitmix_at(splitmix_at(chain_seed, sweep), (uint64_t)(4 * lex + mu));
 }
-// proposal_angle_from_u64 (su3_ensemble.rs:199-213) for a validated angle.
+// proposal_angle_from_u64 (su3_ensemble.rs:199-213) for a validated angle:
+// +-angle * (2m + 1) * 2^-53 with m the word's low 52 bits.  m is written
+// into the mantissa of 2^52 (2^52 + m, exactly) instead of converted, 2m + 1
+// is one exact fma, and the factors 2^-53 and +-1 are exact, so the value is
+// the reference's.
 __device__ __forceinline__ double grid_angle(uint64_t raw, double angle) {
-    uint64_t m = raw & ((1ULL << 52) - 1);
-    double magnitude = angle * (double)(2 * m + 1) * (1.0 / 9007199254740992.0);
-    double sign = (raw >> 63) == 0 ? -1.0 : 1.0;
-    return sign * magnitude;
+    const double m = __longlong_as_double((long long)((raw & ((1ULL << 52) - 1)) | 0x4330000000000000ULL)) - 0x1p52;
+    const double magnitude = angle * fma(2.0, m, 1.0) * 0x1p-53;
+    return __longlong_as_double(__double_as_longlong(magnitude) | (long long)(~raw & 0x8000000000000000ULL));
 }
 
 // ------------------------------------------------- asynchronous staging

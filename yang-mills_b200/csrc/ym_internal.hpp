@@ -13,6 +13,7 @@
 namespace ym {
 
 constexpr int kSweepThreads = 128;   // threads per tile of a sub-sweep
+constexpr int kSweepWarps = kSweepThreads / 32;
 constexpr int kSiteThreads = 128;    // threads per tile of a measurement
 constexpr int64_t kLpPartialStride = 6304;  // floats per tile of learned-proposal gradient partials
 // Groups of 64 tiles in the first stage of the gradient reduction.
@@ -68,7 +69,7 @@ struct ym_ensemble {
     double *d_result2 = nullptr;
     unsigned long long *d_accepts = nullptr;   // SU(3) accepts / SU(2) heat-bath attempts
     unsigned *d_error = nullptr;               // device error bits (bounded loops that gave up)
-    double *d_tr_partial = nullptr;            // 3 x CTAs: plaquette shares of a measured sweep
+    double *d_tr_partial = nullptr;            // 3 x CTAs x kSweepWarps: plaquette shares of a measured sweep
     uint64_t *d_sweep = nullptr;           // next sweep index
     uint64_t *d_rng = nullptr;             // reference-replay stream states
     unsigned long long *d_ref_counts = nullptr;  // reference replay: proposals, accepts
