@@ -156,8 +156,9 @@ int32_t ym_su3_measured_run(ym_ensemble *ens, ym_ensemble *view, const ym_measur
  * chain is small enough for its links to sit in one CTA's shared memory
  * (4^4 and similar), sweeps can run chain-resident: one launch does many
  * whole sweeps of every chain in shared memory.  YM_PATH_AUTO (the default)
- * times a few sweeps on each path in the first call long enough to tell
- * them apart and keeps the faster; YM_PATH_TILED and YM_PATH_RESIDENT force
+ * runs resident when the handle has at most one chain per SM, else times a
+ * few sweeps on each path in the first call long enough to tell them apart
+ * and keeps the faster; YM_PATH_TILED and YM_PATH_RESIDENT force
  * one (RESIDENT fails with YM_ERR_INVALID_ARGUMENT when a chain does not
  * fit, the handle is not SU(3) FP64 or its fast sweeps are on).  Both paths
  * give the same bits:

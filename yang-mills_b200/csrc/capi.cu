@@ -329,6 +329,18 @@ bool resident_candidate(const ym_ensemble *e) {
 }
 
 constexpr int64_t kTuneSweeps = 4;   // sweeps timed per path when choosing
+
+// Whether an undecided handle runs resident without timing: one chain per SM
+// at most, so the launch is a single wave.  4^4, per measured sweep, resident
+// against tiled: 1 to 148 chains 52 against 87-96 us (ordered hits) and 82
+// against 118-126 us (drawn); 4^3 x 6 119 against 140-193 us.  Past one wave
+// it depends on the chains (160: 101 against 117 and 163 against 157 us; 600:
+// 250 against 273 and 406 against 381 us), and the tuner times both.
+bool one_wave(const ym_ensemble *e) {
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
+    return e->n_chains <= sms;
+}
 // Sweeps a call needs before the layout tuner runs: its probes (one warm
 // sweep, then kTuneSweeps per layout, all ordinary sweeps of the chains
 // launched without graph replay) are then at most half of the call.
@@ -701,7 +713,9 @@ int32_t ym_su3_metropolis_sweeps(ym_ensemble *e, double angle, int32_t generator
     // kTuneSweeps sweeps on each sub-sweep layout (item size, chain order)
     // and keeps the fastest.  Every layout gives the same bits, so the probe
     // sweeps are ordinary sweeps of the chains.
-    if (!f32(e) && e->n_chains > 1 && !e->layout_tuned && !e->profiling &&
+    const bool resident = resident_candidate(e) &&
+                          (e->resident_choice == 1 || (e->resident_choice < 0 && one_wave(e)));
+    if (!f32(e) && e->n_chains > 1 && !e->layout_tuned && !e->profiling && !resident &&
         n_sweeps >= kLayoutTuneMin) {
         float best = 0.f;
         int32_t pick = 0;
@@ -727,6 +741,7 @@ int32_t ym_su3_metropolis_sweeps(ym_ensemble *e, double angle, int32_t generator
     // Small chains: the first call long enough times kTuneSweeps sweeps on
     // each path and keeps the faster; the rest go to the chosen path.
     if (resident_candidate(e) && n_sweeps - done >= 2 * kTuneSweeps) {
+        if (e->resident_choice < 0 && one_wave(e)) e->resident_choice = 1;
         if (e->resident_choice < 0) {
             float t_tiled = 0.f, t_res = 0.f;
             YM_CUDA(time_on_stream(e, [&] {
@@ -742,7 +757,7 @@ int32_t ym_su3_metropolis_sweeps(ym_ensemble *e, double angle, int32_t generator
         }
     }
     if (resident_candidate(e)) {
-        if (e->resident_choice == 1 && done < n_sweeps) {
+        if ((e->resident_choice == 1 || (e->resident_choice < 0 && one_wave(e))) && done < n_sweeps) {
             YM_CUDA(ym::launch_su3_resident(e, angle, generator_mode, 1, n_sweeps - done, nullptr));
             done = n_sweeps;
         }
@@ -874,28 +889,37 @@ int32_t ym_su3_measured_sweeps(ym_ensemble *e, double angle, int32_t generator_m
         if (err == cudaSuccess) err = ym::launch_store_series(e, e->d_series, e->d_series_row);
         return err;
     };
-    if (!e->measure_graph || e->measure_graph_angle != angle || e->measure_graph_mode != generator_mode ||
-        e->measure_graph_stride != sweeps_per_measurement) {
+    // the captured cadence, made when the first row needs it (the
+    // chain-resident kernel writes its rows itself)
+    auto step_graph = [&]() -> cudaError_t {
+        if (e->measure_graph && e->measure_graph_angle == angle && e->measure_graph_mode == generator_mode &&
+            e->measure_graph_stride == sweeps_per_measurement)
+            return cudaSuccess;
         if (e->measure_graph) cudaGraphExecDestroy(e->measure_graph);
         e->measure_graph = nullptr;
         cudaGraph_t g = nullptr;
-        YM_CUDA(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
-        cudaError_t err = step();
-        cudaError_t end = cudaStreamEndCapture(e->stream, &g);
+        cudaError_t err = cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal);
+        if (err != cudaSuccess) return err;
+        err = step();
+        const cudaError_t end = cudaStreamEndCapture(e->stream, &g);
         if (err == cudaSuccess) err = end;
         if (err == cudaSuccess) err = cudaGraphInstantiate(&e->measure_graph, g, 0);
         if (g) cudaGraphDestroy(g);
-        YM_CUDA(err);
+        if (err != cudaSuccess) return err;
         e->measure_graph_angle = angle;
         e->measure_graph_mode = generator_mode;
         e->measure_graph_stride = sweeps_per_measurement;
-    }
+        return cudaSuccess;
+    };
     int64_t m = 0;
     if (resident_candidate(e)) {
         // Rows written by the resident kernel go to row m of the series; the
         // tiled graph continues from the device row counter.
+        if (e->resident_choice < 0 && n_measurements * sweeps_per_measurement >= 2 * kTuneSweeps && one_wave(e))
+            e->resident_choice = 1;
         if (e->resident_choice < 0 && n_measurements >= 2 && n_measurements * sweeps_per_measurement >= 2 * kTuneSweeps) {
             float t_tiled = 0.f, t_res = 0.f;
+            YM_CUDA(step_graph());
             YM_CUDA(time_on_stream(e, [&] { return cudaGraphLaunch(e->measure_graph, e->stream); }, &t_tiled));
             YM_CUDA(time_on_stream(e, [&] {
                 return ym::launch_su3_resident(e, angle, generator_mode, 1, sweeps_per_measurement,
@@ -904,7 +928,7 @@ int32_t ym_su3_measured_sweeps(ym_ensemble *e, double angle, int32_t generator_m
             e->resident_choice = t_res < t_tiled ? 1 : 0;
             m = 2;
         }
-        if (e->resident_choice == 1 && m < n_measurements) {
+        if ((e->resident_choice == 1 || (e->resident_choice < 0 && one_wave(e))) && m < n_measurements) {
             YM_CUDA(ym::launch_su3_resident(e, angle, generator_mode, n_measurements - m, sweeps_per_measurement,
                                             e->d_series + m * e->n_chains));
             m = n_measurements;
@@ -915,6 +939,7 @@ int32_t ym_su3_measured_sweeps(ym_ensemble *e, double angle, int32_t generator_m
             YM_CUDA(cudaStreamSynchronize(e->stream));
         }
     }
+    if (m < n_measurements) YM_CUDA(step_graph());
     for (; m < n_measurements; ++m) YM_CUDA(cudaGraphLaunch(e->measure_graph, e->stream));
     YM_CUDA(cudaMemcpyAsync(series, e->d_series, (size_t)(n_measurements * e->n_chains) * sizeof(double),
                             cudaMemcpyDeviceToHost, e->stream));

@@ -34,14 +34,6 @@
 #include "su3_sites.cuh"
 #include "ym_internal.hpp"
 
-#ifndef YM_METRO_MIN_BLOCKS
-// Resident 128-thread blocks per SM the register budget of k_su3_metropolis
-// targets: the staging buffers (54 KB dynamic + the 18 KB accumulator per
-// block) fit three blocks per SM, and at three blocks 168 registers per
-// thread leave no spills.
-#define YM_METRO_MIN_BLOCKS 3
-#endif
-
 // The two compilations live in different namespaces, so that their kernels
 // are told apart by name (profilers show ym::tiled_exact::... and
 // ym::tiled_fast::...).
@@ -57,29 +49,33 @@ namespace {
 
 constexpr int T = kSweepThreads;
 
-__device__ __forceinline__ cplx sa_get(const double2 (*sa)[T], int e) {
-    const double2 v = sa[e][threadIdx.x];
-    return cmake(v.x, v.y);
-}
-__device__ __forceinline__ void sa_put(double2 (*sa)[T], int e, cplx v) {
-    sa[e][threadIdx.x] = make_double2(v.re, v.im);
-}
-
-// Column i of A: A[0][i], A[1][i], A[2][i].
-__device__ __forceinline__ void sa_col(const double2 (*sa)[T], int i, cplx col[3]) {
+// A matrix held as nine double2 in memory, entry e at p[e * stride]: a
+// thread's column of a [9][T] shared buffer (S = T, offsets are immediates),
+// or a link of a chain held in shared memory (S = 0, stride the volume).
+template <int S>
+struct Col {
+    double2 *p;
+    int stride;
+    __device__ __forceinline__ double2 *at(int e) const { return p + e * (S ? S : stride); }
+    __device__ __forceinline__ cplx get(int e) const {
+        const double2 v = *at(e);
+        return cmake(v.x, v.y);
+    }
+    __device__ __forceinline__ void put(int e, cplx v) const { *at(e) = make_double2(v.re, v.im); }
+    // row i (entries 3 i ..), column i (entries i, 3 + i, 6 + i)
+    __device__ __forceinline__ void row(int i, cplx r[3]) const {
 #pragma unroll
-    for (int k = 0; k < 3; ++k) col[k] = sa_get(sa, 3 * k + i);
-}
-
-// Link (s, mu) into this thread's column of the staging buffer.
-__device__ __forceinline__ void stage_link(double2 (*buf)[T], const double2 *links, const ChainInfo &c,
-                                           int64_t s, int mu) {
-    const double2 *p = links + c.offset + (int64_t)(mu * 9) * c.volume + s;
+        for (int k = 0; k < 3; ++k) r[k] = get(3 * i + k);
+    }
+    __device__ __forceinline__ void column(int i, cplx c[3]) const {
 #pragma unroll
-    for (int e = 0; e < 9; ++e) cp_async16(&buf[e][threadIdx.x], p + (int64_t)e * c.volume);
-    cp_async_commit();
-}
+        for (int k = 0; k < 3; ++k) c[k] = get(3 * k + i);
+    }
+};
 
+__device__ __forceinline__ Col<T> column_of(double2 (*buf)[T]) { return Col<T>{&buf[0][threadIdx.x], T}; }
+
+// A link from this thread's column of a staging buffer.
 __device__ __forceinline__ m3 staged_link(const double2 (*buf)[T]) {
     m3 o;
 #pragma unroll
@@ -88,244 +84,6 @@ __device__ __forceinline__ m3 staged_link(const double2 (*buf)[T]) {
         o.e[e / 3][e % 3] = cmake(v.x, v.y);
     }
     return o;
-}
-
-// Staple sum A for link (x, MU): for each NU != MU in ascending order, the
-// forward term U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag, then the backward term
-// U_nu(x-nu+mu)^dag U_mu(x-nu)^dag U_nu(x-nu); P = the first two factors (fma
-// chains from zero), then A += P * third factor.  Every factor is staged by
-// cp.async: the first two one term ahead, the third at the start of its own
-// term, so each product starts on data that has already landed.
-struct TermSites {
-    int64_t s1, s2, s3;   // storage indices of the three factors
-};
-
-template <int MU, int NU, bool BWD>
-__device__ __forceinline__ TermSites term_sites(const ChainInfo &c, const Coord &x, int par,
-                                                const Nb &pm) {
-    if (!BWD) {
-        const Nb pn = step(c, x.x, x.lex, par, NU, +1);
-        return TermSites{storage_index(c, pm.lex, pm.par), storage_index(c, pn.lex, pn.par),
-                         storage_index(c, x.lex, par)};
-    }
-    const Nb mn = step(c, x.x, x.lex, par, NU, -1);
-    const Nb mnpm = step(c, x.x, mn.lex, mn.par, MU, +1);
-    const int64_t smn = storage_index(c, mn.lex, mn.par);
-    return TermSites{storage_index(c, mnpm.lex, mnpm.par), smn, smn};
-}
-
-struct StageBufs {
-    double2 (*l1)[T];
-    double2 (*l2)[T];
-    double2 (*l3)[T];
-};
-
-__device__ __forceinline__ void stage_pair(const StageBufs &b, const double2 *links, const ChainInfo &c,
-                                           const TermSites &t, int d1, int d2) {
-    const double2 *p1 = links + c.offset + (int64_t)(d1 * 9) * c.volume + t.s1;
-    const double2 *p2 = links + c.offset + (int64_t)(d2 * 9) * c.volume + t.s2;
-#pragma unroll
-    for (int e = 0; e < 9; ++e) {
-        cp_async16(&b.l1[e][threadIdx.x], p1 + (int64_t)e * c.volume);
-        cp_async16(&b.l2[e][threadIdx.x], p2 + (int64_t)e * c.volume);
-    }
-    cp_async_commit();
-}
-
-// Term (NU, BWD) with its sites `cur`; stages the next term's first two
-// factors (sites `nxt`, directions NNU / MU) when HAS_NEXT, else the updated
-// link U_MU at storage index nxt.s1 into the first buffer, so it lands
-// during the last product.
-template <int MU, int NU, bool BWD, bool HAS_NEXT, int NNU>
-__device__ __forceinline__ void staged_term(const double2 *links, const ChainInfo &c, const TermSites &cur,
-                                            const TermSites &nxt, const StageBufs &b, double2 (*sa)[T]) {
-    stage_link(b.l3, links, c, cur.s3, NU);
-    cp_async_wait_one();   // this term's first two factors have landed
-    m3 p;
-    {
-        const m3 l1 = staged_link(b.l1), l2 = staged_link(b.l2);
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                cplx v = cmake(0.0, 0.0);
-#pragma unroll
-                for (int j = 0; j < 3; ++j) {
-                    if (!BWD) cfma(v, l1.e[r][j], cconj(l2.e[k][j]));
-                    else cfma(v, cconj(l1.e[j][r]), cconj(l2.e[k][j]));
-                }
-                p.e[r][k] = v;
-            }
-    }
-    if (HAS_NEXT) {
-        stage_pair(b, links, c, nxt, NNU, MU);
-        cp_async_wait_one();   // the third factor (older group) has landed
-    } else {
-        stage_link(b.l1, links, c, nxt.s1, MU);   // the updated link itself (sites `nxt`)
-        cp_async_wait_one();
-    }
-    const m3 l3 = staged_link(b.l3);
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int col = 0; col < 3; ++col) {
-            cplx a = sa_get(sa, 3 * r + col);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                if (!BWD) cfma(a, p.e[r][k], cconj(l3.e[col][k]));
-                else cfma(a, p.e[r][k], l3.e[k][col]);
-            }
-            sa_put(sa, 3 * r + col, a);
-        }
-}
-
-template <int MU, int I>
-struct Nu {   // the I-th direction other than MU
-    static constexpr int v = I < MU ? I : I + 1;
-};
-
-template <int MU>
-__device__ __forceinline__ void staple_pipelined(const double2 *links, const ChainInfo &c, const Coord &x,
-                                                 int par, const Nb &pm, double2 (*sa)[T], const StageBufs &b,
-                                                 int64_t s_self) {
-    constexpr int N0 = Nu<MU, 0>::v, N1 = Nu<MU, 1>::v, N2 = Nu<MU, 2>::v;
-    const TermSites t0 = term_sites<MU, N0, false>(c, x, par, pm);
-    const TermSites t1 = term_sites<MU, N0, true>(c, x, par, pm);
-    stage_pair(b, links, c, t0, N0, MU);
-    staged_term<MU, N0, false, true, N0>(links, c, t0, t1, b, sa);
-    const TermSites t2 = term_sites<MU, N1, false>(c, x, par, pm);
-    staged_term<MU, N0, true, true, N1>(links, c, t1, t2, b, sa);
-    const TermSites t3 = term_sites<MU, N1, true>(c, x, par, pm);
-    staged_term<MU, N1, false, true, N1>(links, c, t2, t3, b, sa);
-    const TermSites t4 = term_sites<MU, N2, false>(c, x, par, pm);
-    staged_term<MU, N1, true, true, N2>(links, c, t3, t4, b, sa);
-    const TermSites t5 = term_sites<MU, N2, true>(c, x, par, pm);
-    staged_term<MU, N2, false, true, N2>(links, c, t4, t5, b, sa);
-    staged_term<MU, N2, true, false, N2>(links, c, t5, TermSites{s_self, 0, 0}, b, sa);
-}
-
-// Metropolis decision shared by the block and diagonal hits.
-__device__ __forceinline__ bool accept_step(double old_tr, double new_tr, double beta3,
-                                            double unif) {
-    const double ds = beta3 * (old_tr - new_tr);
-    const double m = fmax(ds, 0.0);          // (-delta.max(0.0)).exp() su3_ensemble.rs:368
-    return (m == 0.0) ? true : (unif < exp(-m));
-}
-
-// Hit with a block rotation on rows (I0, I1): [[c, i s],[i s, c]] (kind 0),
-// [[c, s],[-s, c]] (kind 1) or diag(c + i s, c - i s) (kind 2).  Candidate
-// rows are Mat3::mul's values (no fused multiply-add).
-template <int I0, int I1>
-__device__ __forceinline__ void hit_block(m3 &u, const double2 (*sa)[T], double rr[3], double &old_tr,
-                                          int kind, double c, double s, double beta3, double unif,
-                                          unsigned &accepted) {
-    cplx n0[3], n1[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const double x0 = u.e[I0][k].re, y0 = u.e[I0][k].im;
-        const double x1 = u.e[I1][k].re, y1 = u.e[I1][k].im;
-        if (kind == 0) {
-            n0[k] = cmake(c * x0 - s * y1, c * y0 + s * x1);
-            n1[k] = cmake(c * x1 - s * y0, s * x0 + c * y1);
-        } else if (kind == 1) {
-            n0[k] = cmake(c * x0 + s * x1, c * y0 + s * y1);
-            n1[k] = cmake(c * x1 - s * x0, c * y1 - s * y0);
-        } else {
-            n0[k] = cmake(c * x0 - s * y0, c * y0 + s * x0);
-            n1[k] = cmake(c * x1 + s * y1, c * y1 - s * x1);
-        }
-    }
-    cplx col0[3], col1[3];
-    sa_col(sa, I0, col0);
-    sa_col(sa, I1, col1);
-    double q[3] = {rr[0], rr[1], rr[2]};
-    q[I0] = retr_row_fma(n0, col0);
-    q[I1] = retr_row_fma(n1, col1);
-    const double new_tr = (q[0] + q[1]) + q[2];
-    if (accept_step(old_tr, new_tr, beta3, unif)) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            u.e[I0][k] = n0[k];
-            u.e[I1][k] = n1[k];
-        }
-        rr[I0] = q[I0];
-        rr[I1] = q[I1];
-        old_tr = new_tr;
-        accepted++;
-    }
-}
-
-__device__ __forceinline__ void hit_diag(m3 &u, const double2 (*sa)[T], double rr[3], double &old_tr,
-                                         cplx e1, cplx e2, double beta3, double unif,
-                                         unsigned &accepted) {
-    cplx n[3][3];
-    double q[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const cplx e = i < 2 ? e1 : e2;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) n[i][k] = cmul(e, u.e[i][k]);
-        cplx col[3];
-        sa_col(sa, i, col);
-        q[i] = retr_row_fma(n[i], col);
-    }
-    const double new_tr = (q[0] + q[1]) + q[2];
-    if (accept_step(old_tr, new_tr, beta3, unif)) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) u.e[i][k] = n[i][k];
-            rr[i] = q[i];
-        }
-        old_tr = new_tr;
-        accepted++;
-    }
-}
-
-// hit_block for a generator drawn per link (g < 7): rows i0, i1 picked by
-// selects and A's columns read from shared memory, so threads of a warp
-// with different SU(2)-subgroup generators stay converged.  Each kind of
-// hit_block writes its candidate entries as c*x + s*a with a one of the
-// other entries or its negation (c*x - s*y == c*x + s*(-y) exactly), so the
-// single formula gives hit_block's bits.
-__device__ __forceinline__ void hit_block_drawn(m3 &u, const double2 (*sa)[T], double rr[3],
-                                                double &old_tr, int g, double c, double s,
-                                                double beta3, double unif, unsigned &accepted) {
-    const int kind = (g == 2) ? 2 : ((g == 1 || g == 4 || g == 6) ? 1 : 0);
-    const int i0 = g <= 4 ? 0 : 1, i1 = g <= 2 ? 1 : 2;
-    cplx n0[3], n1[3], col0[3], col1[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const cplx r0 = i0 == 0 ? u.e[0][k] : u.e[1][k];
-        const cplx r1 = i1 == 1 ? u.e[1][k] : u.e[2][k];
-        const double x0 = r0.re, y0 = r0.im, x1 = r1.re, y1 = r1.im;
-        const double a0 = kind == 0 ? -y1 : (kind == 1 ? x1 : -y0);
-        const double b0 = kind == 0 ? x1 : (kind == 1 ? y1 : x0);
-        const double a1 = kind == 0 ? -y0 : (kind == 1 ? -x0 : y1);
-        const double b1 = kind == 0 ? x0 : (kind == 1 ? -y0 : -x1);
-        n0[k] = cmake(c * x0 + s * a0, c * y0 + s * b0);
-        n1[k] = cmake(c * x1 + s * a1, c * y1 + s * b1);
-    }
-    sa_col(sa, i0, col0);
-    sa_col(sa, i1, col1);
-    const double q0n = retr_row_fma(n0, col0), q1n = retr_row_fma(n1, col1);
-    const double q0 = i0 == 0 ? q0n : rr[0];
-    const double q1 = i0 == 1 ? q0n : (i1 == 1 ? q1n : rr[1]);
-    const double q2 = i1 == 2 ? q1n : rr[2];
-    const double new_tr = (q0 + q1) + q2;
-    if (accept_step(old_tr, new_tr, beta3, unif)) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            if (i0 == 0) u.e[0][k] = n0[k];
-            u.e[1][k] = i0 == 1 ? n0[k] : (i1 == 1 ? n1[k] : u.e[1][k]);
-            if (i1 == 2) u.e[2][k] = n1[k];
-        }
-        rr[0] = q0;
-        rr[1] = q1;
-        rr[2] = q2;
-        old_tr = new_tr;
-        accepted++;
-    }
 }
 
 // Fast form only (YM_TILED_FAST): cos h and sin h as polynomials in
@@ -353,72 +111,16 @@ __device__ __forceinline__ void cos_sin_horner(double h, double &c, double &s) {
     s = h * ps;
 }
 
-// Eight hits on u: generator h (ordered) or bits 52..54 of the hit's angle
-// word (uniform).  Words 2h and 2h+1 of the link's stream.
-__device__ __forceinline__ unsigned visit(m3 &u, const double2 (*sa)[T], double beta3,
-                                          double angle, uint64_t key, int uniform) {
-    double rr[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        cplx col[3];
-        sa_col(sa, i, col);
-        rr[i] = retr_row_fma(u.e[i], col);
-    }
-    double old_tr = (rr[0] + rr[1]) + rr[2];
-    unsigned accepted = 0;
-#pragma unroll 1
-    for (int h = 0; h < 8; ++h) {
-        const uint64_t w_angle = splitmix_at(key, (uint64_t)(2 * h));
-        const uint64_t w_acc = splitmix_at(key, (uint64_t)(2 * h + 1));
-        const int g = uniform ? (int)((w_angle >> 52) & 7) : h;
-        const double theta = grid_angle(w_angle, angle);
-        const double unif = unit_from(w_acc);
-        if (g == 7) {
-            cplx e1, e2;
-#ifdef YM_TILED_FAST
-            double c1, s1, c2, s2;
-            cos_sin_horner<16>((0.5 * kInvSqrt3) * theta, c1, s1);
-            cos_sin_horner<16>((-kInvSqrt3) * theta, c2, s2);
-            e1 = cmake(c1, s1);
-            e2 = cmake(c2, s2);
-#else
-            lambda8_rotation(theta, e1, e2);
-#endif
-            hit_diag(u, sa, rr, old_tr, e1, e2, beta3, unif, accepted);
-        } else {
-            double c, s;
-#ifdef YM_TILED_FAST
-            cos_sin_horner<16>(0.5 * theta, c, s);
-#else
-            taylor_chain(0.5 * theta, c, s);   // |0.5 theta| < 0.5: no squaring
-#endif
-            if (uniform) {
-                hit_block_drawn(u, sa, rr, old_tr, g, c, s, beta3, unif, accepted);
-                continue;
-            }
-            const int kind = (g == 2) ? 2 : ((g == 1 || g == 4 || g == 6) ? 1 : 0);
-            if (g <= 2)
-                hit_block<0, 1>(u, sa, rr, old_tr, kind, c, s, beta3, unif, accepted);
-            else if (g <= 4)
-                hit_block<0, 2>(u, sa, rr, old_tr, kind, c, s, beta3, unif, accepted);
-            else
-                hit_block<1, 2>(u, sa, rr, old_tr, kind, c, s, beta3, unif, accepted);
-        }
-    }
-    return accepted;
-}
-
-// ---- the reference's ordered hits, software-pipelined ---------------------
+// ---- the hits, software-pipelined ------------------------------------------
 // A hit has a link-independent half (its two stream words, the angle, the
 // rotation entries from the Taylor chain, the accept threshold) and a
 // link-dependent half (candidate rows, Re Tr against the staple, the
-// decision).  visit() runs them back to back, and the Taylor chain's early
-// exits split the code into many small blocks; here every hit's
-// link-independent half is computed next to the previous hit's
-// link-dependent half, so each link carries two independent dependency
-// chains instead of one.  The values are visit()'s, bit for bit:
-//   * taylor_fixed<K> adds K terms of taylor_chain's recurrence, without its
-//     1e-18 stop.  A term past the stop is below 1e-18 |h| / 2, less than
+// decision).  Every hit's link-independent half is computed next to the
+// previous hit's link-dependent half, so each link carries two independent
+// dependency chains instead of one.  The values are the reference's, bit for
+// bit:
+//   * taylor_fixed<K> adds K terms of the reference's recurrence (taylor_chain,
+//     su3_exp.cuh), without its 1e-18 stop.  A term past the stop is below 1e-18 |h| / 2, less than
 //     half an ulp of both sums (c >= 0.87; s >= 0.95 |h|), so adding it
 //     changes no bit, and leaving the test out saves a comparison and a
 //     select per term.  K is taken from the proposal half width a: |t_k| <=
@@ -430,8 +132,9 @@ __device__ __forceinline__ unsigned visit(m3 &u, const double2 (*sa)[T], double 
 //     = 4.7e-17 < 2^-54, t_16 <= 7.3e-19), so the sums are the reference's
 //     bit for bit (checked on the CPU against the loop run to the cutoff
 //     over millions of grid angles).
-//   * the decision is accept_step's u < exp(-max(dS, 0)) through accept_log;
-//     the accepted rows are selected, not branched to.
+//   * the decision is the reference's u < exp(-max(dS, 0))
+//     (su3_ensemble.rs:368) through accept_log; the accepted rows are
+//     selected, not branched to.
 template <int K>
 __device__ __forceinline__ void taylor_fixed(double h, double &c, double &s) {
     double t = h;      // k = 1: t = (1 h) 1, s = 0 + t
@@ -468,7 +171,7 @@ __device__ __forceinline__ void lambda8_fixed(double theta, cplx &e1, cplx &e2) 
 // 65,536, return NaN: never sure); __logf adds at most 3.6e-7 on [0.5, 2] and
 // 3 ulp, 2.9e-6, down to log 2^-16 = -11.1; rounding m to binary32 7e-7.
 // Together below kLogBand, so every decision outside the band is
-// accept_step's; one inside (one in a few thousand) evaluates that test.
+// that test's; one inside (one in a few thousand) evaluates it.
 constexpr float kLogBand = 2.5e-5f;
 
 __device__ __forceinline__ float neg_log_unit(uint64_t w) {
@@ -573,15 +276,14 @@ __device__ __forceinline__ void take_row(Row &r, bool acc, const cplx n[3], doub
 // An SU(2)-subgroup hit on rows x and y, whose A columns are ca and cb; z is
 // the third row.  first: the subgroup is (0, 1), so the trace sums as
 // (x + y) + z; else z lies between or before them: (x + z) + y.
-template <int KIND>
-__device__ __forceinline__ void hit_rows(Row &x, Row &y, const Row &z, const double2 (*ca)[T],
-                                         const double2 (*cb)[T], bool first, double &old_tr, const BlockPre &p,
+template <int KIND, class A>
+__device__ __forceinline__ void hit_rows(Row &x, Row &y, const Row &z, const A &a, int ca, int cb, bool first, double &old_tr, const BlockPre &p,
                                          double beta3, unsigned &accepted, uint64_t key, int h) {
     cplx n0[3], n1[3], col[3];
     block_candidate<KIND>(x, y, p.c, p.s, n0, n1);
-    sa_col(ca, 0, col);
+    a.column(ca, col);
     const double q0 = retr_row_fma(n0, col);
-    sa_col(cb, 0, col);
+    a.column(cb, col);
     const double q1 = retr_row_fma(n1, col);
     const double mid = first ? q1 : z.rr, end = first ? z.rr : q1;
     const double new_tr = (q0 + mid) + end;
@@ -603,14 +305,14 @@ __device__ __forceinline__ void swap_rows(Row &x, Row &y) {
 // places between its passes, so one copy of the code serves all three.  Hit
 // h+1's link-independent half is written next to hit h.
 // tr receives Re Tr(U' A) of the final link, the sum of its six plaquettes.
-template <int K>
-__device__ __forceinline__ unsigned visit_ordered(m3 &u, const double2 (*sa)[T], double beta3,
-                                                  double angle, uint64_t key, double &tr) {
+template <int K, class A>
+__device__ __forceinline__ unsigned visit_ordered(m3 &u, const A &sa, double beta3, double angle, uint64_t key,
+                                                  double &tr) {
     Row r[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         cplx col[3];
-        sa_col(sa, i, col);
+        sa.column(i, col);
 #pragma unroll
         for (int k = 0; k < 3; ++k) r[i].e[k] = u.e[i][k];
         r[i].rr = retr_row_fma(u.e[i], col);
@@ -622,16 +324,15 @@ __device__ __forceinline__ unsigned visit_ordered(m3 &u, const double2 (*sa)[T],
     BlockPre p = pre_block<K>(state, angle);
 #pragma unroll 1
     for (int it = 0; it < 3; ++it) {
-        const double2 (*ca)[T] = sa + (it == 2 ? 1 : 0);
-        const double2 (*cb)[T] = sa + (it == 0 ? 1 : 2);
+        const int ca = it == 2 ? 1 : 0, cb = it == 0 ? 1 : 2;
         const int h0 = it == 0 ? 0 : 2 * it + 1;   // the pass's first hit
         BlockPre q = pre_block<K>(state, angle);
-        hit_rows<0>(x, y, z, ca, cb, it == 0, old_tr, p, beta3, accepted, key, h0);
+        hit_rows<0>(x, y, z, sa, ca, cb, it == 0, old_tr, p, beta3, accepted, key, h0);
         if (it < 2) p = pre_block<K>(state, angle);
-        hit_rows<1>(x, y, z, ca, cb, it == 0, old_tr, q, beta3, accepted, key, h0 + 1);
+        hit_rows<1>(x, y, z, sa, ca, cb, it == 0, old_tr, q, beta3, accepted, key, h0 + 1);
         if (it == 0) {
             q = pre_block<K>(state, angle);
-            hit_rows<2>(x, y, z, ca, cb, true, old_tr, p, beta3, accepted, key, 2);
+            hit_rows<2>(x, y, z, sa, ca, cb, true, old_tr, p, beta3, accepted, key, 2);
             p = q;
             swap_rows(y, z);
         } else if (it == 1) {
@@ -647,11 +348,11 @@ __device__ __forceinline__ unsigned visit_ordered(m3 &u, const double2 (*sa)[T],
         n1[k] = cmul(d.e1, x.e[k]);
         n2[k] = cmul(d.e2, y.e[k]);
     }
-    sa_col(sa, 0, col);
+    sa.column(0, col);
     const double q0 = retr_row_fma(n0, col);
-    sa_col(sa, 1, col);
+    sa.column(1, col);
     const double q1 = retr_row_fma(n1, col);
-    sa_col(sa, 2, col);
+    sa.column(2, col);
     const double q2 = retr_row_fma(n2, col);
     const double new_tr = (q0 + q1) + q2;
     const bool acc = accept_log(beta3 * (old_tr - new_tr), d.logu, key, 7);
@@ -667,44 +368,126 @@ __device__ __forceinline__ unsigned visit_ordered(m3 &u, const double2 (*sa)[T],
     return accepted;
 }
 
-// Drawn generators (visit()): three CTAs per SM, the accumulator in shared
-// memory, one staple term staged ahead.
-template <int MU>
-__global__ void __launch_bounds__(T, YM_METRO_MIN_BLOCKS)
-k_su3_metropolis(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles,
-                 double2 *__restrict__ links, int parity, double angle, int uniform,
-                 const uint64_t *__restrict__ sweep_ptr, unsigned long long *__restrict__ accepts,
-                 int log2_item, int reverse) {
-    __shared__ double2 sa[9][T];
-    extern __shared__ __align__(16) double2 stage_mem[];
-    const StageBufs bufs{reinterpret_cast<double2 (*)[T]>(stage_mem),
-                         reinterpret_cast<double2 (*)[T]>(stage_mem + 9 * T),
-                         reinterpret_cast<double2 (*)[T]>(stage_mem + 18 * T)};
-    // The CTA takes T >> log2_item work items of 2^log2_item sites each
-    // (possibly of different chains); padding items have chain < 0.
-    const int64_t cta = reverse ? (int64_t)gridDim.x - 1 - blockIdx.x : (int64_t)blockIdx.x;
-    const Tile tile = tiles[cta * (T >> log2_item) + (threadIdx.x >> log2_item)];
-    const bool live = tile.chain >= 0;
-    const ChainInfo c = chains[live ? tile.chain : 0];
-    const int64_t t = tile.start + (threadIdx.x & ((1u << log2_item) - 1u));
-    const uint64_t sweep = *sweep_ptr;
-    unsigned accepted = 0;
-    if (live && t < c.half) {
-        const int64_t s = (int64_t)parity * c.half + t;
-        const Coord x = decode_storage(c, s);
+// ---- drawn generators ------------------------------------------------------
+// Eight hits whose generator each link draws (bits 52..54 of the angle word).
+// One formula serves all eight generators, so a warp whose links drew
+// different ones stays converged: with rows r0, r1 of the generator's
+// subgroup (lambda3 and lambda8: rows 0, 1) the candidate is
+//   n0 = c r0 + s v0,  n1 = c r1 + s' v1,  v = w or i w,
+//   lambda1, 4, 6: v0 = i r1, v1 = i r0;   lambda2, 5, 7: v0 = r1, v1 = r0, s' = -s;
+//   lambda3: v0 = i r0, v1 = i r1, s' = -s;  lambda8: v0 = i r0, v1 = i r1,
+// entry by entry the reference's two rounded products and their sum (a sign
+// change is exact).  lambda8's second phase on row 2 runs in a short branch.
+// The link's rows and A's columns live in memory (u, a) and are addressed by
+// the generator: picking them among registers took twice the instructions
+// (10,600 per warp and visit, most of them selects and the two divergent
+// sides, against 4,900).
+struct DrawnPre {
+    double c, s;     // block rotation, or lambda8's phase of rows 0 and 1
+    double h2;       // lambda8: half angle of row 2's phase
+    float logu;
+    int g;
+    bool sq;         // lambda8: the phases are squared once
+};
+
+template <int K>
+__device__ __forceinline__ DrawnPre pre_drawn(uint64_t &state, double angle) {
+    DrawnPre p;
+    const uint64_t w = next_word(state);
+    p.g = (int)((w >> 52) & 7);
+    const double theta = grid_angle(w, angle);
+    const double d1 = (0.5 * kInvSqrt3) * theta, d2 = (-kInvSqrt3) * theta;
+    const bool diag = p.g == 7;
+#ifdef YM_TILED_FAST
+    p.sq = false;
+#else
+    p.sq = diag && fmax(fabs(d1), fabs(d2)) > 0.5;
+#endif
+    const double sc = p.sq ? 0.5 : 1.0;
+    p.h2 = d2 * sc;
+    block_rotation<K>(diag ? d1 * sc : 0.5 * theta, p.c, p.s);
+    p.logu = neg_log_unit(next_word(state));
+    return p;
+}
+
+template <int K, class U, class A>
+__device__ __forceinline__ unsigned visit_drawn(const U &u, const A &a, double beta3, double angle, uint64_t key) {
+    double rr[3];
 #pragma unroll
-        for (int e = 0; e < 9; ++e) sa[e][threadIdx.x] = make_double2(0.0, 0.0);
-        const Nb pm = step(c, x.x, x.lex, parity, MU, +1);
-        staple_pipelined<MU>(links, c, x, parity, pm, sa, bufs, s);
-        cp_async_wait_all();
-        m3 u = staged_link(bufs.l1);
-        const uint64_t key = link_key(c.seed, sweep, x.lex, MU);
-        accepted = visit(u, sa, c.beta / 3.0, angle, key, uniform);
-        store_su3(links, c, s, MU, u);
+    for (int i = 0; i < 3; ++i) {
+        cplx row[3], col[3];
+        u.row(i, row);
+        a.column(i, col);
+        rr[i] = retr_row_fma(row, col);
     }
-    const unsigned warp_sum = __reduce_add_sync(0xffffffffu, accepted);
-    if ((threadIdx.x & 31) == 0 && warp_sum)
-        atomicAdd(accepts + tile.chain, (unsigned long long)warp_sum);
+    double old_tr = (rr[0] + rr[1]) + rr[2];
+    unsigned accepted = 0;
+    uint64_t state = key;
+    DrawnPre nx = pre_drawn<K>(state, angle);
+#pragma unroll 1
+    for (int h = 0; h < 8; ++h) {
+        const DrawnPre p = nx;
+        if (h < 7) nx = pre_drawn<K>(state, angle);
+        const int g = p.g;
+        const bool diag = g == 7;
+        const bool low = g <= 2 || diag;                 // rows 0 and 1
+        const int i0 = (g <= 4 || diag) ? 0 : 1, i1 = low ? 1 : 2, i2 = 3 - i0 - i1;
+        const bool plain = g == 1 || g == 4 || g == 6;   // v = w, not i w
+        const bool cross = !(g == 2 || diag);            // w is the other row
+        cplx r0[3], r1[3], n0[3], n1[3], n2[3], col[3];
+        u.row(i0, r0);
+        u.row(i1, r1);
+        double c = p.c, s = p.s;
+        double q2 = i2 == 2 ? rr[2] : (i2 == 1 ? rr[1] : rr[0]);
+        if (diag) {
+            cplx e2;
+            block_rotation<K>(p.h2, e2.re, e2.im);
+            if (p.sq) {
+                const cplx e1 = cmul(cmake(c, s), cmake(c, s));
+                c = e1.re;
+                s = e1.im;
+                e2 = cmul(e2, e2);
+            }
+            cplx r2[3];
+            u.row(2, r2);
+            a.column(2, col);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) n2[k] = cmul(e2, r2[k]);
+            q2 = retr_row_fma(n2, col);
+        }
+        const double s1 = (plain || g == 2) ? -s : s;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const cplx w0 = cross ? r1[k] : r0[k], w1 = cross ? r0[k] : r1[k];
+            const double v0r = plain ? w0.re : -w0.im, v0i = plain ? w0.im : w0.re;
+            const double v1r = plain ? w1.re : -w1.im, v1i = plain ? w1.im : w1.re;
+            n0[k] = cmake(c * r0[k].re + s * v0r, c * r0[k].im + s * v0i);
+            n1[k] = cmake(c * r1[k].re + s1 * v1r, c * r1[k].im + s1 * v1i);
+        }
+        a.column(i0, col);
+        const double q0 = retr_row_fma(n0, col);
+        a.column(i1, col);
+        const double q1 = retr_row_fma(n1, col);
+        const double mid = low ? q1 : q2, end = low ? q2 : q1;
+        const double new_tr = (q0 + mid) + end;
+        if (accept_log(beta3 * (old_tr - new_tr), p.logu, key, h)) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                u.put(3 * i0 + k, n0[k]);
+                u.put(3 * i1 + k, n1[k]);
+            }
+            if (diag) {
+#pragma unroll
+                for (int k = 0; k < 3; ++k) u.put(6 + k, n2[k]);
+            }
+            rr[0] = i0 == 0 ? q0 : rr[0];
+            rr[1] = i0 == 1 ? q0 : (i1 == 1 ? q1 : rr[1]);
+            rr[2] = i1 == 2 ? q1 : (diag ? q2 : rr[2]);
+            old_tr = new_tr;
+            accepted++;
+        }
+    }
+    return accepted;
 }
 
 // ---- ordered hits: two staple terms in flight, two CTAs per SM -----------
@@ -793,25 +576,28 @@ __device__ __forceinline__ void stage_term3(const TermSet &b, const double2 *bas
     cp_async_commit();
 }
 
+// A staple term's two products: P = U V^dag (forward) or U^dag V^dag
+// (backward) as fma chains from zero, then A += P W^dag or P W.
 template <bool BWD>
-__device__ __forceinline__ void term_accumulate(const TermSet &b, m3 &a) {
+__device__ __forceinline__ m3 pair_product(const m3 &l1, const m3 &l2) {
     m3 p;
-    {
-        const m3 l1 = staged_link(b.f[0]), l2 = staged_link(b.f[1]);
 #pragma unroll
-        for (int r = 0; r < 3; ++r)
+    for (int r = 0; r < 3; ++r)
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                cplx v = cmake(0.0, 0.0);
+        for (int k = 0; k < 3; ++k) {
+            cplx v = cmake(0.0, 0.0);
 #pragma unroll
-                for (int j = 0; j < 3; ++j) {
-                    if (!BWD) cfma(v, l1.e[r][j], cconj(l2.e[k][j]));
-                    else cfma(v, cconj(l1.e[j][r]), cconj(l2.e[k][j]));
-                }
-                p.e[r][k] = v;
+            for (int j = 0; j < 3; ++j) {
+                if (!BWD) cfma(v, l1.e[r][j], cconj(l2.e[k][j]));
+                else cfma(v, cconj(l1.e[j][r]), cconj(l2.e[k][j]));
             }
-    }
-    const m3 l3 = staged_link(b.f[2]);
+            p.e[r][k] = v;
+        }
+    return p;
+}
+
+template <bool BWD>
+__device__ __forceinline__ void add_third(const m3 &p, const m3 &l3, m3 &a) {
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
@@ -821,6 +607,16 @@ __device__ __forceinline__ void term_accumulate(const TermSet &b, m3 &a) {
                 if (!BWD) cfma(a.e[r][col], p.e[r][k], cconj(l3.e[col][k]));
                 else cfma(a.e[r][col], p.e[r][k], l3.e[k][col]);
             }
+}
+
+template <bool BWD>
+__device__ __forceinline__ void term_accumulate(const TermSet &b, m3 &a) {
+    m3 p;
+    {
+        const m3 l1 = staged_link(b.f[0]), l2 = staged_link(b.f[1]);
+        p = pair_product<BWD>(l1, l2);
+    }
+    add_third<BWD>(p, staged_link(b.f[2]), a);
 }
 
 // The staple of link (x, mu); term 0 has been staged into s0.  SAVE (mu = 1
@@ -865,7 +661,7 @@ constexpr int kRingBuffers = 6;   // two sets of three factors
 // links here), and each plaquette of plane (nu, MU) holds exactly one
 // odd-site MU-link, so the three launches' sums are the plaquettes of
 // planes (0,1); (0,2), (1,2); (0,3), (1,3), (2,3): all six planes.
-template <int K, bool MEASURE>
+template <int K, bool MEASURE, bool DRAWN>
 __global__ void __launch_bounds__(T, 2)
 k_su3_metropolis_ring(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles, int n_ctas,
                       double2 *__restrict__ links, int parity, int mu, double angle,
@@ -905,7 +701,7 @@ k_su3_metropolis_ring(const ChainInfo *__restrict__ chains, const Tile *__restri
         const int32_t this_chain = chain;
         const bool this_live = live;
         m3 u, part;
-        double2 (*sa)[T] = s1.f[0];
+        const Col<T> sa = column_of(s1.f[0]);
         double beta3 = 0.0;
         uint64_t key = 0;
         double2 *dst = links;
@@ -916,7 +712,7 @@ k_su3_metropolis_ring(const ChainInfo *__restrict__ chains, const Tile *__restri
             u = staged_link(s0.f[0]);
             // the accumulator, for the hits, in the second set's (now free) memory
 #pragma unroll
-            for (int e = 0; e < 9; ++e) sa[e][threadIdx.x] = make_double2(a.e[e / 3][e % 3].re, a.e[e / 3][e % 3].im);
+            for (int e = 0; e < 9; ++e) sa.put(e, a.e[e / 3][e % 3]);
             key = link_key(seed, sweep, x.lex, mu);
             beta3 = beta / 3.0;
             dst = const_cast<double2 *>(base) + (int64_t)(mu * 9) * volume + (parity ? x.half : 0) + (x.lex >> 1);
@@ -924,7 +720,15 @@ k_su3_metropolis_ring(const ChainInfo *__restrict__ chains, const Tile *__restri
         // the next item's first staple term loads while this link's hits run
         if (b + (int)gridDim.x < n_ctas) take_item(b + gridDim.x);
         if (this_live) {
-            accepted = visit_ordered<K>(u, sa, beta3, angle, key, tr);
+            if (DRAWN) {   // the rows in memory, next to the accumulator
+                const Col<T> rows = column_of(s1.f[1]);
+#pragma unroll
+                for (int e = 0; e < 9; ++e) rows.put(e, u.e[e / 3][e % 3]);
+                accepted = visit_drawn<K>(rows, sa, beta3, angle, key);
+                u = staged_link(s1.f[1]);
+            } else {
+                accepted = visit_ordered<K>(u, sa, beta3, angle, key, tr);
+            }
 #pragma unroll
             for (int e = 0; e < 9; ++e)
                 dst[(int64_t)e * this_volume] = make_double2(u.e[e / 3][e % 3].re, u.e[e / 3][e % 3].im);
@@ -951,8 +755,6 @@ k_su3_metropolis_ring(const ChainInfo *__restrict__ chains, const Tile *__restri
 }
 
 
-constexpr size_t kStageBytes = 27 * T * sizeof(double2);   // three staged factors per thread
-
 constexpr size_t kRingBytes = (size_t)kRingBuffers * 9 * T * sizeof(double2);
 
 // Two resident CTAs per SM walk all work items.
@@ -971,25 +773,13 @@ unsigned ring_grid(int64_t ctas) {
 // Both launchers take the handle's sweep layout: work items of 2^log2
 // sites, chain order or by descending chain volume (all layouts give the
 // same bits).
-template <int K>
-void metro_launch_ordered(ym_ensemble *e, int parity, int mu, double angle, int reverse) {
+template <int K, bool DRAWN>
+void metro_launch_ring(ym_ensemble *e, int parity, int mu, double angle, int reverse) {
     const SweepLayout &L = e->layouts[e->sweep_layout];
     const dim3 grid(ring_grid(L.ctas)), block(T);
-    k_su3_metropolis_ring<K, false><<<grid, block, kRingBytes, e->stream>>>(
+    k_su3_metropolis_ring<K, false, DRAWN><<<grid, block, kRingBytes, e->stream>>>(
         e->d_chains, L.d_items, (int)L.ctas, e->d_links, parity, mu, angle, e->d_sweep, e->d_accepts, L.log2_item,
         reverse, nullptr);
-}
-
-void metro_launch_drawn(ym_ensemble *e, int parity, int mu, double angle, int reverse) {
-    const SweepLayout &L = e->layouts[e->sweep_layout];
-    const dim3 grid((unsigned)L.ctas), block(T);
-    const Tile *items = L.d_items;
-    switch (mu) {
-    case 0: k_su3_metropolis<0><<<grid, block, kStageBytes, e->stream>>>(e->d_chains, items, e->d_links, parity, angle, 1, e->d_sweep, e->d_accepts, L.log2_item, reverse); break;
-    case 1: k_su3_metropolis<1><<<grid, block, kStageBytes, e->stream>>>(e->d_chains, items, e->d_links, parity, angle, 1, e->d_sweep, e->d_accepts, L.log2_item, reverse); break;
-    case 2: k_su3_metropolis<2><<<grid, block, kStageBytes, e->stream>>>(e->d_chains, items, e->d_links, parity, angle, 1, e->d_sweep, e->d_accepts, L.log2_item, reverse); break;
-    default: k_su3_metropolis<3><<<grid, block, kStageBytes, e->stream>>>(e->d_chains, items, e->d_links, parity, angle, 1, e->d_sweep, e->d_accepts, L.log2_item, reverse); break;
-    }
 }
 
 // The last sub-sweep of a sweep (parity 1, direction 3, ordered hits) with
@@ -1000,7 +790,7 @@ void metro_launch_measure(ym_ensemble *e, int mu, double angle, double *tr_parti
     const SweepLayout &L = e->layouts[e->sweep_layout];
     const dim3 g(ring_grid(L.ctas)), b(T);
     const int rev = (1 * 4 + mu) & 1;   // the tile order tiled_launch gives (parity 1, mu)
-    k_su3_metropolis_ring<K, true><<<g, b, kRingBytes, e->stream>>>(
+    k_su3_metropolis_ring<K, true, false><<<g, b, kRingBytes, e->stream>>>(
         e->d_chains, L.d_items, (int)L.ctas, e->d_links, 1, mu, angle, e->d_sweep, e->d_accepts, L.log2_item, rev,
         tr_partial);
 }
@@ -1019,13 +809,13 @@ cudaError_t configure_kernels() {
     cudaError_t err = cudaGetDevice(&dev);
     if (err != cudaSuccess) return err;
     if (configured_device != dev) {
-        const void *drawn[4] = {(const void *)k_su3_metropolis<0>, (const void *)k_su3_metropolis<1>,
-                                (const void *)k_su3_metropolis<2>, (const void *)k_su3_metropolis<3>};
-        const void *ordered[4] = {(const void *)k_su3_metropolis_ring<11, false>, (const void *)k_su3_metropolis_ring<14, false>,
-                                  (const void *)k_su3_metropolis_ring<11, true>, (const void *)k_su3_metropolis_ring<14, true>};
-        for (const void *f : drawn)
-            if ((err = set_smem(f, kStageBytes)) != cudaSuccess) return err;
-        for (const void *f : ordered)
+        const void *ring[6] = {(const void *)k_su3_metropolis_ring<11, false, false>,
+                               (const void *)k_su3_metropolis_ring<14, false, false>,
+                               (const void *)k_su3_metropolis_ring<11, true, false>,
+                               (const void *)k_su3_metropolis_ring<14, true, false>,
+                               (const void *)k_su3_metropolis_ring<11, false, true>,
+                               (const void *)k_su3_metropolis_ring<14, false, true>};
+        for (const void *f : ring)
             if ((err = set_smem(f, kRingBytes)) != cudaSuccess) return err;
         configured_device = dev;
     }
@@ -1042,9 +832,10 @@ cudaError_t tiled_launch(ym_ensemble *e, int parity, int mu, double angle, int u
     // one touched last and finds its first waves' staple links in L2.  The
     // links of one sub-sweep are independent, so the order changes no bit.
     const int reverse = (parity * 4 + mu) & 1;
-    if (uniform) metro_launch_drawn(e, parity, mu, angle, reverse);
-    else if (angle <= 0.3) metro_launch_ordered<11>(e, parity, mu, angle, reverse);
-    else metro_launch_ordered<14>(e, parity, mu, angle, reverse);
+    if (uniform && angle <= 0.3) metro_launch_ring<11, true>(e, parity, mu, angle, reverse);
+    else if (uniform) metro_launch_ring<14, true>(e, parity, mu, angle, reverse);
+    else if (angle <= 0.3) metro_launch_ring<11, false>(e, parity, mu, angle, reverse);
+    else metro_launch_ring<14, false>(e, parity, mu, angle, reverse);
     return cudaGetLastError();
 }
 
