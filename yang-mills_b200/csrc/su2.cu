@@ -36,20 +36,23 @@ __device__ __forceinline__ void su2_staple(const double2 *__restrict__ links, co
     comp[0] = comp[1] = comp[2] = comp[3] = 0.0;
     const Nb self{x.lex, par};
     const Nb pm = step(c, x.x, x.lex, par, MU, +1);
-#pragma unroll
-    for (int nu = 0; nu < 4; ++nu) {
-        if (nu == MU) continue;
-        const Nb pn = step(c, x.x, x.lex, par, nu, +1);
-        const Nb mn = step(c, x.x, x.lex, par, nu, -1);
+    // one direction's forward and backward term at a time, side by side
+#pragma unroll 1
+    for (int i = 0; i < 3; ++i) {
+        const int nu = i + (i >= MU ? 1 : 0);
+        const Nb pn = step_any(c, x.x, x.lex, par, nu, +1);
+        const Nb mn = step_any(c, x.x, x.lex, par, nu, -1);
         const Nb mnpm = step(c, x.x, mn.lex, mn.par, MU, +1);
-        const q4 fwd = qmul(qmul(link_q(links, c, pm, nu), qdag(link_q(links, c, pn, MU))),
-                            qdag(link_q(links, c, self, nu)));
-        const q4 bwd = qmul(qmul(qdag(link_q(links, c, mnpm, nu)), qdag(link_q(links, c, mn, MU))),
-                            link_q(links, c, mn, nu));
+        const q4 first[2] = {link_q(links, c, pm, nu), qdag(link_q(links, c, mnpm, nu))};
+        const q4 second[2] = {qdag(link_q(links, c, pn, MU)), qdag(link_q(links, c, mn, MU))};
+        const q4 third[2] = {qdag(link_q(links, c, self, nu)), link_q(links, c, mn, nu)};
+        q4 p[2], t[2];
+        qmul_many<2>(first, second, p);
+        qmul_many<2>(p, third, t);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) comp[i] += fwd.c[i];
+        for (int m = 0; m < 2; ++m)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) comp[i] += bwd.c[i];
+            for (int k = 0; k < 4; ++k) comp[k] += t[m].c[k];
     }
 }
 
@@ -112,14 +115,19 @@ __device__ __forceinline__ double staple_norm(const double comp[4]) {
 }
 
 // The reference sampler (su2_ensemble.rs:220-254) on the link's stream:
-// words 2k, 2k+1 for attempt k+1, then two for the S^2 direction.
+// words 2k, 2k+1 for attempt k+1, then two for the S^2 direction.  The
+// direction is drawn after the attempt loop, where the warp has met again:
+// inside it, each attempt that some lane accepts would run it once more for
+// the whole warp (a warp needs four or five attempts).
 __device__ __forceinline__ bool sample_reference(double alpha, uint64_t key, int max_attempts,
                                                  q4 &out, int &attempts) {
     uint64_t j = 0;
     const double mass = alpha <= kAlphaZeroLimit ? 0.0 : -expm1(-2.0 * alpha);
-    for (int a = 1; a <= max_attempts; ++a) {
+    double r0 = 0.0, radial = 0.0;
+    bool found = false;
+    int a = 1;
+    for (; a <= max_attempts; ++a) {
         const double pu = unit_from(splitmix_at(key, j++));
-        double r0;
         if (alpha <= kAlphaZeroLimit) {
             r0 = 2.0 * pu - 1.0;
         } else {
@@ -127,58 +135,75 @@ __device__ __forceinline__ bool sample_reference(double alpha, uint64_t key, int
             r0 = 1.0 - y;
             r0 = r0 < -1.0 ? -1.0 : (r0 > 1.0 ? 1.0 : r0);
         }
-        const double radial = sqrt(fmax(1.0 - r0 * r0, 0.0));
+        radial = sqrt(fmax(1.0 - r0 * r0, 0.0));
         if (unit_from(splitmix_at(key, j++)) <= radial) {
-            const double z = 2.0 * unit_from(splitmix_at(key, j++)) - 1.0;
-            const double phi = kTau * unit_from(splitmix_at(key, j++));
-            const double planar = sqrt(fmax(1.0 - z * z, 0.0));
-            const double v[4] = {r0, radial * (planar * cos(phi)), radial * (planar * sin(phi)),
-                                 radial * z};
-            if (!normalize_scaled<4>(v, out.c)) return false;
-            attempts = a;
-            return true;
+            found = true;
+            break;
         }
     }
-    attempts = max_attempts;
-    return false;
+    attempts = found ? a : max_attempts;
+    if (!found) return false;
+    const double z = 2.0 * unit_from(splitmix_at(key, j)) - 1.0;
+    const double phi = kTau * unit_from(splitmix_at(key, j + 1));
+    const double planar = sqrt(fmax(1.0 - z * z, 0.0));
+    const double v[4] = {r0, radial * (planar * cos(phi)), radial * (planar * sin(phi)), radial * z};
+    if (!normalize_scaled<4>(v, out.c)) {
+        attempts = 0;
+        return false;
+    }
+    return true;
 }
 
 // Kennedy-Pendleton (Phys. Lett. B 156 (1985) 393) for the same density
 // exp(alpha r0) sqrt(1 - r0^2): x = -(ln u1 + cos^2(2 pi u2) ln u3)/alpha,
-// accept if u4^2 <= 1 - x/2, r0 = 1 - x.  Uniforms in (0, 1].
+// accept if u4^2 <= 1 - x/2, r0 = 1 - x.  Uniforms in (0, 1].  The direction
+// after the loop, as above.
 __device__ __forceinline__ bool sample_kp(double alpha, uint64_t key, int max_attempts, q4 &out,
                                           int &attempts) {
     uint64_t j = 0;
     if (alpha <= kAlphaZeroLimit) return sample_reference(alpha, key, max_attempts, out, attempts);
-    for (int a = 1; a <= max_attempts; ++a) {
+    double x = 0.0;
+    bool found = false;
+    int a = 1;
+    for (; a <= max_attempts; ++a) {
         const double u1 = 1.0 - unit_from(splitmix_at(key, j++));
         const double u2 = unit_from(splitmix_at(key, j++));
         const double u3 = 1.0 - unit_from(splitmix_at(key, j++));
         const double u4 = unit_from(splitmix_at(key, j++));
         const double cs = cospi(2.0 * u2);
-        const double x = -(log(u1) + cs * cs * log(u3)) / alpha;
+        x = -(log(u1) + cs * cs * log(u3)) / alpha;
         if (u4 * u4 <= 1.0 - 0.5 * x) {
-            const double r0 = 1.0 - x;
-            const double radial = sqrt(fmax(1.0 - r0 * r0, 0.0));
-            const double z = 2.0 * unit_from(splitmix_at(key, j++)) - 1.0;
-            double sn, cn;
-            sincospi(2.0 * unit_from(splitmix_at(key, j++)), &sn, &cn);
-            const double planar = sqrt(fmax(1.0 - z * z, 0.0));
-            const double v[4] = {r0, radial * (planar * cn), radial * (planar * sn), radial * z};
-            if (!normalize_scaled<4>(v, out.c)) return false;
-            attempts = a;
-            return true;
+            found = true;
+            break;
         }
     }
-    attempts = max_attempts;
-    return false;
+    attempts = found ? a : max_attempts;
+    if (!found) return false;
+    const double r0 = 1.0 - x;
+    const double radial = sqrt(fmax(1.0 - r0 * r0, 0.0));
+    const double z = 2.0 * unit_from(splitmix_at(key, j)) - 1.0;
+    double sn, cn;
+    sincospi(2.0 * unit_from(splitmix_at(key, j + 1)), &sn, &cn);
+    const double planar = sqrt(fmax(1.0 - z * z, 0.0));
+    const double v[4] = {r0, radial * (planar * cn), radial * (planar * sn), radial * z};
+    if (!normalize_scaled<4>(v, out.c)) {
+        attempts = 0;
+        return false;
+    }
+    return true;
 }
 
 // Error flag bits.
 constexpr unsigned kErrAttempts = 1u;
 constexpr unsigned kErrNonFinite = 2u;
 
-// One thread per link (large sub-sweeps, throughput-bound).
+// One thread per link (large sub-sweeps).  What bounds it: binary64 latency
+// and issue of the normalised products.  24^4, per launch under the profiler:
+// overrelaxation 48 us with plain divisions and one product at a time, 34 us
+// with shared reciprocals and a direction's two terms side by side (binary64
+// pipe 36 -> 47 %); heat-bath 75 us to 66, and with the direction drawn after
+// the attempt loop a sweep of one heat-bath and one overrelaxation went from
+// 758 to 721 us live (918 at first).
 template <int MU>
 __global__ void __launch_bounds__(T)
 k_su2_heatbath_thread(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles,
@@ -337,19 +362,25 @@ k_su2_plaquette(const ChainInfo *__restrict__ chains, const Tile *__restrict__ t
     if (s < c.volume) {
         const Coord x = decode_storage(c, s);
         const Nb self{x.lex, x.par};
-        bool first = true;
+        // planes (0,1),(0,2) then (0,3),(1,2) then (1,3),(2,3), side by side
 #pragma unroll 1
-        for (int mu = 0; mu < 3; ++mu) {
-            const Nb pm = step(c, x.x, x.lex, x.par, mu, +1);
-#pragma unroll 1
-            for (int nu = mu + 1; nu < 4; ++nu) {
-                const Nb pn = step(c, x.x, x.lex, x.par, nu, +1);
-                q4 p = qmul(link_q(links, c, self, mu), link_q(links, c, pm, nu));
-                p = qmul(p, qdag(link_q(links, c, pn, mu)));
-                p = qmul(p, qdag(link_q(links, c, self, nu)));
-                v = first ? p.c[0] : v + p.c[0];
-                first = false;
+        for (int k = 0; k < 3; ++k) {
+            const int mu[2] = {k < 2 ? 0 : 1, k == 0 ? 0 : k}, nu[2] = {k == 0 ? 1 : 3, k < 2 ? 2 : 3};
+            q4 a[2], b[2], d[2], e[2];
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                const Nb pm = step_any(c, x.x, x.lex, x.par, mu[m], +1);
+                const Nb pn = step_any(c, x.x, x.lex, x.par, nu[m], +1);
+                a[m] = link_q(links, c, self, mu[m]);
+                b[m] = link_q(links, c, pm, nu[m]);
+                d[m] = qdag(link_q(links, c, pn, mu[m]));
+                e[m] = qdag(link_q(links, c, self, nu[m]));
             }
+            qmul_many<2>(a, b, a);
+            qmul_many<2>(a, d, a);
+            qmul_many<2>(a, e, a);
+            v = k == 0 ? a[0].c[0] : v + a[0].c[0];
+            v = v + a[1].c[0];
         }
     }
 #pragma unroll
