@@ -37,8 +37,12 @@ constexpr uint64_t kWaitNs = 200000000ull;  // 0.2 s per MMA group
 constexpr unsigned kErrWait = 1u;
 
 // Shared-memory layouts (bytes from the 1024-aligned base).
+// The sub-sweep keeps each thread's staple sum and link rows (nine float2
+// each) where the activations were, once the last MMA group has read them.
+constexpr uint32_t kHitBytes = 18 * kRows * sizeof(float2);
 struct FwdLayout {   // forward-only kernels: H2 overwrites H1
-    static constexpr uint32_t X = kImageBytes, H1 = X + kTileX, H2 = H1, BIAS = H1 + kTileH,
+    static constexpr uint32_t X = kImageBytes, H1 = X + kTileX, H2 = H1,
+                              BIAS = H1 + (kHitBytes > kTileH ? kHitBytes : kTileH),
                               MBAR = BIAS + 144 * 4, SLOT = MBAR + 8, BYTES = SLOT + 56;
 };
 struct GradLayout {
@@ -627,11 +631,22 @@ k_lp_sweep(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles,
         if (!ok) break;   // block-uniform: the wait gave up and set the error bit
         unsigned accepted = 0;
         if (valid) {
-            float cum[7], scale;
-            proposal_from(y, cum, scale);
+            DrawLearned draw;
+            float scale;
+            proposal_from(y, draw.cum, scale);
             m3f u = load_f(links, c, s, MU);
             const uint64_t key = link_key(c.seed, sweep, x.lex, MU);
-            accepted = visit_learned_f(u, a, c.beta / 3.0, cum, scale, key);
+            // the staple and the rows in the activation tiles' memory, free
+            // since the last MMA group was waited for
+            float2 (*own)[kRows] = reinterpret_cast<float2 (*)[kRows]>(sm + L::H1);
+            const StapleColF<kRows> sa{own};
+            const RowCol<kRows> rows{own + 9};
+            put_staple(sa, a);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) rows.put_row(i, u.e[i]);
+            accepted = visit_drawn_f(rows, sa, c.beta / 3.0, (double)scale, key, draw);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) rows.row(i, u.e[i]);
             store_f(links, c, s, MU, u);
         }
         const unsigned warp_sum = __reduce_add_sync(0xffffffffu, accepted);

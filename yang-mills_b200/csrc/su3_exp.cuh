@@ -127,4 +127,29 @@ __device__ __forceinline__ m3 generator_rotation_dense(int g, double theta) {
     return r;
 }
 
+// The decision u < exp(-m), m = max(dS, 0), taken as m < -log u in binary32
+// away from equality.  neg_log_unit's error: the word's 32 high bits give u
+// to 2^-32, so log u to 2^-16 = 1.53e-5 for u >= 2^-16 (smaller u, one in
+// 65,536, return NaN: never sure); __logf adds at most 3.6e-7 on [0.5, 2] and
+// 3 ulp, 2.9e-6, down to log 2^-16 = -11.1; rounding m to binary32 7e-7.
+// Together below kLogBand, so every decision outside the band is
+// that test's; one inside (one in a few thousand) evaluates it.
+constexpr float kLogBand = 2.5e-5f;
+
+__device__ __forceinline__ float neg_log_unit(uint64_t w) {
+    const uint32_t hi = (uint32_t)(w >> 32);
+    const float l = -__logf((float)hi * 0x1p-32f);
+    return hi < 65536u ? __int_as_float(0x7fffffff) : l;
+}
+
+__device__ __forceinline__ bool accept_log(double ds, float logu, uint64_t key, int h) {
+    const float d = fmaxf((float)ds, 0.0f) - logu;
+    bool acc = d < 0.0f;
+    if (!(fabsf(d) > kLogBand)) acc = unit_from(splitmix_at(key, (uint64_t)(2 * h + 1))) < exp(-fmax(ds, 0.0));
+    return acc;
+}
+
+// The stream's next word (state starts at the link's key).
+__device__ __forceinline__ uint64_t next_word(uint64_t &state) { return mix64(state += kGolden); }
+
 }  // namespace ym

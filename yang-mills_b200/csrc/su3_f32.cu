@@ -31,27 +31,55 @@ using namespace f32;
 #define YM_F32_MIN_BLOCKS 4
 #endif
 
-template <int MU>
+// Shared memory of a block: two sets of three staged factors.
+constexpr size_t kRingF = (size_t)36 * T * sizeof(float2);
+
+// What bounds it: instruction issue (63 % of cycles; 16 warps per SM).  The
+// staple is one looped copy for all directions with its factors two terms
+// ahead; the ordered hits stay unrolled (looped: 32^4 839 against 811 us per
+// sweep, 4 x 16^4 224 against 209), the drawn ones loop on rows in memory.
+// Per sweep, before (compile-time directions, one term ahead, exp in every
+// decision, the staple converted and picked by selects in every hit) and
+// after: 32^4 ordered 992 -> 811 us, drawn 1202 -> 1055; 4 x 16^4 ordered
+// 237 -> 209, drawn 320 -> 280; 16^4 drawn 118 -> 109.  Persistent blocks
+// with the next tile's first term under the hits were slower here (32^4
+// drawn 1093, 4 x 16^4 drawn 315 us: the static split of 1.7 tiles per block
+// leaves SMs idle), as were three or five blocks per SM.
+template <bool DRAWN>
 __global__ void __launch_bounds__(T, YM_F32_MIN_BLOCKS)
 k_f32_metropolis(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles,
-                 float2 *__restrict__ links, int parity, double angle, int uniform,
+                 float2 *__restrict__ links, int parity, int mu, double angle,
                  const uint64_t *__restrict__ sweep_ptr, unsigned long long *__restrict__ accepts,
                  int reverse) {
-    __shared__ __align__(16) float2 stage[18][T];   // 18 KB: three staged factors
-    const StageF<T> bufs{stage, stage + 6, stage + 12};
+    extern __shared__ __align__(16) float2 ring_mem[];
+    auto buf = [&](int i) { return reinterpret_cast<float2 (*)[T]>(ring_mem + (size_t)i * 6 * T); };
+    const SetF<T> s0{{buf(0), buf(1), buf(2)}}, s1{{buf(3), buf(4), buf(5)}};
     const Tile tile = tiles[reverse ? gridDim.x - 1 - blockIdx.x : blockIdx.x];
     const ChainInfo c = chains[tile.chain];
     const int64_t t = tile.start + threadIdx.x;
     const uint64_t sweep = *sweep_ptr;
     unsigned accepted = 0;
     if (t < c.half) {
-        const int64_t s = (int64_t)parity * c.half + t;
-        const Coord x = decode_storage(c, s);
-        const m3f a = staple_f_staged<MU>(links, c, x, parity, bufs);
-        m3f u = load_f(links, c, s, MU);
-        const uint64_t key = link_key(c.seed, sweep, x.lex, MU);
-        accepted = visit_f(u, a, c.beta / 3.0, angle, key, uniform);
-        store_f(links, c, s, MU, u);
+        const Site x = site_of(c, decode_storage(c, (int64_t)parity * c.half + t));
+        const float2 *base = links + c.offset;
+        stage_term_f<false>(s0, base, c.volume, x, parity, mu, mu == 0 ? 1 : 0);
+        const m3f sum = staple_ring_f(base, c.volume, x, parity, mu, s0, s1);
+        m3f u = staged_f(s0.f[0]);
+        // the sum goes, in binary64, to this thread's slots of the second set
+        const StapleCol<T> a{reinterpret_cast<double (*)[T]>(ring_mem + (size_t)18 * T)};
+        put_staple(a, sum);
+        const uint64_t key = link_key(c.seed, sweep, x.lex, mu);
+        if (DRAWN) {
+            const RowCol<T> rows{reinterpret_cast<float2 (*)[T]>(ring_mem)};   // and the rows to the first set's
+#pragma unroll
+            for (int i = 0; i < 3; ++i) rows.put_row(i, u.e[i]);
+            accepted = visit_drawn_f(rows, a, c.beta / 3.0, angle, key, DrawUniform{});
+#pragma unroll
+            for (int i = 0; i < 2; ++i) rows.row(i, u.e[i]);
+        } else {
+            accepted = visit_ordered_f(u, a, c.beta / 3.0, angle, key);
+        }
+        store_f(links, c, (int64_t)parity * c.half + t, mu, u);
     }
     const unsigned warp_sum = __reduce_add_sync(0xffffffffu, accepted);
     if ((threadIdx.x & 31) == 0 && warp_sum)
@@ -113,8 +141,8 @@ k_f32_plaquette(const ChainInfo *__restrict__ chains, const Tile *__restrict__ t
 #pragma unroll 1
             for (int nu = mu + 1; nu < 4; ++nu) {
                 const Nb pn = step(c, x.x, x.lex, x.par, nu, +1);
-                m3 p = mul(umu, load_as_f64(links, c, storage_index(c, pm.lex, pm.par), nu));
-                p = mul_adj(p, load_as_f64(links, c, storage_index(c, pn.lex, pn.par), mu));
+                m3 p = mul_fma(umu, load_as_f64(links, c, storage_index(c, pm.lex, pm.par), nu));
+                p = mul_adj_fma(p, load_as_f64(links, c, storage_index(c, pn.lex, pn.par), mu));
                 const double val = retrace_mul_adj(p, load_as_f64(links, c, s, nu)) / 3.0;
                 v = first ? val : v + val;
                 first = false;
@@ -237,19 +265,19 @@ float2 *f32_links(ym_ensemble *e) { return reinterpret_cast<float2 *>(e->d_links
 
 }  // namespace
 
+template <bool DRAWN>
+static cudaError_t launch_f32_form(ym_ensemble *e, int parity, int mu, double angle, int reverse) {
+    k_f32_metropolis<DRAWN><<<(unsigned)e->n_half_tiles, T, kRingF, e->stream>>>(
+        e->d_chains, e->d_half_tiles, f32_links(e), parity, mu, angle, e->d_sweep, e->d_accepts, reverse);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_f32_metropolis(ym_ensemble *e, int parity, int mu, double angle, int uniform) {
-    const dim3 g((unsigned)e->n_half_tiles), b(T);
-    float2 *l = f32_links(e);
     // consecutive sub-sweeps in opposite tile orders (each starts on the
     // links the previous one left in L2; the order changes no bit)
     const int reverse = (parity * 4 + mu) & 1;
-    switch (mu) {
-    case 0: k_f32_metropolis<0><<<g, b, 0, e->stream>>>(e->d_chains, e->d_half_tiles, l, parity, angle, uniform, e->d_sweep, e->d_accepts, reverse); break;
-    case 1: k_f32_metropolis<1><<<g, b, 0, e->stream>>>(e->d_chains, e->d_half_tiles, l, parity, angle, uniform, e->d_sweep, e->d_accepts, reverse); break;
-    case 2: k_f32_metropolis<2><<<g, b, 0, e->stream>>>(e->d_chains, e->d_half_tiles, l, parity, angle, uniform, e->d_sweep, e->d_accepts, reverse); break;
-    default: k_f32_metropolis<3><<<g, b, 0, e->stream>>>(e->d_chains, e->d_half_tiles, l, parity, angle, uniform, e->d_sweep, e->d_accepts, reverse); break;
-    }
-    return cudaGetLastError();
+    return uniform ? launch_f32_form<true>(e, parity, mu, angle, reverse)
+                   : launch_f32_form<false>(e, parity, mu, angle, reverse);
 }
 
 cudaError_t launch_f32_reunitarize(ym_ensemble *e) {

@@ -48,13 +48,13 @@ __device__ __forceinline__ m3 resident_link(const double2 *p, int v) {
 // a += the staple term (nu, BWD) of link (x, mu): the products of
 // tiled_exact::term_accumulate on links read in place.
 template <bool BWD>
-__device__ __forceinline__ void resident_term(const double2 *sl, int v, const tiled_exact::Site &x, int par, int mu,
+__device__ __forceinline__ void resident_term(const double2 *sl, int v, const Site &x, int par, int mu,
                                               int nu, m3 &a) {
     const int same = par ? x.half : 0, other = par ? 0 : x.half;
-    const int o = BWD ? x.lex + tiled_exact::pick(x.bwd, nu) : x.lex;
+    const int o = BWD ? x.lex + pick(x.bwd, nu) : x.lex;
     const double2 *ln = sl + nu * 9 * v, *lm = sl + mu * 9 * v;
-    const int i1 = (BWD ? same : other) + ((o + tiled_exact::pick(x.fwd, mu)) >> 1);
-    const int i2 = other + ((BWD ? o : x.lex + tiled_exact::pick(x.fwd, nu)) >> 1);
+    const int i1 = (BWD ? same : other) + ((o + pick(x.fwd, mu)) >> 1);
+    const int i2 = other + ((BWD ? o : x.lex + pick(x.fwd, nu)) >> 1);
     const int i3 = BWD ? i2 : same + (x.lex >> 1);
     m3 p;
     {

@@ -165,28 +165,6 @@ __device__ __forceinline__ void lambda8_fixed(double theta, cplx &e1, cplx &e2) 
     e2 = sq ? q2 : e2;
 }
 
-// The decision u < exp(-m), m = max(dS, 0), taken as m < -log u in binary32
-// away from equality.  neg_log_unit's error: the word's 32 high bits give u
-// to 2^-32, so log u to 2^-16 = 1.53e-5 for u >= 2^-16 (smaller u, one in
-// 65,536, return NaN: never sure); __logf adds at most 3.6e-7 on [0.5, 2] and
-// 3 ulp, 2.9e-6, down to log 2^-16 = -11.1; rounding m to binary32 7e-7.
-// Together below kLogBand, so every decision outside the band is
-// that test's; one inside (one in a few thousand) evaluates it.
-constexpr float kLogBand = 2.5e-5f;
-
-__device__ __forceinline__ float neg_log_unit(uint64_t w) {
-    const uint32_t hi = (uint32_t)(w >> 32);
-    const float l = -__logf((float)hi * 0x1p-32f);
-    return hi < 65536u ? __int_as_float(0x7fffffff) : l;
-}
-
-__device__ __forceinline__ bool accept_log(double ds, float logu, uint64_t key, int h) {
-    const float d = fmaxf((float)ds, 0.0f) - logu;
-    bool acc = d < 0.0f;
-    if (!(fabsf(d) > kLogBand)) acc = unit_from(splitmix_at(key, (uint64_t)(2 * h + 1))) < exp(-fmax(ds, 0.0));
-    return acc;
-}
-
 // Rotation entries of a hit: the reference's bits (taylor_fixed,
 // lambda8_fixed), or in the fast form cos_sin_horner for both generators'
 // phases (lambda8's two directly, without halving and squaring).
@@ -220,9 +198,6 @@ struct DiagPre {
     cplx e1, e2;
     float logu;
 };
-
-// The stream's next word (state starts at the link's key).
-__device__ __forceinline__ uint64_t next_word(uint64_t &state) { return mix64(state += kGolden); }
 
 template <int K>
 __device__ __forceinline__ BlockPre pre_block(uint64_t &state, double angle) {
@@ -517,33 +492,6 @@ __device__ __forceinline__ unsigned visit_drawn(const U &u, const A &a, double b
 struct TermSet {
     double2 (*f[3])[T];
 };
-
-// A link's site within its chain and the steps to its neighbours, in
-// lexicographic positions.  Sweeps need even extents, so every step changes
-// the parity; 32 bits hold any site (a lattice of 2^31 sites takes 1.2 TB).
-struct Site {
-    int32_t lex, half;
-    int32_t fwd[4], bwd[4];
-};
-
-__device__ __forceinline__ Site site_of(const ChainInfo &c, const Coord &x) {
-    Site k;
-    k.lex = (int32_t)x.lex;
-    k.half = (int32_t)c.half;
-    int32_t st = 1;
-#pragma unroll
-    for (int d = 3; d >= 0; --d) {
-        const int32_t span = c.n[d] * st;
-        k.fwd[d] = x.x[d] == c.n[d] - 1 ? st - span : st;
-        k.bwd[d] = x.x[d] == 0 ? span - st : -st;
-        st = span;
-    }
-    return k;
-}
-
-__device__ __forceinline__ int32_t pick(const int32_t *v, int d) {
-    return d == 0 ? v[0] : (d == 1 ? v[1] : (d == 2 ? v[2] : v[3]));
-}
 
 // The three factors of staple term (nu, BWD) of link (x, mu):
 //   forward  U_nu(x+mu), U_mu(x+nu), U_nu(x)

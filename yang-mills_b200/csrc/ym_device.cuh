@@ -394,6 +394,33 @@ __device__ __forceinline__ Nb step_any(const ChainInfo &c, const int32_t *x, int
     return Nb{nl, par ^ flip};
 }
 
+// A link's site within its chain and the steps to its neighbours, in
+// lexicographic positions.  Sweeps need even extents, so every step changes
+// the parity; 32 bits hold any site (a lattice of 2^31 sites takes 1.2 TB).
+struct Site {
+    int32_t lex, half;
+    int32_t fwd[4], bwd[4];
+};
+
+__device__ __forceinline__ Site site_of(const ChainInfo &c, const Coord &x) {
+    Site k;
+    k.lex = (int32_t)x.lex;
+    k.half = (int32_t)c.half;
+    int32_t st = 1;
+#pragma unroll
+    for (int d = 3; d >= 0; --d) {
+        const int32_t span = c.n[d] * st;
+        k.fwd[d] = x.x[d] == c.n[d] - 1 ? st - span : st;
+        k.bwd[d] = x.x[d] == 0 ? span - st : -st;
+        st = span;
+    }
+    return k;
+}
+
+__device__ __forceinline__ int32_t pick(const int32_t *v, int d) {
+    return d == 0 ? v[0] : (d == 1 ? v[1] : (d == 2 ? v[2] : v[3]));
+}
+
 // SU(3) FP64 link access: plane (mu*9 + entry) of a chain's block.
 __device__ __forceinline__ m3 load_su3(const double2 *__restrict__ links, const ChainInfo &c,
                                        int64_t s, int mu) {
