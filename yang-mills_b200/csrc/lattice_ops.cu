@@ -49,7 +49,7 @@ constexpr unsigned kQNonFiniteAction = 16u;
 // reference's order of checks.
 __device__ __forceinline__ unsigned su3_gate(const m3 &u) {
     if (!finite3(u)) return kQNonFiniteMatrix;
-    if (unitarity_res2(u) > kSu3Tol * kSu3Tol) return kQNonUnitary;
+    if (!unitary_within(u)) return kQNonUnitary;
     if (norm2(csub(det3(u), cmake(1.0, 0.0))) > kSu3Tol * kSu3Tol) return kQDeterminant;
     return 0u;
 }

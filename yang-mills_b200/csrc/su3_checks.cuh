@@ -76,29 +76,43 @@ __device__ __forceinline__ cplx det3(const m3 &m) {
     return cadd(csub(t1, t2), t3);
 }
 
-// Square of Mat3::unitarity_residual (su3.rs:219-223): max |U^dag U - 1|^2
-// and |U U^dag - 1|^2 over all entries.  Both products are Hermitian, so
+// max |entry|^2 of u u^dag - 1 (ROWS) or u^dag u - 1.  Both are Hermitian, so
 // the upper triangle (diagonal included) carries every distinct magnitude;
-// only those six entries of each are formed.
-__device__ __forceinline__ double unitarity_res2(const m3 &u) {
+// only those six entries are formed.
+template <bool ROWS>
+__device__ __forceinline__ double gram_res2(const m3 &u) {
     double r = 0.0;
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const double dl = norm2(u.e[0][i]) + norm2(u.e[1][i]) + norm2(u.e[2][i]) - 1.0;
-        const double dr = norm2(u.e[i][0]) + norm2(u.e[i][1]) + norm2(u.e[i][2]) - 1.0;
-        r = fmax(r, fmax(dl * dl, dr * dr));
+    for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int j = i + 1; j < 3; ++j) {
-            cplx l = cmul(cconj(u.e[0][i]), u.e[0][j]);
-            l = cadd(l, cmul(cconj(u.e[1][i]), u.e[1][j]));
-            l = cadd(l, cmul(cconj(u.e[2][i]), u.e[2][j]));
-            cplx g = cmul(u.e[i][0], cconj(u.e[j][0]));
-            g = cadd(g, cmul(u.e[i][1], cconj(u.e[j][1])));
-            g = cadd(g, cmul(u.e[i][2], cconj(u.e[j][2])));
-            r = fmax(r, fmax(norm2(l), norm2(g)));
+        for (int j = i; j < 3; ++j) {
+            cplx g = cmake(i == j ? -1.0 : 0.0, 0.0);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                if (i == j) {
+                    const cplx z = ROWS ? u.e[i][k] : u.e[k][i];
+                    g.re = fma(z.re, z.re, g.re);
+                    g.re = fma(z.im, z.im, g.re);
+                } else if (ROWS) {
+                    cfma(g, u.e[i][k], cconj(u.e[j][k]));
+                } else {
+                    cfma(g, cconj(u.e[k][i]), u.e[k][j]);
+                }
+            }
+            r = fmax(r, i == j ? g.re * g.re : norm2(g));
         }
-    }
     return r;
+}
+
+// Whether Mat3::unitarity_residual (su3.rs:219-223), the larger of
+// max |U U^dag - 1| and max |U^dag U - 1|, is at most kSu3Tol.  The two
+// deviations have the same singular values, so the largest entry of one is
+// at most their common Frobenius norm, at most three times the largest entry
+// of the other: below a quarter of the tolerance the first decides both.
+__device__ __forceinline__ bool unitary_within(const m3 &u) {
+    const double r = gram_res2<true>(u);
+    if (r <= kSu3Tol * kSu3Tol * (1.0 / 16.0)) return true;
+    return r <= kSu3Tol * kSu3Tol && gram_res2<false>(u) <= kSu3Tol * kSu3Tol;
 }
 
 // Su3::from_checked_matrix gate (su3.rs:20, 241-252): finite, unitarity residual
@@ -106,7 +120,7 @@ __device__ __forceinline__ double unitarity_res2(const m3 &u) {
 // which is the same number (det U^dag is the conjugate of det U).
 __device__ __forceinline__ bool in_su3(const m3 &u) {
     if (!finite3(u)) return false;
-    if (unitarity_res2(u) > kSu3Tol * kSu3Tol) return false;
+    if (!unitary_within(u)) return false;
     return norm2(csub(det3(u), cmake(1.0, 0.0))) <= kSu3Tol * kSu3Tol;
 }
 
