@@ -186,33 +186,37 @@ k_f32_hot_start(const ChainInfo *__restrict__ chains, const Tile *__restrict__ t
 }
 
 // Reference AoS (18 doubles per link) <-> two-row binary32.
-__global__ void k_f32_from_aos(const ChainInfo *__restrict__ chains, int chain, float2 *links,
-                               const double2 *__restrict__ staging) {
+__global__ void __launch_bounds__(kAosThreads)
+k_f32_from_aos(const ChainInfo *__restrict__ chains, int chain, float2 *links, const double2 *__restrict__ staging) {
+    __shared__ AosBlock b;
     const ChainInfo c = chains[chain];
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < c.volume;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        const Coord x = decode_storage(c, s);
-        for (int mu = 0; mu < 4; ++mu) {
-            const double2 *src = staging + (x.lex * 4 + mu) * 9;
-            float2 *dst = links + c.offset + (int64_t)(mu * 6) * c.volume + s;
-            for (int e = 0; e < 6; ++e)
-                dst[(int64_t)e * c.volume] = make_float2((float)src[e].x, (float)src[e].y);
-        }
+    int64_t s;
+    bool live;
+    const int n = aos_sites(c, b, s, live), mu = threadIdx.x >> 5;
+    aos_read(b, n, staging);
+    if (!live) return;
+    float2 *dst = links + c.offset + (int64_t)(mu * 6) * c.volume + s;
+#pragma unroll
+    for (int e = 0; e < 6; ++e) {
+        const double2 v = b.v[threadIdx.x & 31][mu * 9 + e];
+        dst[(int64_t)e * c.volume] = make_float2((float)v.x, (float)v.y);
     }
 }
 
-__global__ void k_f32_to_aos(const ChainInfo *__restrict__ chains, int chain,
-                             const float2 *__restrict__ links, double2 *staging) {
+__global__ void __launch_bounds__(kAosThreads)
+k_f32_to_aos(const ChainInfo *__restrict__ chains, int chain, const float2 *__restrict__ links, double2 *staging) {
+    __shared__ AosBlock b;
     const ChainInfo c = chains[chain];
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < c.volume;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        const Coord x = decode_storage(c, s);
-        for (int mu = 0; mu < 4; ++mu) {
-            const m3 u = load_as_f64(links, c, s, mu);
-            double2 *dst = staging + (x.lex * 4 + mu) * 9;
-            for (int e = 0; e < 9; ++e) dst[e] = make_double2(u.e[e / 3][e % 3].re, u.e[e / 3][e % 3].im);
-        }
+    int64_t s;
+    bool live;
+    const int n = aos_sites(c, b, s, live), mu = threadIdx.x >> 5;
+    if (live) {
+        const m3 u = load_as_f64(links, c, s, mu);
+#pragma unroll
+        for (int e = 0; e < 9; ++e)
+            b.v[threadIdx.x & 31][mu * 9 + e] = make_double2(u.e[e / 3][e % 3].re, u.e[e / 3][e % 3].im);
     }
+    aos_write(b, n, staging);
 }
 
 // One link of a two-row chain as binary64 (the third row rebuilt, as
@@ -311,13 +315,13 @@ cudaError_t launch_f32_hot_start(ym_ensemble *e) {
 }
 
 cudaError_t launch_f32_from_aos(ym_ensemble *e, int64_t chain) {
-    k_f32_from_aos<<<grid_for(e->chains[chain].volume, 128), 128, 0, e->stream>>>(
+    k_f32_from_aos<<<aos_blocks(e->chains[chain].volume), kAosThreads, 0, e->stream>>>(
         e->d_chains, (int)chain, f32_links(e), reinterpret_cast<const double2 *>(e->d_staging));
     return cudaGetLastError();
 }
 
 cudaError_t launch_f32_to_aos(ym_ensemble *e, int64_t chain) {
-    k_f32_to_aos<<<grid_for(e->chains[chain].volume, 128), 128, 0, e->stream>>>(
+    k_f32_to_aos<<<aos_blocks(e->chains[chain].volume), kAosThreads, 0, e->stream>>>(
         e->d_chains, (int)chain, f32_links(e), reinterpret_cast<double2 *>(e->d_staging));
     return cudaGetLastError();
 }

@@ -332,32 +332,33 @@ __global__ void k_su3_identity(const ChainInfo *__restrict__ chains, double2 *li
 }
 
 // staging holds the reference AoS image: link = lex*4+mu, 18 doubles.
-__global__ void k_su3_from_aos(const ChainInfo *__restrict__ chains, int chain, double2 *links,
-                               const double2 *__restrict__ staging) {
+__global__ void __launch_bounds__(kAosThreads)
+k_su3_from_aos(const ChainInfo *__restrict__ chains, int chain, double2 *links, const double2 *__restrict__ staging) {
+    __shared__ AosBlock b;
     const ChainInfo c = chains[chain];
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < c.volume;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        const Coord x = decode_storage(c, s);
-        for (int mu = 0; mu < 4; ++mu) {
-            const double2 *src = staging + (x.lex * 4 + mu) * 9;
-            double2 *dst = links + c.offset + (int64_t)(mu * 9) * c.volume + s;
-            for (int e = 0; e < 9; ++e) dst[(int64_t)e * c.volume] = src[e];
-        }
-    }
+    int64_t s;
+    bool live;
+    const int n = aos_sites(c, b, s, live), mu = threadIdx.x >> 5;
+    aos_read(b, n, staging);
+    if (!live) return;
+    double2 *dst = links + c.offset + (int64_t)(mu * 9) * c.volume + s;
+#pragma unroll
+    for (int e = 0; e < 9; ++e) dst[(int64_t)e * c.volume] = b.v[threadIdx.x & 31][mu * 9 + e];
 }
 
-__global__ void k_su3_to_aos(const ChainInfo *__restrict__ chains, int chain,
-                             const double2 *__restrict__ links, double2 *staging) {
+__global__ void __launch_bounds__(kAosThreads)
+k_su3_to_aos(const ChainInfo *__restrict__ chains, int chain, const double2 *__restrict__ links, double2 *staging) {
+    __shared__ AosBlock b;
     const ChainInfo c = chains[chain];
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < c.volume;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        const Coord x = decode_storage(c, s);
-        for (int mu = 0; mu < 4; ++mu) {
-            double2 *dst = staging + (x.lex * 4 + mu) * 9;
-            const double2 *src = links + c.offset + (int64_t)(mu * 9) * c.volume + s;
-            for (int e = 0; e < 9; ++e) dst[e] = src[(int64_t)e * c.volume];
-        }
+    int64_t s;
+    bool live;
+    const int n = aos_sites(c, b, s, live), mu = threadIdx.x >> 5;
+    if (live) {
+        const double2 *src = links + c.offset + (int64_t)(mu * 9) * c.volume + s;
+#pragma unroll
+        for (int e = 0; e < 9; ++e) b.v[threadIdx.x & 31][mu * 9 + e] = src[(int64_t)e * c.volume];
     }
+    aos_write(b, n, staging);
 }
 
 // ------------------------------------------------------------ launchers
@@ -382,13 +383,13 @@ cudaError_t launch_su3_identity(ym_ensemble *e) {
 }
 
 cudaError_t launch_su3_from_aos(ym_ensemble *e, int64_t chain) {
-    k_su3_from_aos<<<grid_for(e->chains[chain].volume, 128), 128, 0, e->stream>>>(
+    k_su3_from_aos<<<aos_blocks(e->chains[chain].volume), kAosThreads, 0, e->stream>>>(
         e->d_chains, (int)chain, e->d_links, reinterpret_cast<const double2 *>(e->d_staging));
     return cudaGetLastError();
 }
 
 cudaError_t launch_su3_to_aos(ym_ensemble *e, int64_t chain) {
-    k_su3_to_aos<<<grid_for(e->chains[chain].volume, 128), 128, 0, e->stream>>>(
+    k_su3_to_aos<<<aos_blocks(e->chains[chain].volume), kAosThreads, 0, e->stream>>>(
         e->d_chains, (int)chain, e->d_links, reinterpret_cast<double2 *>(e->d_staging));
     return cudaGetLastError();
 }

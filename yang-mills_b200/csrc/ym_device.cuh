@@ -453,4 +453,41 @@ __device__ __forceinline__ void store_su3(double2 *links, const ChainInfo &c, in
     for (int e = 0; e < 9; ++e) p[(int64_t)e * c.volume] = make_double2(u.e[e / 3][e % 3].re, u.e[e / 3][e % 3].im);
 }
 
+// ---- host layout ----------------------------------------------------------
+// The layout conversions take 32 storage sites per 128-thread block, warp mu
+// their mu-links: planes are read and written 32 sites at a time, and a site's
+// 36 entries go through shared memory so that the host side is moved in
+// runs of 576 bytes.  (One thread per site, entry by entry: every access a
+// 16-byte piece, and 10 us for a 4^4 chain, whose two blocks waited for 36
+// loads in turn.)
+constexpr int kAosSites = 32, kAosThreads = 4 * kAosSites, kAosPitch = 37;
+
+struct AosBlock {
+    double2 v[kAosSites][kAosPitch];
+    int64_t lex[kAosSites];
+};
+
+// This thread's site (storage slot) and the block's site count; fills lex.
+__device__ __forceinline__ int aos_sites(const ChainInfo &c, AosBlock &b, int64_t &s, bool &live) {
+    const int64_t first = (int64_t)blockIdx.x * kAosSites;
+    const int n = c.volume - first < kAosSites ? (int)(c.volume - first) : kAosSites;
+    const int lane = threadIdx.x & 31;
+    s = first + lane;
+    live = lane < n;
+    if (threadIdx.x < n) b.lex[threadIdx.x] = decode_storage(c, s).lex;
+    return n;
+}
+
+// Between the block's sites in shared memory and the host layout.
+__device__ __forceinline__ void aos_write(const AosBlock &b, int n, double2 *staging) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < n * 36; i += kAosThreads) staging[b.lex[i / 36] * 36 + i % 36] = b.v[i / 36][i % 36];
+}
+
+__device__ __forceinline__ void aos_read(AosBlock &b, int n, const double2 *staging) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < n * 36; i += kAosThreads) b.v[i / 36][i % 36] = staging[b.lex[i / 36] * 36 + i % 36];
+    __syncthreads();
+}
+
 }  // namespace ym

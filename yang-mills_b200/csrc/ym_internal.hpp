@@ -19,6 +19,9 @@ constexpr int64_t kLpPartialStride = 6304;  // floats per tile of learned-propos
 // Groups of 64 tiles in the first stage of the gradient reduction.
 inline int64_t lp_reduce_groups(int64_t tiles) { return (tiles + 63) / 64; }
 
+// Blocks of the layout conversions (ym_device.cuh).
+inline unsigned aos_blocks(int64_t volume) { return (unsigned)((volume + kAosSites - 1) / kAosSites); }
+
 // Maps a CUDA error onto a status (YM_OK or YM_ERR_CUDA) and records a
 // failure as the calling thread's ym_last_cuda_error (capi.cu).
 int32_t record_cuda_status(cudaError_t err);
