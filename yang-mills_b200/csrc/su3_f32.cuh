@@ -158,8 +158,9 @@ __device__ __forceinline__ m3f staple_f(const float2 *__restrict__ links, const 
 // Every factor is copied global -> shared by cp.async two terms ahead of its
 // use, into a ring of two sets of three [6][TT] float2 buffers (two stored
 // rows per link, a column per thread), so loads in flight hold no registers.
-// Same terms, order and arithmetic as staple_f, so the same bits; mu and nu
-// are run-time values, so one copy of the code serves every direction.
+// The staple's terms and their order are the FP64 path's: for each nu != mu
+// ascending, forward then backward.  mu and nu are run-time values, so one
+// copy of the code serves every direction.
 template <int TT>
 struct SetF {
     float2 (*f[3])[TT];
@@ -200,23 +201,26 @@ __device__ __forceinline__ void stage_term_f(const SetF<TT> &b, const float2 *ba
 }
 
 template <bool BWD, int TT>
-__device__ __forceinline__ void term_f(const SetF<TT> &b, m3f &a) {
+__device__ __forceinline__ m3f pair_f(const SetF<TT> &b) {
     m3f p;
-    {
-        const m3f l1 = staged_f(b.f[0]), l2 = staged_f(b.f[1]);
+    const m3f l1 = staged_f(b.f[0]), l2 = staged_f(b.f[1]);
 #pragma unroll
-        for (int r = 0; r < 3; ++r)
+    for (int r = 0; r < 3; ++r)
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                cf v = cfm(0.f, 0.f);
+        for (int k = 0; k < 3; ++k) {
+            cf v = cfm(0.f, 0.f);
 #pragma unroll
-                for (int j = 0; j < 3; ++j) {
-                    if (!BWD) cffma(v, l1.e[r][j], cfconj(l2.e[k][j]));
-                    else cffma(v, cfconj(l1.e[j][r]), cfconj(l2.e[k][j]));
-                }
-                p.e[r][k] = v;
+            for (int j = 0; j < 3; ++j) {
+                if (!BWD) cffma(v, l1.e[r][j], cfconj(l2.e[k][j]));
+                else cffma(v, cfconj(l1.e[j][r]), cfconj(l2.e[k][j]));
             }
-    }
+            p.e[r][k] = v;
+        }
+    return p;
+}
+
+template <bool BWD, int TT>
+__device__ __forceinline__ void third_f(const SetF<TT> &b, const m3f &p, m3f &a) {
     const m3f l3 = staged_f(b.f[2]);
 #pragma unroll
     for (int r = 0; r < 3; ++r)
@@ -227,6 +231,12 @@ __device__ __forceinline__ void term_f(const SetF<TT> &b, m3f &a) {
                 if (!BWD) cffma(a.e[r][col], p.e[r][k], cfconj(l3.e[col][k]));
                 else cffma(a.e[r][col], p.e[r][k], l3.e[k][col]);
             }
+}
+
+template <bool BWD, int TT>
+__device__ __forceinline__ void term_f(const SetF<TT> &b, m3f &a) {
+    const m3f p = pair_f<BWD>(b);
+    third_f<BWD>(b, p, a);
 }
 
 // The staple of link (x, mu); its first term has been staged into s0.  The
