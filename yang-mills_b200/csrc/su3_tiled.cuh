@@ -275,10 +275,11 @@ __device__ __forceinline__ void swap_rows(Row &x, Row &y) {
     y = t;
 }
 
-// The eight ordered hits (generators 1..8, su3_ensemble.rs:361) in a loop
-// over the three SU(2) subgroups (rows (0,1), (0,2), (1,2)): the rows trade
-// places between its passes, so one copy of the code serves all three.  Hit
-// h+1's link-independent half is written next to hit h.
+// The eight ordered hits (generators 1..8, su3_ensemble.rs:361), the three
+// SU(2) subgroups (rows (0,1), (0,2), (1,2)) one after the other, unrolled (as
+// a loop, with the rows moved between its passes: 32^4 sweep 1373 against
+// 1335 us, measured 1433 against 1365, 16^4 95 against 90).  Hit h+1's
+// link-independent half is written next to hit h.
 // tr receives Re Tr(U' A) of the final link, the sum of its six plaquettes.
 template <int K, class A>
 __device__ __forceinline__ unsigned visit_ordered(m3 &u, const A &sa, double beta3, double angle, uint64_t key,
@@ -297,7 +298,7 @@ __device__ __forceinline__ unsigned visit_ordered(m3 &u, const A &sa, double bet
     Row x = r[0], y = r[1], z = r[2];
     uint64_t state = key;
     BlockPre p = pre_block<K>(state, angle);
-#pragma unroll 1
+#pragma unroll
     for (int it = 0; it < 3; ++it) {
         const int ca = it == 2 ? 1 : 0, cb = it == 0 ? 1 : 2;
         const int h0 = it == 0 ? 0 : 2 * it + 1;   // the pass's first hit
@@ -478,17 +479,18 @@ __device__ __forceinline__ unsigned visit_drawn(const U &u, const A &a, double b
 // (1) The CTAs are persistent, and the next item's first term loads into the
 // first set while this item's hits run, so no item starts on an empty
 // pipeline (chain table, then links: three dependent trips to L2).  (2) The
-// code is small: directions and subgroups are loops, not copies.  Unrolled
+// code is small: directions are loops, not copies.  Unrolled
 // (66 KB, four directions of it) the warps, which drift apart once they are
 // persistent, waited for instructions as long as for data.  Per issued
 // instruction on a 32^4 lattice, half width 0.3: unrolled and one tile per
 // CTA 1.57 cycles on loads + 0.40 on instruction fetch (168 us per launch
 // under the profiler), persistent unrolled 0.85-1.13 + 0.52-0.91 (169 us),
-// persistent loops 0.76 + 0.12 (161 us; 10 % more integer instructions).
+// persistent with looped directions 0.76 + 0.12 (161 us, hits looped too).
 // Three CTAs per SM (one term ahead, 168 registers with 150 bytes spilled):
-// 1.52 + 0.62, 180 us.  Sweep of 32^4 live, same box: 1438 -> 1300 us at
-// half width 0.3, 1439 -> 1289 us at 0.35 (of which the shorter rotations
-// and accept_log 6 %); 8^4 94 -> 73 us, 16^4 102 -> 97 us.
+// 1.52 + 0.62, 180 us.  Sweep live, start of this design -> now, same
+// boxes: 32^4 1487 -> 1319 us at half width 0.3 (of which the shorter
+// rotations and accept_log 6 %), 16^4 103 -> 92, 8^4 88 -> 76, 32 chains of
+// 6^3 x 10 130 -> 121; drawn generators 2409 -> 1755 (32^4), 230 -> 135 (16^4).
 struct TermSet {
     double2 (*f[3])[T];
 };
