@@ -197,35 +197,6 @@ __device__ __forceinline__ bool sample_kp(double alpha, uint64_t key, int max_at
 constexpr unsigned kErrAttempts = 1u;
 constexpr unsigned kErrNonFinite = 2u;
 
-// The chain of a block's tile.  A handle of one chain passes its geometry by
-// value (`one`, its extents never change), so that a block starts on its links
-// without the two dependent trips to L2 for the tile and the chain; beta and
-// the seed, which may change between launches of a captured graph, are read
-// where they are needed, late.
-struct Block {
-    ChainInfo c;
-    int64_t start;
-    int32_t chain;
-};
-
-__device__ __forceinline__ Block block_of(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles,
-                                          const ChainInfo &one, int64_t tile) {
-    Block b;
-    if (one.volume) {
-        b.c = one;
-        b.start = tile * T;
-        b.chain = 0;
-        b.c.beta = chains[0].beta;
-        b.c.seed = chains[0].seed;
-    } else {
-        const Tile t = tiles[tile];
-        b.c = chains[t.chain];
-        b.start = t.start;
-        b.chain = t.chain;
-    }
-    return b;
-}
-
 // One thread per link (large sub-sweeps).  What bounds it: binary64 latency
 // and issue of the normalised products.  24^4, per launch under the profiler:
 // overrelaxation 48 us with plain divisions and one product at a time, 34 us
@@ -239,7 +210,7 @@ k_su2_heatbath_thread(const ChainInfo *__restrict__ chains, const Tile *__restri
                const __grid_constant__ ChainInfo one, double2 *__restrict__ links, int parity, int max_attempts, int kp,
                const uint64_t *__restrict__ sweep_ptr, unsigned long long *__restrict__ proposals,
                unsigned *__restrict__ err) {
-    const Block block = block_of(chains, tiles, one, blockIdx.x);
+    const ItemChain block = block_of(chains, tiles, one, blockIdx.x, T);
     const ChainInfo &c = block.c;
     const int64_t t = block.start + threadIdx.x;
     unsigned attempts_used = 0;
@@ -281,7 +252,7 @@ template <int MU>
 __global__ void __launch_bounds__(T)
 k_su2_overrelax_thread(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles,
                 const __grid_constant__ ChainInfo one, double2 *__restrict__ links, int parity, unsigned *__restrict__ err) {
-    const Block block = block_of(chains, tiles, one, blockIdx.x);
+    const ItemChain block = block_of(chains, tiles, one, blockIdx.x, T);
     const ChainInfo &c = block.c;
     const int64_t t = block.start + threadIdx.x;
     if (t >= c.half) return;
@@ -312,7 +283,7 @@ k_su2_heatbath_group(const ChainInfo *__restrict__ chains, const Tile *__restric
                const __grid_constant__ ChainInfo one, double2 *__restrict__ links, int parity, int max_attempts, int kp,
                const uint64_t *__restrict__ sweep_ptr, unsigned long long *__restrict__ proposals,
                unsigned *__restrict__ err) {
-    const Block block = block_of(chains, tiles, one, blockIdx.x / kGroup);
+    const ItemChain block = block_of(chains, tiles, one, blockIdx.x / kGroup, T);
     const ChainInfo &c = block.c;
     const int64_t t = block.start + (int64_t)(blockIdx.x % kGroup) * kGroupLinks + threadIdx.x / kGroup;
     const bool leader = (threadIdx.x & (kGroup - 1)) == 0;
@@ -356,7 +327,7 @@ template <int MU>
 __global__ void __launch_bounds__(T)
 k_su2_overrelax_group(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles,
                 const __grid_constant__ ChainInfo one, double2 *__restrict__ links, int parity, unsigned *__restrict__ err) {
-    const Block block = block_of(chains, tiles, one, blockIdx.x / kGroup);
+    const ItemChain block = block_of(chains, tiles, one, blockIdx.x / kGroup, T);
     const ChainInfo &c = block.c;
     const int64_t t = block.start + (int64_t)(blockIdx.x % kGroup) * kGroupLinks + threadIdx.x / kGroup;
     const bool leader = (threadIdx.x & (kGroup - 1)) == 0;
@@ -546,9 +517,6 @@ int grid_for(int64_t n, int threads) {
 }
 
 }  // namespace
-
-// The geometry of a handle of one chain, else an empty one.
-static ChainInfo single_chain(const ym_ensemble *e) { return e->n_chains == 1 ? e->chains[0] : ChainInfo{}; }
 
 // The grouped kernels give each link kGroup lanes; they win while a
 // sub-sweep has too few links to hide the one-thread kernels' latency

@@ -48,15 +48,15 @@ constexpr size_t kRingF = (size_t)36 * T * sizeof(float2);
 template <bool DRAWN>
 __global__ void __launch_bounds__(T, YM_F32_MIN_BLOCKS)
 k_f32_metropolis(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles,
-                 float2 *__restrict__ links, int parity, int mu, double angle,
+                 const __grid_constant__ ChainInfo one, float2 *__restrict__ links, int parity, int mu, double angle,
                  const uint64_t *__restrict__ sweep_ptr, unsigned long long *__restrict__ accepts,
                  int reverse) {
     extern __shared__ __align__(16) float2 ring_mem[];
     auto buf = [&](int i) { return reinterpret_cast<float2 (*)[T]>(ring_mem + (size_t)i * 6 * T); };
     const SetF<T> s0{{buf(0), buf(1), buf(2)}}, s1{{buf(3), buf(4), buf(5)}};
-    const Tile tile = tiles[reverse ? gridDim.x - 1 - blockIdx.x : blockIdx.x];
-    const ChainInfo c = chains[tile.chain];
-    const int64_t t = tile.start + threadIdx.x;
+    const ItemChain block = block_of(chains, tiles, one, reverse ? gridDim.x - 1 - blockIdx.x : blockIdx.x, T);
+    const ChainInfo &c = block.c;
+    const int64_t t = block.start + threadIdx.x;
     const uint64_t sweep = *sweep_ptr;
     unsigned accepted = 0;
     if (t < c.half) {
@@ -83,7 +83,7 @@ k_f32_metropolis(const ChainInfo *__restrict__ chains, const Tile *__restrict__ 
     }
     const unsigned warp_sum = __reduce_add_sync(0xffffffffu, accepted);
     if ((threadIdx.x & 31) == 0 && warp_sum)
-        atomicAdd(accepts + tile.chain, (unsigned long long)warp_sum);
+        atomicAdd(accepts + block.chain, (unsigned long long)warp_sum);
 }
 
 // Gram-Schmidt of rows 0-1 in binary64, rounded back once.
@@ -272,7 +272,7 @@ float2 *f32_links(ym_ensemble *e) { return reinterpret_cast<float2 *>(e->d_links
 template <bool DRAWN>
 static cudaError_t launch_f32_form(ym_ensemble *e, int parity, int mu, double angle, int reverse) {
     k_f32_metropolis<DRAWN><<<(unsigned)e->n_half_tiles, T, kRingF, e->stream>>>(
-        e->d_chains, e->d_half_tiles, f32_links(e), parity, mu, angle, e->d_sweep, e->d_accepts, reverse);
+        e->d_chains, e->d_half_tiles, single_chain(e), f32_links(e), parity, mu, angle, e->d_sweep, e->d_accepts, reverse);
     return cudaGetLastError();
 }
 

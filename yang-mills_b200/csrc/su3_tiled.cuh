@@ -614,15 +614,12 @@ constexpr int kRingBuffers = 6;   // two sets of three factors
 template <int K, bool MEASURE, bool DRAWN>
 __global__ void __launch_bounds__(T, 2)
 k_su3_metropolis_ring(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles, int n_ctas,
-                      double2 *__restrict__ links, int parity, int mu, double angle,
+                      const __grid_constant__ ChainInfo one, double2 *__restrict__ links, int parity, int mu, double angle,
                       const uint64_t *__restrict__ sweep_ptr, unsigned long long *__restrict__ accepts,
                       int log2_item, int reverse, double *__restrict__ tr_partial = nullptr) {
     extern __shared__ __align__(16) double2 ring_mem[];
     auto buf = [&](int i) { return reinterpret_cast<double2 (*)[T]>(ring_mem + (size_t)i * 9 * T); };
     const TermSet s0{{buf(0), buf(1), buf(2)}}, s1{{buf(3), buf(4), buf(5)}};
-    auto tile_of = [&](int b) {
-        return tiles[(int64_t)(reverse ? n_ctas - 1 - b : b) * (T >> log2_item) + (threadIdx.x >> log2_item)];
-    };
     const int64_t lane = threadIdx.x & ((1u << log2_item) - 1u);
     const uint64_t sweep = *sweep_ptr;
     int32_t chain;        // of the item in hand
@@ -633,11 +630,13 @@ k_su3_metropolis_ring(const ChainInfo *__restrict__ chains, const Tile *__restri
     double beta;
     uint64_t seed;
     auto take_item = [&](int b) {
-        const Tile tile = tile_of(b);
-        const ChainInfo c = chains[tile.chain >= 0 ? tile.chain : 0];
-        chain = tile.chain;
-        live = tile.chain >= 0 && tile.start + lane < c.half;
-        x = site_of(c, decode_storage(c, (int64_t)parity * c.half + (live ? tile.start + lane : 0)));
+        // padding items (chain < 0) read the first chain's geometry and stay idle
+        const int64_t item = (int64_t)(reverse ? n_ctas - 1 - b : b) * (T >> log2_item) + (threadIdx.x >> log2_item);
+        const ItemChain it = block_of(chains, tiles, one, item, 1 << log2_item);
+        const ChainInfo &c = it.c;
+        chain = it.chain;
+        live = it.chain >= 0 && it.start + lane < c.half;
+        x = site_of(c, decode_storage(c, (int64_t)parity * c.half + (live ? it.start + lane : 0)));
         base = links + c.offset;
         volume = c.volume;
         beta = c.beta;
@@ -728,7 +727,7 @@ void metro_launch_ring(ym_ensemble *e, int parity, int mu, double angle, int rev
     const SweepLayout &L = e->layouts[e->sweep_layout];
     const dim3 grid(ring_grid(L.ctas)), block(T);
     k_su3_metropolis_ring<K, false, DRAWN><<<grid, block, kRingBytes, e->stream>>>(
-        e->d_chains, L.d_items, (int)L.ctas, e->d_links, parity, mu, angle, e->d_sweep, e->d_accepts, L.log2_item,
+        e->d_chains, L.d_items, (int)L.ctas, single_chain(e), e->d_links, parity, mu, angle, e->d_sweep, e->d_accepts, L.log2_item,
         reverse, nullptr);
 }
 
@@ -741,7 +740,7 @@ void metro_launch_measure(ym_ensemble *e, int mu, double angle, double *tr_parti
     const dim3 g(ring_grid(L.ctas)), b(T);
     const int rev = (1 * 4 + mu) & 1;   // the tile order tiled_launch gives (parity 1, mu)
     k_su3_metropolis_ring<K, true, false><<<g, b, kRingBytes, e->stream>>>(
-        e->d_chains, L.d_items, (int)L.ctas, e->d_links, 1, mu, angle, e->d_sweep, e->d_accepts, L.log2_item, rev,
+        e->d_chains, L.d_items, (int)L.ctas, single_chain(e), e->d_links, 1, mu, angle, e->d_sweep, e->d_accepts, L.log2_item, rev,
         tr_partial);
 }
 

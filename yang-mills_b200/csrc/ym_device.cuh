@@ -421,6 +421,35 @@ __device__ __forceinline__ int32_t pick(const int32_t *v, int d) {
     return d == 0 ? v[0] : (d == 1 ? v[1] : (d == 2 ? v[2] : v[3]));
 }
 
+// The chain of a block's tile.  A handle of one chain passes its geometry by
+// value (`one`, its extents never change), so that a block starts on its links
+// without the two dependent trips to L2 for the tile and the chain; beta and
+// the seed, which may change between launches of a captured graph, are read
+// where they are needed, late.
+struct ItemChain {
+    ChainInfo c;
+    int64_t start;
+    int32_t chain;
+};
+
+__device__ __forceinline__ ItemChain block_of(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles,
+                                              const ChainInfo &one, int64_t tile, int tile_sites) {
+    ItemChain b;
+    if (one.volume) {
+        b.c = one;
+        b.start = tile * tile_sites;
+        b.chain = 0;
+        b.c.beta = chains[0].beta;
+        b.c.seed = chains[0].seed;
+    } else {
+        const Tile t = tiles[tile];
+        b.c = chains[t.chain >= 0 ? t.chain : 0];
+        b.start = t.start;
+        b.chain = t.chain;
+    }
+    return b;
+}
+
 // SU(3) FP64 link access: plane (mu*9 + entry) of a chain's block.
 __device__ __forceinline__ m3 load_su3(const double2 *__restrict__ links, const ChainInfo &c,
                                        int64_t s, int mu) {

@@ -159,6 +159,11 @@ struct ym_ensemble {
     size_t events_used[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 };
 
+// The geometry of a handle of one chain, else an empty one (block_of).
+inline ym::ChainInfo single_chain(const ym_ensemble *e) {
+    return e->n_chains == 1 ? e->chains[0] : ym::ChainInfo{};
+}
+
 // A learned-proposal model on one device (include/ym_learned.h).
 struct ym_proposal_model {
     int32_t device = 0;
