@@ -332,10 +332,10 @@ constexpr int64_t kTuneSweeps = 4;   // sweeps timed per path when choosing
 
 // Whether an undecided handle runs resident without timing: one chain per SM
 // at most, so the launch is a single wave.  4^4, per measured sweep, resident
-// against tiled: 1 to 148 chains 52 against 87-96 us (ordered hits) and 82
-// against 118-126 us (drawn); 4^3 x 6 119 against 140-193 us.  Past one wave
-// it depends on the chains (160: 101 against 117 and 163 against 157 us; 600:
-// 250 against 273 and 406 against 381 us), and the tuner times both.
+// against tiled: 1 to 148 chains 46-48 against 87-97 us (ordered hits) and
+// 72-78 against 117-126 us (drawn); 4^3 x 6 118 against 138-192 us.  Past one
+// wave the gap closes (600 chains: 222 against 270 and 383 against 384 us),
+// and the tuner times both.
 bool one_wave(const ym_ensemble *e) {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);

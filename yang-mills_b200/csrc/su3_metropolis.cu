@@ -29,9 +29,11 @@ constexpr int T = kSweepThreads;
 // instructions than executing them), each thread owns one link of each
 // sub-sweep for the whole launch, and the hits run on the links in place:
 // nobody else reads a link that is being updated.  64 chains of 4^4, drawn
-// generators, per measured sweep: 247 us in the unrolled form, 83 now (ordered
-// hits 189 and 52); 2.8 cycles per instruction, of which 1.3 wait for a
-// binary64 result and 0.2 for an instruction.
+// generators, per measured sweep: 247 us in the unrolled form, 82 as one loop
+// (2.8 cycles per instruction, of which 1.3 wait for a binary64 result and
+// 0.2 for an instruction), 78 with the hits' link-independent halves made by
+// the threads that have no link, 72 with lambda8's row outside a branch;
+// ordered hits 189, 52 and 46.
 constexpr int kResidentThreads = 256;   // resident chains have at most 201 links per sub-sweep
 
 // A link of the chain in shared memory.
@@ -64,9 +66,69 @@ __device__ __forceinline__ void resident_term(const double2 *sl, int v, const Si
     tiled_exact::add_third<BWD>(p, resident_link(ln + i3, v), a);
 }
 
-// SA: the accumulator waits in shared memory for the hits, else (chains that
-// leave no room for it) in local memory.
-template <int K, bool DRAWN, bool SA>
+// The hits' link-independent halves of one sub-sweep, made by the threads that
+// have no link of their own while the others form their staples: entry h of
+// link t at [h][t].
+struct PreTable {
+    double2 e1[8][kResidentThreads / 2];   // rotation, or lambda8's phase of rows 0 and 1
+    double2 e2[8][kResidentThreads / 2];   // lambda8's phase of row 2
+    float logu[8][kResidentThreads / 2];
+    int gen[8][kResidentThreads / 2];      // drawn generators
+};
+
+template <int K, bool DRAWN>
+__device__ __forceinline__ void fill_table(PreTable &tab, int t, uint64_t key, double angle) {
+    using namespace tiled_exact;
+    uint64_t state = key;
+#pragma unroll 1
+    for (int h = 0; h < 8; ++h) {
+        if (DRAWN) {
+            const DrawnPre p = pre_drawn<K>(state, angle);
+            tab.e1[h][t] = make_double2(p.e1.re, p.e1.im);
+            tab.e2[h][t] = make_double2(p.e2.re, p.e2.im);
+            tab.logu[h][t] = p.logu;
+            tab.gen[h][t] = p.g;
+        } else if (h < 7) {
+            const BlockPre p = pre_block<K>(state, angle);
+            tab.e1[h][t] = make_double2(p.c, p.s);
+            tab.logu[h][t] = p.logu;
+        } else {
+            const DiagPre p = pre_diag<K>(state, angle);
+            tab.e1[h][t] = make_double2(p.e1.re, p.e1.im);
+            tab.e2[h][t] = make_double2(p.e2.re, p.e2.im);
+            tab.logu[h][t] = p.logu;
+        }
+    }
+}
+
+struct TablePre {
+    const PreTable &tab;
+    int t, h;
+    __device__ __forceinline__ tiled_exact::BlockPre block() {
+        const double2 v = tab.e1[h][t];
+        return tiled_exact::BlockPre{v.x, v.y, tab.logu[h++][t]};
+    }
+    __device__ __forceinline__ tiled_exact::DiagPre diag() {
+        const double2 v = tab.e1[h][t], w = tab.e2[h][t];
+        return tiled_exact::DiagPre{cmake(v.x, v.y), cmake(w.x, w.y), tab.logu[h][t]};
+    }
+    __device__ __forceinline__ tiled_exact::DrawnPre next() {
+        const double2 v = tab.e1[h][t], w = tab.e2[h][t];
+        const tiled_exact::DrawnPre p{cmake(v.x, v.y), cmake(w.x, w.y), tab.logu[h][t], tab.gen[h][t]};
+        ++h;
+        return p;
+    }
+};
+
+// The three forms: where the staple sum waits for the hits, and who makes the
+// hits' link-independent halves.
+enum ResidentForm {
+    kLocal,     // in local memory (chains that leave no room for it), each thread its own
+    kShared,    // in shared memory, each thread its own
+    kTable      // in shared memory, the upper half of the block (at most 128 links per sub-sweep)
+};
+
+template <int K, bool DRAWN, int FORM>
 __global__ void __launch_bounds__(kResidentThreads, 1)
 k_su3_resident(const ChainInfo *__restrict__ chains, double2 *__restrict__ links, double angle,
                const uint64_t *__restrict__ sweep_ptr, int64_t n_meas, int64_t sweeps_per_meas,
@@ -83,9 +145,13 @@ k_su3_resident(const ChainInfo *__restrict__ chains, double2 *__restrict__ links
     for (int i = threadIdx.x; i < n; i += kResidentThreads) cp_async16(sl + i, links + c.offset + i);
     cp_async_commit();
     const int t = threadIdx.x;
-    const bool live = t < half;
-    double2 local_a[SA ? 1 : 9];
-    const Col<SA ? kResidentThreads : 1> sa{SA ? sl + n + t : local_a, 0};
+    double2 local_a[FORM == kLocal ? 9 : 1];
+    constexpr int kLinks = FORM == kTable ? kResidentThreads / 2 : kResidentThreads;
+    const Col<FORM == kLocal ? 1 : kLinks> sa{FORM == kLocal ? local_a : sl + n + t % kLinks, 0};
+    PreTable &tab = *reinterpret_cast<PreTable *>(sl + n + (FORM == kTable ? 9 * kLinks : 0));
+    const bool helper = FORM == kTable && t >= kLinks;   // makes link t - kLinks's table
+    const int mine = helper ? t - kLinks : t;
+    const bool live = mine < half;
     const double beta3 = c.beta / 3.0;
     cp_async_wait_all();
     __syncthreads();
@@ -98,8 +164,14 @@ k_su3_resident(const ChainInfo *__restrict__ chains, double2 *__restrict__ links
 #pragma unroll 1
             for (int sub = 0; sub < 8; ++sub) {
                 const int par = sub >> 2, mu = sub & 3;
+                uint64_t key = 0;
                 if (live) {
-                    if (mu == 0) x = site_of(c, decode_storage(c, par * half + t));
+                    if (mu == 0) x = site_of(c, decode_storage(c, par * half + mine));
+                    key = link_key(c.seed, sweep, x.lex, mu);
+                }
+                if (helper) {
+                    if (live) fill_table<K, DRAWN>(tab, mine, key, angle);
+                } else if (live) {
                     m3 a;
 #pragma unroll
                     for (int r = 0; r < 3; ++r)
@@ -113,15 +185,20 @@ k_su3_resident(const ChainInfo *__restrict__ chains, double2 *__restrict__ links
                     }
 #pragma unroll
                     for (int e = 0; e < 9; ++e) sa.put(e, a.e[e / 3][e % 3]);
-                    const uint64_t key = link_key(c.seed, sweep, x.lex, mu);
+                }
+                if (FORM == kTable) __syncthreads();
+                if (live && !helper) {
                     double2 *p = sl + mu * 9 * v + (par ? half : 0) + (x.lex >> 1);
                     const Col<0> rows{p, v};
                     if (DRAWN) {
-                        accepted += visit_drawn<K>(rows, sa, beta3, angle, key);
+                        accepted += FORM == kTable ? visit_drawn<K>(rows, sa, beta3, key, TablePre{tab, mine, 0})
+                                                   : visit_drawn<K>(rows, sa, beta3, key, DrawnStream<K>{key, angle});
                     } else {
                         m3 u = resident_link(p, v);
                         double tr;
-                        accepted += visit_ordered<K>(u, sa, beta3, angle, key, tr);
+                        accepted += FORM == kTable
+                                        ? visit_ordered(u, sa, beta3, key, TablePre{tab, mine, 0}, tr)
+                                        : visit_ordered(u, sa, beta3, key, OrderedStream<K>{key, angle}, tr);
 #pragma unroll
                         for (int e = 0; e < 9; ++e) rows.put(e, u.e[e / 3][e % 3]);
                     }
@@ -201,9 +278,17 @@ template <int K, bool DRAWN>
 static cudaError_t resident_launch(ym_ensemble *e, double angle, int64_t n_meas, int64_t sweeps_per_meas,
                                    double *series) {
     const size_t links = resident_smem_bytes(e);
-    const bool sa = links + kResidentAccumulator + kResidentFixed <= (size_t)optin_smem();
-    const size_t smem = links + (sa ? kResidentAccumulator : 0);
-    auto kernel = sa ? k_su3_resident<K, DRAWN, true> : k_su3_resident<K, DRAWN, false>;
+    int64_t vmax = 0;
+    for (const ChainInfo &c : e->chains) vmax = c.volume > vmax ? c.volume : vmax;
+    auto kernel = k_su3_resident<K, DRAWN, kLocal>;
+    size_t smem = links;
+    if (vmax <= kResidentThreads) {   // half as many links per sub-sweep as threads
+        kernel = k_su3_resident<K, DRAWN, kTable>;
+        smem = links + kResidentAccumulator / 2 + sizeof(PreTable);
+    } else if (links + kResidentAccumulator + kResidentFixed <= (size_t)optin_smem()) {
+        kernel = k_su3_resident<K, DRAWN, kShared>;
+        smem = links + kResidentAccumulator;
+    }
     const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
     kernel<<<(unsigned)e->n_chains, kResidentThreads, smem, e->stream>>>(

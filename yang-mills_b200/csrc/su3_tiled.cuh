@@ -215,6 +215,14 @@ __device__ __forceinline__ DiagPre pre_diag(uint64_t &state, double angle) {
     return p;
 }
 
+template <int K>
+struct OrderedStream {
+    uint64_t state;
+    double angle;
+    __device__ __forceinline__ BlockPre block() { return pre_block<K>(state, angle); }
+    __device__ __forceinline__ DiagPre diag() { return pre_diag<K>(state, angle); }
+};
+
 // One row of a link and its Re Tr share.
 struct Row {
     cplx e[3];
@@ -281,9 +289,10 @@ __device__ __forceinline__ void swap_rows(Row &x, Row &y) {
 // 1335 us, measured 1433 against 1365, 16^4 95 against 90).  Hit h+1's
 // link-independent half is written next to hit h.
 // tr receives Re Tr(U' A) of the final link, the sum of its six plaquettes.
-template <int K, class A>
-__device__ __forceinline__ unsigned visit_ordered(m3 &u, const A &sa, double beta3, double angle, uint64_t key,
-                                                  double &tr) {
+// pre gives the hits' link-independent halves in order (OrderedStream, or a
+// table made by other threads).
+template <class A, class Pre>
+__device__ __forceinline__ unsigned visit_ordered(m3 &u, const A &sa, double beta3, uint64_t key, Pre pre, double &tr) {
     Row r[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
@@ -296,18 +305,17 @@ __device__ __forceinline__ unsigned visit_ordered(m3 &u, const A &sa, double bet
     double old_tr = (r[0].rr + r[1].rr) + r[2].rr;
     unsigned accepted = 0;
     Row x = r[0], y = r[1], z = r[2];
-    uint64_t state = key;
-    BlockPre p = pre_block<K>(state, angle);
+    BlockPre p = pre.block();
 #pragma unroll
     for (int it = 0; it < 3; ++it) {
         const int ca = it == 2 ? 1 : 0, cb = it == 0 ? 1 : 2;
         const int h0 = it == 0 ? 0 : 2 * it + 1;   // the pass's first hit
-        BlockPre q = pre_block<K>(state, angle);
+        BlockPre q = pre.block();
         hit_rows<0>(x, y, z, sa, ca, cb, it == 0, old_tr, p, beta3, accepted, key, h0);
-        if (it < 2) p = pre_block<K>(state, angle);
+        if (it < 2) p = pre.block();
         hit_rows<1>(x, y, z, sa, ca, cb, it == 0, old_tr, q, beta3, accepted, key, h0 + 1);
         if (it == 0) {
-            q = pre_block<K>(state, angle);
+            q = pre.block();
             hit_rows<2>(x, y, z, sa, ca, cb, true, old_tr, p, beta3, accepted, key, 2);
             p = q;
             swap_rows(y, z);
@@ -316,7 +324,7 @@ __device__ __forceinline__ unsigned visit_ordered(m3 &u, const A &sa, double bet
         }
     }
     // now x is row 1, y row 2, z row 0
-    const DiagPre d = pre_diag<K>(state, angle);
+    const DiagPre d = pre.diag();
     cplx n0[3], n1[3], n2[3], col[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -353,17 +361,18 @@ __device__ __forceinline__ unsigned visit_ordered(m3 &u, const A &sa, double bet
 //   lambda1, 4, 6: v0 = i r1, v1 = i r0;   lambda2, 5, 7: v0 = r1, v1 = r0, s' = -s;
 //   lambda3: v0 = i r0, v1 = i r1, s' = -s;  lambda8: v0 = i r0, v1 = i r1,
 // entry by entry the reference's two rounded products and their sum (a sign
-// change is exact).  lambda8's second phase on row 2 runs in a short branch.
+// change is exact).  lambda8's second phase on row 2 is formed for every
+// link: a warp has a lambda8 in 98 of 100 hits, and in a branch it would wait
+// outside the other products.
 // The link's rows and A's columns live in memory (u, a) and are addressed by
 // the generator: picking them among registers took twice the instructions
 // (10,600 per warp and visit, most of them selects and the two divergent
 // sides, against 4,900).
 struct DrawnPre {
-    double c, s;     // block rotation, or lambda8's phase of rows 0 and 1
-    double h2;       // lambda8: half angle of row 2's phase
+    cplx e1;         // block rotation c + i s, or lambda8's phase of rows 0 and 1
+    cplx e2;         // lambda8's phase of row 2
     float logu;
     int g;
-    bool sq;         // lambda8: the phases are squared once
 };
 
 template <int K>
@@ -375,19 +384,29 @@ __device__ __forceinline__ DrawnPre pre_drawn(uint64_t &state, double angle) {
     const double d1 = (0.5 * kInvSqrt3) * theta, d2 = (-kInvSqrt3) * theta;
     const bool diag = p.g == 7;
 #ifdef YM_TILED_FAST
-    p.sq = false;
+    const bool sq = false;
 #else
-    p.sq = diag && fmax(fabs(d1), fabs(d2)) > 0.5;
+    const bool sq = diag && fmax(fabs(d1), fabs(d2)) > 0.5;
 #endif
-    const double sc = p.sq ? 0.5 : 1.0;
-    p.h2 = d2 * sc;
-    block_rotation<K>(diag ? d1 * sc : 0.5 * theta, p.c, p.s);
+    const double sc = sq ? 0.5 : 1.0;
+    block_rotation<K>(diag ? d1 * sc : 0.5 * theta, p.e1.re, p.e1.im);
+    block_rotation<K>(d2 * sc, p.e2.re, p.e2.im);
+    const cplx q1 = cmul(p.e1, p.e1), q2 = cmul(p.e2, p.e2);
+    p.e1 = sq ? q1 : p.e1;
+    p.e2 = sq ? q2 : p.e2;
     p.logu = neg_log_unit(next_word(state));
     return p;
 }
 
-template <int K, class U, class A>
-__device__ __forceinline__ unsigned visit_drawn(const U &u, const A &a, double beta3, double angle, uint64_t key) {
+template <int K>
+struct DrawnStream {
+    uint64_t state;
+    double angle;
+    __device__ __forceinline__ DrawnPre next() { return pre_drawn<K>(state, angle); }
+};
+
+template <int K, class U, class A, class Pre>
+__device__ __forceinline__ unsigned visit_drawn(const U &u, const A &a, double beta3, uint64_t key, Pre pre) {
     double rr[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
@@ -398,12 +417,11 @@ __device__ __forceinline__ unsigned visit_drawn(const U &u, const A &a, double b
     }
     double old_tr = (rr[0] + rr[1]) + rr[2];
     unsigned accepted = 0;
-    uint64_t state = key;
-    DrawnPre nx = pre_drawn<K>(state, angle);
+    DrawnPre nx = pre.next();
 #pragma unroll 1
     for (int h = 0; h < 8; ++h) {
         const DrawnPre p = nx;
-        if (h < 7) nx = pre_drawn<K>(state, angle);
+        if (h < 7) nx = pre.next();
         const int g = p.g;
         const bool diag = g == 7;
         const bool low = g <= 2 || diag;                 // rows 0 and 1
@@ -413,24 +431,13 @@ __device__ __forceinline__ unsigned visit_drawn(const U &u, const A &a, double b
         cplx r0[3], r1[3], n0[3], n1[3], n2[3], col[3];
         u.row(i0, r0);
         u.row(i1, r1);
-        double c = p.c, s = p.s;
-        double q2 = i2 == 2 ? rr[2] : (i2 == 1 ? rr[1] : rr[0]);
-        if (diag) {
-            cplx e2;
-            block_rotation<K>(p.h2, e2.re, e2.im);
-            if (p.sq) {
-                const cplx e1 = cmul(cmake(c, s), cmake(c, s));
-                c = e1.re;
-                s = e1.im;
-                e2 = cmul(e2, e2);
-            }
-            cplx r2[3];
-            u.row(2, r2);
-            a.column(2, col);
+        const double c = p.e1.re, s = p.e1.im;
+        cplx r2[3];
+        u.row(2, r2);
+        a.column(2, col);
 #pragma unroll
-            for (int k = 0; k < 3; ++k) n2[k] = cmul(e2, r2[k]);
-            q2 = retr_row_fma(n2, col);
-        }
+        for (int k = 0; k < 3; ++k) n2[k] = cmul(p.e2, r2[k]);
+        const double q2 = diag ? retr_row_fma(n2, col) : (i2 == 2 ? rr[2] : (i2 == 1 ? rr[1] : rr[0]));
         const double s1 = (plain || g == 2) ? -s : s;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
@@ -673,10 +680,10 @@ k_su3_metropolis_ring(const ChainInfo *__restrict__ chains, const Tile *__restri
                 const Col<T> rows = column_of(s1.f[1]);
 #pragma unroll
                 for (int e = 0; e < 9; ++e) rows.put(e, u.e[e / 3][e % 3]);
-                accepted = visit_drawn<K>(rows, sa, beta3, angle, key);
+                accepted = visit_drawn<K>(rows, sa, beta3, key, DrawnStream<K>{key, angle});
                 u = staged_link(s1.f[1]);
             } else {
-                accepted = visit_ordered<K>(u, sa, beta3, angle, key, tr);
+                accepted = visit_ordered(u, sa, beta3, key, OrderedStream<K>{key, angle}, tr);
             }
 #pragma unroll
             for (int e = 0; e < 9; ++e)
