@@ -6,7 +6,7 @@ fewer items than CTAs, a second pass that only some CTAs take, items with
 idle threads and several chains per launch.  Resident: one CTA of 256 threads
 per chain, the staple sum in shared memory or (chains that leave no room for
 it) in local memory.  Both generator modes and both rotation lengths (half
-width <= 0.3 and above; 1.0 reaches lambda8's halved angles).  The plaquette
+width <= 0.4 and above; 1.0 reaches lambda8's halved angles).  The plaquette
 the sweep measures must agree with the oracle's to 1e-12.
 """
 import numpy as np
@@ -40,10 +40,10 @@ def _check(oracle, extents, chains, angle, mode, path):
 @pytest.mark.parametrize("mode", ["ordered", "uniform"])
 @pytest.mark.parametrize("extents,chains,angle", [
     ([2, 2, 2, 2], 1, 0.3),          # eight live threads
-    ([4, 4, 4, 6], 3, 0.35),         # 2 items per chain, the second half empty
+    ([4, 4, 4, 6], 3, 0.4),          # 2 items per chain, the second half empty
     ([4, 4, 4, 4], 2, 1.0),
     ([16, 16, 16, 20], 1, 0.3),      # 320 items: a partial second pass on 148 SMs
-    ([6, 6, 6, 10], 40, 0.35),       # 360 items of 40 chains, every ninth partial
+    ([6, 6, 6, 10], 40, 0.45),       # 360 items of 40 chains, every ninth partial
 ])
 def test_tiled_sweep_is_the_oracles(oracle, extents, chains, angle, mode):
     _check(oracle, extents, chains, angle, mode, "tiled")

@@ -136,3 +136,18 @@ def test_chains_without_the_stop_have_the_reference_bits():
         for i, d in enumerate((d1, d2)):
             c, s = _plain_chain(d * sc, K)
             assert np.array_equal(c, ref[0][i]) and np.array_equal(s, ref[1][i])
+
+
+def test_eleven_terms_serve_half_widths_up_to_04():
+    # t_12 <= 0.231^12 / 12! = 4.8e-17 is below half an ulp (2^-54) of the
+    # cosine sum, whichever generator; the grid's largest angles included
+    for a in (0.31, 0.35, 0.4):
+        theta = _grid_thetas(a, 1_000_000, 8)
+        for h in (0.5 * theta, (0.5 * INV_SQRT3) * theta, (-INV_SQRT3) * theta):
+            ref = _chains([h], 64)
+            c, s = _plain_chain(h, 11)
+            assert np.array_equal(c, ref[0][0]) and np.array_equal(s, ref[1][0])
+    top = np.linspace(0.4 - 1e-6, 0.4, 200_001)
+    ref = _chains([INV_SQRT3 * top], 64)
+    c, s = _plain_chain(INV_SQRT3 * top, 11)
+    assert np.array_equal(c, ref[0][0]) and np.array_equal(s, ref[1][0])

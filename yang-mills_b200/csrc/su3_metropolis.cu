@@ -298,7 +298,7 @@ static cudaError_t resident_launch(ym_ensemble *e, double angle, int64_t n_meas,
 
 cudaError_t launch_su3_resident(ym_ensemble *e, double angle, int uniform, int64_t n_meas,
                                 int64_t sweeps_per_meas, double *series) {
-    const bool small = angle <= 0.3;   // the rotation length, as in tiled_launch
+    const bool small = angle <= tiled_exact::kShortRotation;
     const cudaError_t err =
         uniform ? (small ? resident_launch<11, true>(e, angle, n_meas, sweeps_per_meas, series)
                          : resident_launch<14, true>(e, angle, n_meas, sweeps_per_meas, series))

@@ -89,7 +89,7 @@ __device__ __forceinline__ m3 staged_link(const double2 (*buf)[T]) {
 // Fast form only (YM_TILED_FAST): cos h and sin h as polynomials in
 // y = h^2 by Horner's rule with fused multiply-adds, the Taylor coefficients
 // 1/k! truncated where the next term is below 1e-19 for the half widths
-// served: through h^14 / h^15 for K <= 13 (|h| <= 0.173), through h^18 /
+// served: through h^14 / h^15 for K <= 13 (|h| <= 0.231), through h^18 /
 // h^19 above (|h| <= 0.578).
 template <int K>
 __device__ __forceinline__ void cos_sin_horner(double h, double &c, double &s) {
@@ -126,15 +126,17 @@ __device__ __forceinline__ void cos_sin_horner(double h, double &c, double &s) {
 //     select per term.  K is taken from the proposal half width a: |t_k| <=
 //     |h|^k / k! with |h| <= a/2 for generators 1..7 and |h| <= 0.5774 a (at
 //     most 0.5 after lambda8's halving) for generator 8, and terms past K
-//     must be below half an ulp too: for a <= 0.3, K = 11 (t_12 <=
-//     0.1732^12/12! = 1.5e-18 against sums near 0.985, t_13 / s <=
-//     0.1732^12/13! = 1.2e-19); for a <= 1, K = 14 (t_15 / s <= 0.5^14/15!
+//     must be below half an ulp too: for a <= 0.4, K = 11 (t_12 <=
+//     0.231^12/12! = 4.8e-17 < 2^-54 against sums in [0.97, 1), t_13 / s <=
+//     0.231^12/13! = 3.7e-18); for a <= 1, K = 14 (t_15 / s <= 0.5^14/15!
 //     = 4.7e-17 < 2^-54, t_16 <= 7.3e-19), so the sums are the reference's
 //     bit for bit (checked on the CPU against the loop run to the cutoff
 //     over millions of grid angles).
 //   * the decision is the reference's u < exp(-max(dS, 0))
 //     (su3_ensemble.rs:368) through accept_log; the accepted rows are
 //     selected, not branched to.
+constexpr double kShortRotation = 0.4;   // half widths that eleven terms serve
+
 template <int K>
 __device__ __forceinline__ void taylor_fixed(double h, double &c, double &s) {
     double t = h;      // k = 1: t = (1 h) 1, s = 0 + t
@@ -788,9 +790,9 @@ cudaError_t tiled_launch(ym_ensemble *e, int parity, int mu, double angle, int u
     // one touched last and finds its first waves' staple links in L2.  The
     // links of one sub-sweep are independent, so the order changes no bit.
     const int reverse = (parity * 4 + mu) & 1;
-    if (uniform && angle <= 0.3) metro_launch_ring<11, true>(e, parity, mu, angle, reverse);
+    if (uniform && angle <= kShortRotation) metro_launch_ring<11, true>(e, parity, mu, angle, reverse);
     else if (uniform) metro_launch_ring<14, true>(e, parity, mu, angle, reverse);
-    else if (angle <= 0.3) metro_launch_ring<11, false>(e, parity, mu, angle, reverse);
+    else if (angle <= kShortRotation) metro_launch_ring<11, false>(e, parity, mu, angle, reverse);
     else metro_launch_ring<14, false>(e, parity, mu, angle, reverse);
     return cudaGetLastError();
 }
@@ -800,7 +802,7 @@ cudaError_t tiled_launch(ym_ensemble *e, int parity, int mu, double angle, int u
 // tr_partial[cta] (the handle's layout must hold one chain per CTA).
 cudaError_t tiled_launch_measure(ym_ensemble *e, int mu, double angle, double *tr_partial) {
     if (cudaError_t err = configure_kernels()) return err;
-    if (angle <= 0.3) metro_launch_measure<11>(e, mu, angle, tr_partial);
+    if (angle <= kShortRotation) metro_launch_measure<11>(e, mu, angle, tr_partial);
     else metro_launch_measure<14>(e, mu, angle, tr_partial);
     return cudaGetLastError();
 }
