@@ -765,9 +765,9 @@ def main():
             "plaquette_mean": float(np.mean(plaq)),
             "acceptance": leg["acceptance"],
             "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e,
-            # measured steps: 8 sub-sweeps (3 measuring), sweep counter, reduction, series store;
+            # measured steps: 8 sub-sweeps (3 measuring), the reduction that stores the row;
             # per-launch steps: 8 sub-sweeps, sweep counter, plaquette, reduction
-            "gpu_launches": int((args.steps - leg["roofline"]["per_launch_steps"]) * 11
+            "gpu_launches": int((args.steps - leg["roofline"]["per_launch_steps"]) * 9
                                 + leg["roofline"]["per_launch_steps"] * 11),
             "clocks": leg["clocks"],
             "clocks_leg": dict(leg["clocks_leg"] or {}, note="every sample of the FP64 leg: "

@@ -199,6 +199,14 @@ size_t reals_per_link(const ym_ensemble *e) { return e->group == YM_GROUP_SU3 ? 
 
 bool f32(const ym_ensemble *e) { return e->precision == YM_PREC_F32_TWO_ROW; }
 
+// The sweep counter's entries (ym_internal.hpp).
+cudaError_t write_sweep_index(ym_ensemble *e, uint64_t sweep) {
+    uint64_t slots[ym::kSweepSlots];
+    for (int j = 0; j < ym::kSweepSlots; ++j) slots[j] = sweep + (uint64_t)j;
+    const cudaError_t err = cudaMemcpyAsync(e->d_sweep, slots, sizeof slots, cudaMemcpyHostToDevice, e->stream);
+    return err == cudaSuccess ? cudaStreamSynchronize(e->stream) : err;
+}
+
 cudaError_t identity(ym_ensemble *e) {
     if (f32(e)) return ym::launch_f32_identity(e);
     return e->group == YM_GROUP_SU3 ? ym::launch_su3_identity(e) : ym::launch_su2_identity(e);
@@ -522,7 +530,7 @@ int32_t ym_ensemble_create(const ym_ensemble_desc *desc, ym_ensemble **out) {
     if (err == cudaSuccess) err = dalloc(&e->d_result, (size_t)e->n_chains);
     if (err == cudaSuccess) err = dalloc(&e->d_result2, (size_t)e->n_chains);
     if (err == cudaSuccess) err = dalloc(&e->d_accepts, (size_t)e->n_chains);
-    if (err == cudaSuccess) err = dalloc(&e->d_sweep, 1);
+    if (err == cudaSuccess) err = dalloc(&e->d_sweep, ym::kSweepSlots + 1);
     if (err == cudaSuccess) err = dalloc(&e->d_rng, (size_t)e->n_chains);
     if (err == cudaSuccess) err = dalloc(&e->d_ref_counts, 2 * (size_t)e->n_chains);
     if (err == cudaSuccess) err = dalloc(&e->d_error, 1);
@@ -555,7 +563,8 @@ int32_t ym_ensemble_create(const ym_ensemble_desc *desc, ym_ensemble **out) {
     if (err == cudaSuccess)
         err = cudaMemcpy(e->d_site_tile_first, first.data(), first.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
     if (err == cudaSuccess) err = cudaMemset(e->d_accepts, 0, (size_t)e->n_chains * sizeof(unsigned long long));
-    if (err == cudaSuccess) err = cudaMemset(e->d_sweep, 0, sizeof(uint64_t));
+    if (err == cudaSuccess) err = cudaMemset(e->d_sweep + ym::kSweepSlots, 0, sizeof(uint64_t));
+    if (err == cudaSuccess) err = write_sweep_index(e, 0);
     if (err == cudaSuccess) err = identity(e);
     if (err == cudaSuccess) err = cudaStreamSynchronize(e->stream);
     if (err != cudaSuccess) {
@@ -634,8 +643,7 @@ int32_t ym_ensemble_set_sweep_index(ym_ensemble *e, uint64_t sweep) {
     if (!e) return YM_ERR_NULL_ARGUMENT;
     int32_t st = set_device(e);
     if (st) return st;
-    YM_CUDA(cudaMemcpyAsync(e->d_sweep, &sweep, sizeof sweep, cudaMemcpyHostToDevice, e->stream));
-    YM_CUDA(cudaStreamSynchronize(e->stream));
+    YM_CUDA(write_sweep_index(e, sweep));
     return YM_OK;
 }
 
@@ -829,16 +837,18 @@ static cudaError_t cadence_sweep(ym_ensemble *e, double angle, int mode, bool me
             if (err != cudaSuccess) return err;
         }
     cudaError_t err = f32(e) ? ym::launch_f32_reunitarize(e) : cudaSuccess;
-    return err == cudaSuccess ? ym::launch_advance_sweep(e) : err;
+    return err == cudaSuccess ? ym::count_sweep(e) : err;
 }
 
-// The average plaquette of every chain into d_result after cadence_sweep.
+// The average plaquette of every chain after cadence_sweep into the next row
+// of the device series.
 static cudaError_t cadence_plaquette(ym_ensemble *e, bool fused) {
     if (f32(e)) {
         cudaError_t err = ym::launch_f32_plaquette_partials(e);
-        return err == cudaSuccess ? ym::launch_chain_reduce(e, e->d_partial, e->d_result, 0, 6.0) : err;
+        return err == cudaSuccess ? ym::launch_chain_reduce(e, e->d_partial, e->d_result, 0, 6.0, e->d_series) : err;
     }
-    return fused ? ym::launch_su3_plaquette_from_sweep(e, e->d_tr_partial) : ym::launch_su3_plaquette(e);
+    return fused ? ym::launch_su3_plaquette_from_sweep(e, e->d_tr_partial, e->d_series)
+                 : ym::launch_su3_plaquette(e, e->d_series);
 }
 
 static cudaError_t ensure_series(ym_ensemble *e, int64_t n_measurements) {
@@ -881,13 +891,12 @@ int32_t ym_su3_measured_sweeps(ym_ensemble *e, double angle, int32_t generator_m
     YM_CUDA(cudaMemsetAsync(e->d_series_row, 0, sizeof(uint64_t), e->stream));
     const bool fused = sweeps_per_measurement > 0 && fused_plaquette(e, generator_mode);
     auto step = [&]() -> cudaError_t {
+        const ym::SweepSlotScope scope(e);
         for (int64_t k = 0; k < sweeps_per_measurement; ++k) {
             cudaError_t err = cadence_sweep(e, angle, generator_mode, fused && k == sweeps_per_measurement - 1);
             if (err != cudaSuccess) return err;
         }
-        cudaError_t err = cadence_plaquette(e, fused);
-        if (err == cudaSuccess) err = ym::launch_store_series(e, e->d_series, e->d_series_row);
-        return err;
+        return cadence_plaquette(e, fused);
     };
     // the captured cadence, made when the first row needs it (the
     // chain-resident kernel writes its rows itself)
@@ -1009,10 +1018,10 @@ int32_t ym_su3_measured_run(ym_ensemble *e, ym_ensemble *view, const ym_measured
     const double angle = run->proposal_angle;
     const bool fused = fused_plaquette(e, mode);
     auto block = [&]() -> cudaError_t {
+        const ym::SweepSlotScope scope(e);
         for (int64_t k = 0; k < spb; ++k) {
             cudaError_t err = cadence_sweep(e, angle, mode, fused);
             if (err == cudaSuccess) err = cadence_plaquette(e, fused);
-            if (err == cudaSuccess) err = ym::launch_store_series(e, e->d_series, e->d_series_row);
             if (err != cudaSuccess) return err;
         }
         cudaError_t err = m != e ? ym::launch_convert(e, m) : cudaSuccess;
@@ -1748,19 +1757,19 @@ int32_t ym_su2_measured_sweeps(ym_ensemble *e, int64_t max_attempts_per_link, in
     // one measurement: the sweeps of ym_su2_markov_sweeps, then the average
     // plaquette of every chain into the next row of the device series
     auto step = [&]() -> cudaError_t {
+        const ym::SweepSlotScope scope(e);
         cudaError_t err = cudaSuccess;
         for (int64_t k = 0; k < sweeps_per_measurement && err == cudaSuccess; ++k) {
             for (int parity = 0; parity < 2 && err == cudaSuccess; ++parity)
                 for (int mu = 0; mu < 4 && err == cudaSuccess; ++mu)
                     err = ym::launch_su2_heatbath(e, parity, mu, (int)max_attempts_per_link, sampler);
-            if (err == cudaSuccess) err = ym::launch_advance_sweep(e);
+            if (err == cudaSuccess) err = ym::count_sweep(e);
             for (int64_t o = 0; o < overrelaxation_sweeps && err == cudaSuccess; ++o)
                 for (int parity = 0; parity < 2 && err == cudaSuccess; ++parity)
                     for (int mu = 0; mu < 4 && err == cudaSuccess; ++mu) err = ym::launch_su2_overrelax(e, parity, mu);
         }
         if (err == cudaSuccess) err = ym::launch_su2_plaquette_partials(e);
-        if (err == cudaSuccess) err = ym::launch_chain_reduce(e, e->d_partial, e->d_result, 0, 6.0);
-        if (err == cudaSuccess) err = ym::launch_store_series(e, e->d_series, e->d_series_row);
+        if (err == cudaSuccess) err = ym::launch_chain_reduce(e, e->d_partial, e->d_result, 0, 6.0, e->d_series);
         return err;
     };
     const int64_t key[4] = {max_attempts_per_link, overrelaxation_sweeps, sampler, sweeps_per_measurement};
@@ -1963,9 +1972,10 @@ cudaError_t plain_uniform_sweep(ym_ensemble *e, double angle) {
             if (err != cudaSuccess) return err;
         }
     cudaError_t err = ym::launch_f32_reunitarize(e);
-    return err == cudaSuccess ? ym::launch_advance_sweep(e) : err;
+    return err == cudaSuccess ? ym::count_sweep(e) : err;
 }
 
+// (counted by count_sweep, as plain_uniform_sweep)
 cudaError_t learned_sweep(ym_ensemble *e, ym_proposal_model *m) {
     for (int parity = 0; parity < 2; ++parity)
         for (int mu = 0; mu < 4; ++mu) {
@@ -1973,7 +1983,7 @@ cudaError_t learned_sweep(ym_ensemble *e, ym_proposal_model *m) {
             if (err != cudaSuccess) return err;
         }
     cudaError_t err = timed(e, YM_KERNEL_AUX, [&] { return ym::launch_f32_reunitarize(e); });
-    return err == cudaSuccess ? ym::launch_advance_sweep(e) : err;
+    return err == cudaSuccess ? ym::count_sweep(e) : err;
 }
 
 int64_t half_sites(const ym_ensemble *e) {
@@ -2169,6 +2179,7 @@ int32_t ym_model_train(ym_proposal_model *m, ym_ensemble *e, int64_t n_steps, in
     YM_CUDA(ensure_objectives(m, n_steps));
     YM_CUDA(cudaStreamSynchronize(m->stream));   // model-stream work before ensemble-stream work
     const int64_t n_valid = half_sites(e);
+    const ym::SweepSlotScope scope(e);
     for (int64_t step = 0; step < n_steps; ++step) {
         for (int64_t k = 0; k < sweeps_per_step; ++k) YM_CUDA(plain_uniform_sweep(e, plain_angle));
         const int sub = (int)(step % 8);
@@ -2177,6 +2188,7 @@ int32_t ym_model_train(ym_proposal_model *m, ym_ensemble *e, int64_t n_steps, in
         YM_CUDA(ym::launch_lp_adam(m, e->n_half_tiles, n_valid, (float)lr, 1, nullptr,
                                    m->d_objective + step, e->stream));
     }
+    YM_CUDA(ym::launch_counted_sweeps(e));
     if (objective_history)
         YM_CUDA(cudaMemcpyAsync(objective_history, m->d_objective, sizeof(double) * (size_t)n_steps,
                                 cudaMemcpyDeviceToHost, e->stream));
@@ -2193,7 +2205,9 @@ int32_t ym_su3_learned_sweeps(ym_ensemble *e, ym_proposal_model *m, int64_t n_sw
     st = set_device(e);
     if (st) return st;
     YM_CUDA(cudaStreamSynchronize(m->stream));
+    const ym::SweepSlotScope scope(e);
     for (int64_t k = 0; k < n_sweeps; ++k) YM_CUDA(learned_sweep(e, m));
+    YM_CUDA(ym::launch_counted_sweeps(e));
     for (int64_t ch = 0; ch < e->n_chains; ++ch)
         e->proposals[ch] += (uint64_t)n_sweeps * 32u * (uint64_t)e->chains[ch].volume;
     return take_model_error(m, e->stream);
@@ -2211,11 +2225,11 @@ int32_t ym_su3_learned_measured_sweeps(ym_ensemble *e, ym_proposal_model *m, int
     YM_CUDA(cudaStreamSynchronize(m->stream));
     YM_CUDA(ensure_series(e, n_measurements));
     YM_CUDA(cudaMemsetAsync(e->d_series_row, 0, sizeof(uint64_t), e->stream));
+    const ym::SweepSlotScope scope(e);
     for (int64_t meas = 0; meas < n_measurements; ++meas) {
         for (int64_t k = 0; k < sweeps_per_measurement; ++k) YM_CUDA(learned_sweep(e, m));
         YM_CUDA(ym::launch_f32_plaquette_partials(e));
-        YM_CUDA(ym::launch_chain_reduce(e, e->d_partial, e->d_result, 0, 6.0));
-        YM_CUDA(ym::launch_store_series(e, e->d_series, e->d_series_row));
+        YM_CUDA(ym::launch_chain_reduce(e, e->d_partial, e->d_result, 0, 6.0, e->d_series));
     }
     YM_CUDA(cudaMemcpyAsync(series, e->d_series, (size_t)(n_measurements * e->n_chains) * sizeof(double),
                             cudaMemcpyDeviceToHost, e->stream));

@@ -813,10 +813,10 @@ cudaError_t launch_lp_sweep(ym_ensemble *e, ym_proposal_model *m, int parity, in
     const uint4 *img = reinterpret_cast<const uint4 *>(m->d_image);
     const uint32_t sm = lp::FwdLayout::BYTES;
     switch (mu) {
-        case 0: lp::k_lp_sweep<0><<<grid, lp::kRows, sm, e->stream>>>(e->d_chains, e->d_half_tiles, n, links, parity, img, m->d_params, e->d_sweep, e->d_accepts, m->d_error); break;
-        case 1: lp::k_lp_sweep<1><<<grid, lp::kRows, sm, e->stream>>>(e->d_chains, e->d_half_tiles, n, links, parity, img, m->d_params, e->d_sweep, e->d_accepts, m->d_error); break;
-        case 2: lp::k_lp_sweep<2><<<grid, lp::kRows, sm, e->stream>>>(e->d_chains, e->d_half_tiles, n, links, parity, img, m->d_params, e->d_sweep, e->d_accepts, m->d_error); break;
-        default: lp::k_lp_sweep<3><<<grid, lp::kRows, sm, e->stream>>>(e->d_chains, e->d_half_tiles, n, links, parity, img, m->d_params, e->d_sweep, e->d_accepts, m->d_error); break;
+        case 0: lp::k_lp_sweep<0><<<grid, lp::kRows, sm, e->stream>>>(e->d_chains, e->d_half_tiles, n, links, parity, img, m->d_params, sweep_index(e), e->d_accepts, m->d_error); break;
+        case 1: lp::k_lp_sweep<1><<<grid, lp::kRows, sm, e->stream>>>(e->d_chains, e->d_half_tiles, n, links, parity, img, m->d_params, sweep_index(e), e->d_accepts, m->d_error); break;
+        case 2: lp::k_lp_sweep<2><<<grid, lp::kRows, sm, e->stream>>>(e->d_chains, e->d_half_tiles, n, links, parity, img, m->d_params, sweep_index(e), e->d_accepts, m->d_error); break;
+        default: lp::k_lp_sweep<3><<<grid, lp::kRows, sm, e->stream>>>(e->d_chains, e->d_half_tiles, n, links, parity, img, m->d_params, sweep_index(e), e->d_accepts, m->d_error); break;
     }
     return cudaGetLastError();
 }

@@ -184,11 +184,7 @@ __global__ void k_tile_mean(const double *__restrict__ partial, const int32_t *_
                             double *__restrict__ out) {
     const int chain = blockIdx.x, k = blockIdx.y;
     const int b = first[chain], e = first[chain + 1];
-    double v = 0.0;
-    for (int i = b + threadIdx.x; i < e; i += blockDim.x) {
-        const double p = partial[(int64_t)i * width + k];
-        v = (i == b + (int)threadIdx.x) ? p : v + p;
-    }
+    double v = strided_sum(b, e, [&](int i) { return partial[(int64_t)i * width + k]; });
     v = block_reduce<false>(v);
     if (threadIdx.x == 0) {
         const ChainInfo &c = chains[chain];
@@ -339,26 +335,27 @@ k_operator_sites(const ChainInfo *__restrict__ chains, const Tile *__restrict__ 
 __global__ void k_operator_reduce(const ChainInfo *__restrict__ chains, const int32_t *__restrict__ slice_chain,
                                   const int32_t *__restrict__ slice_t, const double2 *__restrict__ site_vals,
                                   double *__restrict__ out_plaq, double *__restrict__ out_rect) {
-    __shared__ double red[2][8];
+    __shared__ double red[2][32];
     const int slice = blockIdx.x;
     const ChainInfo c = chains[slice_chain[slice]];
     const int t = slice_t[slice];
-    const int64_t vs = (int64_t)c.n[0] * c.n[1] * c.n[2];
+    const uint32_t n1 = c.n[1], n2 = c.n[2];
+    const uint32_t vs = (uint32_t)c.n[0] * n1 * n2;
+    const double2 *vals = site_vals + c.offset / 36;
     double p = 0.0, r = 0.0;
-    bool first = true;
-    for (int64_t i = threadIdx.x; i < vs; i += blockDim.x) {
-        const int64_t lex = i * c.n[3] + t;
-        int32_t x[4];
-        int64_t q = i;
-        x[2] = (int32_t)(q % c.n[2]); q /= c.n[2];
-        x[1] = (int32_t)(q % c.n[1]);
-        x[0] = (int32_t)(q / c.n[1]);
-        x[3] = t;
-        const int par = (x[0] + x[1] + x[2] + x[3]) & 1;
-        const double2 v = site_vals[c.offset / 36 + storage_index(c, lex, par)];
-        p = first ? v.x : p + v.x;
-        r = first ? v.y : r + v.y;
-        first = false;
+    // four sites in flight
+    for (uint32_t i0 = threadIdx.x; i0 < vs; i0 += 4 * blockDim.x) {
+        double2 v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t i = i0 + j * blockDim.x;
+            const uint32_t row = i / n2, x0 = row / n1;
+            const int par = ((i - row * n2) + (row - x0 * n1) + x0 + t) & 1;
+            v[j] = make_double2(0.0, 0.0);
+            if (i < vs) v[j] = vals[storage_index(c, (int64_t)i * c.n[3] + t, par)];
+        }
+        p += (v[0].x + v[1].x) + (v[2].x + v[3].x);
+        r += (v[0].y + v[1].y) + (v[2].y + v[3].y);
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
@@ -376,8 +373,8 @@ __global__ void k_operator_reduce(const ChainInfo *__restrict__ chains, const in
             a += red[0][w];
             b += red[1][w];
         }
-        out_plaq[slice] = a / (double)(3 * vs);
-        out_rect[slice] = b / (double)(6 * vs);
+        out_plaq[slice] = a / (3.0 * (double)vs);
+        out_rect[slice] = b / (6.0 * (double)vs);
     }
 }
 
@@ -420,7 +417,10 @@ cudaError_t launch_operator_basis(ym_ensemble *e, double2 *d_site_vals, const in
                                   double *d_rect, const double2 *links) {
     k_operator_sites<<<(unsigned)e->n_site_tiles, T, 0, e->stream>>>(e->d_chains, e->d_site_tiles,
                                                                     links ? links : e->d_links, d_site_vals);
-    k_operator_reduce<<<(unsigned)n_slices, 256, 0, e->stream>>>(e->d_chains, d_slice_chain, d_slice_t,
+    // a round of a block takes four sites per thread; slices of more than
+    // 1024 sites get blocks of 1024 threads
+    const int threads = (int64_t)e->n_site_tiles * T > 1024 * n_slices ? 1024 : 256;
+    k_operator_reduce<<<(unsigned)n_slices, threads, 0, e->stream>>>(e->d_chains, d_slice_chain, d_slice_t,
                                                                 d_site_vals, d_plaq, d_rect);
     return cudaGetLastError();
 }

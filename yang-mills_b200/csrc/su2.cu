@@ -543,19 +543,19 @@ cudaError_t launch_su2_heatbath(ym_ensemble *e, int parity, int mu, int max_atte
     if (su2_grouped(e)) {
         const dim3 g((unsigned)(e->n_half_tiles * kGroup));
         switch (mu) {
-        case 0: k_su2_heatbath_group<0><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, max_attempts, kp, e->d_sweep, e->d_accepts, e->d_error); break;
-        case 1: k_su2_heatbath_group<1><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, max_attempts, kp, e->d_sweep, e->d_accepts, e->d_error); break;
-        case 2: k_su2_heatbath_group<2><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, max_attempts, kp, e->d_sweep, e->d_accepts, e->d_error); break;
-        default: k_su2_heatbath_group<3><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, max_attempts, kp, e->d_sweep, e->d_accepts, e->d_error); break;
+        case 0: k_su2_heatbath_group<0><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, max_attempts, kp, sweep_index(e), e->d_accepts, e->d_error); break;
+        case 1: k_su2_heatbath_group<1><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, max_attempts, kp, sweep_index(e), e->d_accepts, e->d_error); break;
+        case 2: k_su2_heatbath_group<2><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, max_attempts, kp, sweep_index(e), e->d_accepts, e->d_error); break;
+        default: k_su2_heatbath_group<3><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, max_attempts, kp, sweep_index(e), e->d_accepts, e->d_error); break;
         }
         return cudaGetLastError();
     }
     const dim3 g((unsigned)e->n_half_tiles);
     switch (mu) {
-    case 0: k_su2_heatbath_thread<0><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, max_attempts, kp, e->d_sweep, e->d_accepts, e->d_error); break;
-    case 1: k_su2_heatbath_thread<1><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, max_attempts, kp, e->d_sweep, e->d_accepts, e->d_error); break;
-    case 2: k_su2_heatbath_thread<2><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, max_attempts, kp, e->d_sweep, e->d_accepts, e->d_error); break;
-    default: k_su2_heatbath_thread<3><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, max_attempts, kp, e->d_sweep, e->d_accepts, e->d_error); break;
+    case 0: k_su2_heatbath_thread<0><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, max_attempts, kp, sweep_index(e), e->d_accepts, e->d_error); break;
+    case 1: k_su2_heatbath_thread<1><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, max_attempts, kp, sweep_index(e), e->d_accepts, e->d_error); break;
+    case 2: k_su2_heatbath_thread<2><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, max_attempts, kp, sweep_index(e), e->d_accepts, e->d_error); break;
+    default: k_su2_heatbath_thread<3><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, max_attempts, kp, sweep_index(e), e->d_accepts, e->d_error); break;
     }
     return cudaGetLastError();
 }

@@ -272,7 +272,7 @@ float2 *f32_links(ym_ensemble *e) { return reinterpret_cast<float2 *>(e->d_links
 template <bool DRAWN>
 static cudaError_t launch_f32_form(ym_ensemble *e, int parity, int mu, double angle, int reverse) {
     k_f32_metropolis<DRAWN><<<(unsigned)e->n_half_tiles, T, kRingF, e->stream>>>(
-        e->d_chains, e->d_half_tiles, single_chain(e), f32_links(e), parity, mu, angle, e->d_sweep, e->d_accepts, reverse);
+        e->d_chains, e->d_half_tiles, single_chain(e), f32_links(e), parity, mu, angle, sweep_index(e), e->d_accepts, reverse);
     return cudaGetLastError();
 }
 

@@ -237,9 +237,8 @@ k_su3_resident(const ChainInfo *__restrict__ chains, double2 *__restrict__ links
     if ((threadIdx.x & 31) == 0 && sum) atomicAdd(accepts + chain, (unsigned long long)sum);
 }
 
-__global__ void k_advance_sweep_by(uint64_t *sweep, int64_t n) { *sweep += (uint64_t)n; }
-
-__global__ void k_advance_sweep(uint64_t *sweep) { *sweep += 1; }
+// (kSweepSlots threads)
+__global__ void k_advance_sweep(uint64_t *sweep, uint64_t n) { sweep[threadIdx.x] += n; }
 
 }  // namespace
 
@@ -292,7 +291,7 @@ static cudaError_t resident_launch(ym_ensemble *e, double angle, int64_t n_meas,
     const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
     kernel<<<(unsigned)e->n_chains, kResidentThreads, smem, e->stream>>>(
-        e->d_chains, e->d_links, angle, e->d_sweep, n_meas, sweeps_per_meas, series, e->n_chains, e->d_accepts);
+        e->d_chains, e->d_links, angle, sweep_index(e), n_meas, sweeps_per_meas, series, e->n_chains, e->d_accepts);
     return cudaGetLastError();
 }
 
@@ -305,13 +304,20 @@ cudaError_t launch_su3_resident(ym_ensemble *e, double angle, int uniform, int64
                 : (small ? resident_launch<11, false>(e, angle, n_meas, sweeps_per_meas, series)
                          : resident_launch<14, false>(e, angle, n_meas, sweeps_per_meas, series));
     if (err != cudaSuccess) return err;
-    k_advance_sweep_by<<<1, 1, 0, e->stream>>>(e->d_sweep, n_meas * sweeps_per_meas);
+    k_advance_sweep<<<1, kSweepSlots, 0, e->stream>>>(e->d_sweep, (uint64_t)(n_meas * sweeps_per_meas));
+    return cudaGetLastError();
+}
+
+cudaError_t launch_counted_sweeps(ym_ensemble *e) {
+    if (e->sweep_slot == 0) return cudaSuccess;
+    k_advance_sweep<<<1, kSweepSlots, 0, e->stream>>>(e->d_sweep, (uint64_t)e->sweep_slot);
+    e->sweep_slot = 0;
     return cudaGetLastError();
 }
 
 cudaError_t launch_advance_sweep(ym_ensemble *e) {
-    k_advance_sweep<<<1, 1, 0, e->stream>>>(e->d_sweep);
-    return cudaGetLastError();
+    ++e->sweep_slot;
+    return launch_counted_sweeps(e);
 }
 
 }  // namespace ym

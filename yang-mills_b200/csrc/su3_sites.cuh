@@ -15,6 +15,24 @@ __device__ __forceinline__ m3 link_at(const double2 *links, const ChainInfo &c, 
     return RESIDENT ? load_su3_rw(links, c, s, mu) : load_su3(links, c, s, mu);
 }
 
+// Thread's share of the sum of at(b) .. at(e - 1), entries threadIdx.x,
+// threadIdx.x + blockDim.x, ... of the range in a fixed order.  The chain of
+// dependent loads bounds these sums (a few blocks, no more work per SM than
+// that), so four entries are in flight: 5184 tiles 14 -> 5 us (1024 threads,
+// 256 before), 32^4's 12288 shares of three planes 14 -> 12, the operators of
+// 2560 slices of 64 to 512 sites 19 -> 13.
+template <class At>
+__device__ __forceinline__ double strided_sum(int b, int e, At at) {
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int i = b + threadIdx.x; i < e; i += 4 * blockDim.x)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int k = i + j * blockDim.x;
+            if (k < e) a[j] += at(k);
+        }
+    return (a[0] + a[1]) + (a[2] + a[3]);
+}
+
 // Fixed-shape block reduction: a shuffle-down tree within each warp, then
 // the warp results (zeros past the last warp) by the same tree in warp 0.
 // The result is valid in thread 0.

@@ -736,7 +736,7 @@ void metro_launch_ring(ym_ensemble *e, int parity, int mu, double angle, int rev
     const SweepLayout &L = e->layouts[e->sweep_layout];
     const dim3 grid(ring_grid(L.ctas)), block(T);
     k_su3_metropolis_ring<K, false, DRAWN><<<grid, block, kRingBytes, e->stream>>>(
-        e->d_chains, L.d_items, (int)L.ctas, single_chain(e), e->d_links, parity, mu, angle, e->d_sweep, e->d_accepts, L.log2_item,
+        e->d_chains, L.d_items, (int)L.ctas, single_chain(e), e->d_links, parity, mu, angle, sweep_index(e), e->d_accepts, L.log2_item,
         reverse, nullptr);
 }
 
@@ -749,7 +749,7 @@ void metro_launch_measure(ym_ensemble *e, int mu, double angle, double *tr_parti
     const dim3 g(ring_grid(L.ctas)), b(T);
     const int rev = (1 * 4 + mu) & 1;   // the tile order tiled_launch gives (parity 1, mu)
     k_su3_metropolis_ring<K, true, false><<<g, b, kRingBytes, e->stream>>>(
-        e->d_chains, L.d_items, (int)L.ctas, single_chain(e), e->d_links, 1, mu, angle, e->d_sweep, e->d_accepts, L.log2_item, rev,
+        e->d_chains, L.d_items, (int)L.ctas, single_chain(e), e->d_links, 1, mu, angle, sweep_index(e), e->d_accepts, L.log2_item, rev,
         tr_partial);
 }
 

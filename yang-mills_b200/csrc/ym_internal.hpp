@@ -15,6 +15,7 @@ namespace ym {
 constexpr int kSweepThreads = 128;   // threads per tile of a sub-sweep
 constexpr int kSweepWarps = kSweepThreads / 32;
 constexpr int kSiteThreads = 128;    // threads per tile of a measurement
+constexpr int kSweepSlots = 32;      // sweeps of a cadence between two advances of the sweep counter
 constexpr int64_t kLpPartialStride = 6304;  // floats per tile of learned-proposal gradient partials
 // Groups of 64 tiles in the first stage of the gradient reduction.
 inline int64_t lp_reduce_groups(int64_t tiles) { return (tiles + 63) / 64; }
@@ -73,7 +74,8 @@ struct ym_ensemble {
     unsigned long long *d_accepts = nullptr;   // SU(3) accepts / SU(2) heat-bath attempts
     unsigned *d_error = nullptr;               // device error bits (bounded loops that gave up)
     double *d_tr_partial = nullptr;            // 3 x CTAs x kSweepWarps: plaquette shares of a measured sweep
-    uint64_t *d_sweep = nullptr;           // next sweep index
+    uint64_t *d_sweep = nullptr;           // kSweepSlots: next sweep index + j in entry j; then end_row's ticket
+    int sweep_slot = 0;                    // sweeps of the cadence being launched that the entries don't count yet
     uint64_t *d_rng = nullptr;             // reference-replay stream states
     unsigned long long *d_ref_counts = nullptr;  // reference replay: proposals, accepts
     std::vector<uint64_t> proposals;       // host-counted proposals per chain
@@ -159,6 +161,9 @@ struct ym_ensemble {
     size_t events_used[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 };
 
+// Device pointer to the index of the sweep being launched.
+inline const uint64_t *sweep_index(const ym_ensemble *e) { return e->d_sweep + e->sweep_slot; }
+
 // The geometry of a handle of one chain, else an empty one (block_of).
 inline ym::ChainInfo single_chain(const ym_ensemble *e) {
     return e->n_chains == 1 ? e->chains[0] : ym::ChainInfo{};
@@ -222,23 +227,41 @@ cudaError_t launch_su3_metropolis_measure(ym_ensemble *e, int mu, double angle, 
 cudaError_t launch_su3_metropolis_measure_fast(ym_ensemble *e, int mu, double angle, double *tr_partial);
 // After a sweep whose last three sub-sweeps measured into tr_partial
 // (three arrays of the layout's CTA count): each chain's average plaquette
-// into d_result.
-cudaError_t launch_su3_plaquette_from_sweep(ym_ensemble *e, const double *tr_partial);
+// into d_result.  (series: see launch_chain_reduce.)
+cudaError_t launch_su3_plaquette_from_sweep(ym_ensemble *e, const double *tr_partial, double *series = nullptr);
+// The deferred sweeps onto the device's sweep counter.
+cudaError_t launch_counted_sweeps(ym_ensemble *e);
+// Counts the sweep just launched (and those deferred) on the device.
 cudaError_t launch_advance_sweep(ym_ensemble *e);
+// Counts the sweep just launched; the device's counter follows with the row
+// that ends the cadence, with launch_counted_sweeps, or here every kSweepSlots.
+inline cudaError_t count_sweep(ym_ensemble *e) {
+    if (e->sweep_slot + 1 == kSweepSlots) return launch_advance_sweep(e);
+    ++e->sweep_slot;
+    return cudaSuccess;
+}
+// Sweeps that an abandoned cadence deferred are not carried into the next.
+struct SweepSlotScope {
+    ym_ensemble *e;
+    explicit SweepSlotScope(ym_ensemble *e_) : e(e_) { e->sweep_slot = 0; }
+    ~SweepSlotScope() { e->sweep_slot = 0; }
+};
 // Chain-resident sweeps (su3_metropolis.cu): every chain small enough that
 // its links fit in one CTA's shared memory.  series (device, may be null)
 // receives the plaquette of every chain after each group of sweeps.
 bool resident_fits(const ym_ensemble *e);
 cudaError_t launch_su3_resident(ym_ensemble *e, double angle, int uniform, int64_t n_meas,
                                 int64_t sweeps_per_meas, double *series);
-cudaError_t launch_su3_plaquette(ym_ensemble *e);
+cudaError_t launch_su3_plaquette(ym_ensemble *e, double *series = nullptr);
 cudaError_t launch_su3_residuals(ym_ensemble *e);
 cudaError_t launch_su3_reference_sweeps(ym_ensemble *e, double angle, int64_t n_sweeps);
 cudaError_t launch_su3_reference_plaquette(ym_ensemble *e);
 cudaError_t launch_su3_hot_start(ym_ensemble *e);
+// series (device, may be null): the same launch also ends the row of a
+// cadence -- the results into row *d_series_row of series, that counter
+// advanced by one and the sweep counter by the sweeps deferred.
 cudaError_t launch_chain_reduce(ym_ensemble *e, const double *partial, double *out, int mode,
-                                double per_site);
-cudaError_t launch_store_series(ym_ensemble *e, double *series, uint64_t *counter);
+                                double per_site, double *series = nullptr);
 // Row *counter of dst (rows of n doubles) = src; advance bumps the counter.
 cudaError_t launch_store_rows(cudaStream_t st, const double *src, int64_t n, double *dst,
                               uint64_t *counter, int advance);
