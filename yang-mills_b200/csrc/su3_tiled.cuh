@@ -22,11 +22,10 @@
 //     recurrence (ym_ensemble_set_fast_sweeps).
 //
 // Layout: every factor of the six staple terms is copied global -> shared by
-// cp.async ahead of its use.  Ordered hits (k_su3_metropolis_ring) keep the
-// staple accumulator in registers and stage two terms ahead, two persistent
-// 128-thread blocks per SM; drawn generators (k_su3_metropolis) keep it in shared
-// memory (nine double2 per thread, conflict-free column layout) and stage
-// one term ahead, three blocks per SM.
+// cp.async ahead of its use.  k_su3_metropolis_ring keeps the staple
+// accumulator in registers and stages two terms ahead, two persistent
+// 128-thread blocks per SM; for the hits the accumulator goes to shared
+// memory (nine double2 per thread, conflict-free column layout).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -475,10 +474,10 @@ __device__ __forceinline__ unsigned visit_drawn(const U &u, const A &a, double b
     return accepted;
 }
 
-// ---- ordered hits: two staple terms in flight, two CTAs per SM -----------
-// The ordered-hit sub-sweep keeps the staple accumulator in registers and a
+// ---- the sub-sweep: two staple terms in flight, two CTAs per SM ----------
+// The sub-sweep keeps the staple accumulator in registers and a
 // ring of two three-factor staging sets, so term k+2's factors are loading
-// while term k multiplies (one term ahead in k_su3_metropolis).  Two
+// while term k multiplies.  Two
 // 128-thread CTAs per SM fit (registers and 108 KB of staging each); after
 // the staple the accumulator is written once to the second set's memory for
 // the hits.  The products and their order are staple_pipelined's, so A has
@@ -494,12 +493,13 @@ __device__ __forceinline__ unsigned visit_drawn(const U &u, const A &a, double b
 // instruction on a 32^4 lattice, half width 0.3: unrolled and one tile per
 // CTA 1.57 cycles on loads + 0.40 on instruction fetch (168 us per launch
 // under the profiler), persistent unrolled 0.85-1.13 + 0.52-0.91 (169 us),
-// persistent with looped directions 0.76 + 0.12 (161 us, hits looped too).
+// persistent with looped directions 0.76 + 0.12 (161 us, hits looped too;
+// with the ordered hits unrolled again 155).
 // Three CTAs per SM (one term ahead, 168 registers with 150 bytes spilled):
 // 1.52 + 0.62, 180 us.  Sweep live, start of this design -> now, same
 // boxes: 32^4 1487 -> 1319 us at half width 0.3 (of which the shorter
-// rotations and accept_log 6 %), 16^4 103 -> 92, 8^4 88 -> 76, 32 chains of
-// 6^3 x 10 130 -> 121; drawn generators 2409 -> 1755 (32^4), 230 -> 135 (16^4).
+// rotations and accept_log 6 %), 16^4 103 -> 90, 8^4 88 -> 73, 32 chains of
+// 6^3 x 10 130 -> 120; drawn generators 2409 -> 1709 (32^4), 230 -> 132 (16^4).
 struct TermSet {
     double2 (*f[3])[T];
 };
@@ -780,9 +780,8 @@ cudaError_t configure_kernels() {
     return cudaSuccess;
 }
 
-// One sub-sweep of the handle: ordered hits on the ring kernel with the
-// term count the half width allows (angles are validated to lie in
-// [1e-8, 1] for binary64 handles), drawn generators on the three-CTA kernel.
+// One sub-sweep of the handle with the term count the half width allows
+// (angles are validated to lie in [1e-8, 1] for binary64 handles).
 cudaError_t tiled_launch(ym_ensemble *e, int parity, int mu, double angle, int uniform) {
     if (cudaError_t err = configure_kernels()) return err;
     // Consecutive sub-sweeps walk the lattice in opposite directions (odd
