@@ -69,35 +69,37 @@ __device__ __forceinline__ q4 qdag_if(const q4 &a, bool d) {
     return q4{{a.c[0], s * a.c[1], s * a.c[2], s * a.c[3]}};
 }
 
-// Term j of the staple of link (x, MU):
+// The three links of term j of the staple of link (x, mu):
 //   forward  U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag
 //   backward U_nu(x-nu+mu)^dag U_mu(x-nu)^dag U_nu(x-nu)
-template <int MU>
-__device__ __forceinline__ q4 su2_staple_term(const double2 *__restrict__ links, const ChainInfo &c,
-                                              const Coord &x, int par, int j) {
+// mu is a run-time value, so one copy of the code serves a sweep's launches.
+struct TermLinks {
+    q4 a, b, c;
+    bool fwd;
+};
+
+__device__ __forceinline__ TermLinks su2_term_links(const double2 *__restrict__ links, const ChainInfo &c,
+                                                    const Site &x, int par, int mu, int j) {
     const int k = j >> 1;
-    const int nu = k < MU ? k : k + 1;
-    const bool fwd = (j & 1) == 0;
-    const Nb pm = step(c, x.x, x.lex, par, MU, +1);
-    const Nb pn = step_any(c, x.x, x.lex, par, nu, +1);
-    const Nb mn = step_any(c, x.x, x.lex, par, nu, -1);
-    const Nb mnpm = step(c, x.x, mn.lex, mn.par, MU, +1);   // x - nu keeps x's mu coordinate
-    const Nb sa = fwd ? pm : mnpm, sb = fwd ? pn : mn, sc = fwd ? Nb{x.lex, par} : mn;
-    const q4 a = qdag_if(link_q(links, c, sa, nu), !fwd);
-    const q4 b = qdag(link_q(links, c, sb, MU));
-    const q4 cc = qdag_if(link_q(links, c, sc, nu), fwd);
-    return qmul(qmul(a, b), cc);
+    const int nu = k < mu ? k : k + 1;
+    const int32_t same = par ? x.half : 0, other = par ? 0 : x.half;
+    const int32_t up = pick(x.fwd, mu);
+    TermLinks t;
+    t.fwd = (j & 1) == 0;
+    const int32_t beside = x.lex + (t.fwd ? pick(x.fwd, nu) : pick(x.bwd, nu));   // x + nu or x - nu
+    t.a = load_q(links, c, t.fwd ? other + ((x.lex + up) >> 1) : same + ((beside + up) >> 1), nu);
+    t.b = load_q(links, c, other + (beside >> 1), mu);
+    t.c = load_q(links, c, t.fwd ? same + (x.lex >> 1) : other + (beside >> 1), nu);
+    return t;
 }
 
 // The group's staple sum (every lane of the group gets it): terms computed
-// by lanes 0..5 of the group (`active` false: the group's lanes load nothing
-// and the sum is meaningless), added in term order.
-template <int MU>
-__device__ __forceinline__ void su2_staple_group(const double2 *__restrict__ links, const ChainInfo &c,
-                                                 const Coord &x, int par, bool active, double comp[4]) {
+// by lanes 0..5 of the group from the links they hold (`active` false: the
+// sum is meaningless), added in term order.
+__device__ __forceinline__ void su2_staple_group(const TermLinks &l, bool active, double comp[4]) {
     const int lane = threadIdx.x & 31, j = lane & (kGroup - 1), base = lane - j;
     q4 term{{0.0, 0.0, 0.0, 0.0}};
-    if (active && j < 6) term = su2_staple_term<MU>(links, c, x, par, j);
+    if (active && j < 6) term = qmul(qmul(qdag_if(l.a, !l.fwd), qdag(l.b)), qdag_if(l.c, l.fwd));
     comp[0] = comp[1] = comp[2] = comp[3] = 0.0;
 #pragma unroll
     for (int jj = 0; jj < 6; ++jj)
@@ -158,25 +160,39 @@ __device__ __forceinline__ bool sample_reference(double alpha, uint64_t key, int
 // exp(alpha r0) sqrt(1 - r0^2): x = -(ln u1 + cos^2(2 pi u2) ln u3)/alpha,
 // accept if u4^2 <= 1 - x/2, r0 = 1 - x.  Uniforms in (0, 1].  The direction
 // after the loop, as above.
-__device__ __forceinline__ bool sample_kp(double alpha, uint64_t key, int max_attempts, q4 &out,
+//
+// An attempt's draws do not know alpha: `first` is the first attempt's, which
+// a caller can make while it waits for the staple's links.
+struct KpDraw {
+    double num, u4;   // x = num / alpha
+};
+
+__device__ __forceinline__ KpDraw kp_draw(uint64_t key, uint64_t j) {
+    const double u1 = 1.0 - unit_from(splitmix_at(key, j));
+    const double u2 = unit_from(splitmix_at(key, j + 1));
+    const double u3 = 1.0 - unit_from(splitmix_at(key, j + 2));
+    const double u4 = unit_from(splitmix_at(key, j + 3));
+    const double cs = cospi(2.0 * u2);
+    return KpDraw{-(log(u1) + cs * cs * log(u3)), u4};
+}
+
+__device__ __forceinline__ bool sample_kp(double alpha, uint64_t key, const KpDraw &first, int max_attempts, q4 &out,
                                           int &attempts) {
-    uint64_t j = 0;
     if (alpha <= kAlphaZeroLimit) return sample_reference(alpha, key, max_attempts, out, attempts);
     double x = 0.0;
     bool found = false;
     int a = 1;
-    for (; a <= max_attempts; ++a) {
-        const double u1 = 1.0 - unit_from(splitmix_at(key, j++));
-        const double u2 = unit_from(splitmix_at(key, j++));
-        const double u3 = 1.0 - unit_from(splitmix_at(key, j++));
-        const double u4 = unit_from(splitmix_at(key, j++));
-        const double cs = cospi(2.0 * u2);
-        x = -(log(u1) + cs * cs * log(u3)) / alpha;
-        if (u4 * u4 <= 1.0 - 0.5 * x) {
+    KpDraw d = first;
+    for (;;) {
+        x = d.num / alpha;
+        if (d.u4 * d.u4 <= 1.0 - 0.5 * x) {
             found = true;
             break;
         }
+        if (++a > max_attempts) break;
+        d = kp_draw(key, 4 * (uint64_t)(a - 1));
     }
+    const uint64_t j = 4 * (uint64_t)a;
     attempts = found ? a : max_attempts;
     if (!found) return false;
     const double r0 = 1.0 - x;
@@ -227,7 +243,7 @@ k_su2_heatbath_thread(const ChainInfo *__restrict__ chains, const Tile *__restri
             const uint64_t key = link_key(c.seed, *sweep_ptr, x.lex, MU);
             q4 r;
             int att = 0;
-            const bool ok = kp ? sample_kp(alpha, key, max_attempts, r, att)
+            const bool ok = kp ? sample_kp(alpha, key, kp_draw(key, 0), max_attempts, r, att)
                                : sample_reference(alpha, key, max_attempts, r, att);
             attempts_used = (unsigned)att;
             if (!ok) {
@@ -258,6 +274,7 @@ k_su2_overrelax_thread(const ChainInfo *__restrict__ chains, const Tile *__restr
     if (t >= c.half) return;
     const int64_t s = (int64_t)parity * c.half + t;
     const Coord x = decode_storage(c, s);
+    const q4 u = load_q_rw(links, c, s, MU);
     double comp[4];
     su2_staple<MU>(links, c, x, parity, comp);
     const double norm = staple_norm(comp);
@@ -269,7 +286,7 @@ k_su2_overrelax_thread(const ChainInfo *__restrict__ chains, const Tile *__restr
     q4 vhat;
     normalize_scaled<4>(comp, vhat.c);
     const q4 nd = qdag(vhat);
-    store_q(links, c, s, MU, qmul(qmul(nd, qdag(load_q_rw(links, c, s, MU))), nd));
+    store_q(links, c, s, MU, qmul(qmul(nd, qdag(u)), nd));
 }
 
 // Grouped form (small sub-sweeps, latency-bound: a 10^4 lattice updates
@@ -277,10 +294,15 @@ k_su2_overrelax_thread(const ChainInfo *__restrict__ chains, const Tile *__restr
 // One block: kGroupLinks links of the tile blockIdx.x / kGroup (sub-block
 // blockIdx.x % kGroup), kGroup lanes per link; the update is evaluated by
 // every lane of the group alike and written by its first lane.
-template <int MU>
+// What bounds it: the launch and one update's dependency chain (5 to 7 us a
+// launch).  The link's words, the first Kennedy-Pendleton attempt's
+// logarithms and the overrelaxed link are therefore had while the staple's
+// links load, and one copy of the code serves all directions: a measured
+// sweep of one heat-bath and three overrelaxations 8^4 158 -> 151 us, 10^4
+// 197 -> 195.
 __global__ void __launch_bounds__(T)
 k_su2_heatbath_group(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles,
-               const __grid_constant__ ChainInfo one, double2 *__restrict__ links, int parity, int max_attempts, int kp,
+               const __grid_constant__ ChainInfo one, double2 *__restrict__ links, int parity, int mu, int max_attempts, int kp,
                const uint64_t *__restrict__ sweep_ptr, unsigned long long *__restrict__ proposals,
                unsigned *__restrict__ err) {
     const ItemChain block = block_of(chains, tiles, one, blockIdx.x / kGroup, T);
@@ -290,8 +312,16 @@ k_su2_heatbath_group(const ChainInfo *__restrict__ chains, const Tile *__restric
     const bool active = t < c.half;
     const int64_t s = (int64_t)parity * c.half + (active ? t : 0);
     const Coord x = decode_storage(c, s);
+    const uint64_t sweep = *sweep_ptr;
+    TermLinks l;
+    if (active && (threadIdx.x & (kGroup - 1)) < 6)
+        l = su2_term_links(links, c, site_of(c, x), parity, mu, threadIdx.x & (kGroup - 1));
+    // made while the links load
+    const uint64_t key = link_key(c.seed, sweep, x.lex, mu);
+    KpDraw first{0.0, 0.0};
+    if (kp) first = kp_draw(key, 0);
     double comp[4];
-    su2_staple_group<MU>(links, c, x, parity, active, comp);
+    su2_staple_group(l, active, comp);
     unsigned attempts_used = 0;
     if (active) {
         const double norm = staple_norm(comp);
@@ -299,10 +329,9 @@ k_su2_heatbath_group(const ChainInfo *__restrict__ chains, const Tile *__restric
         if (!isfinite(norm) || !isfinite(alpha)) {
             if (leader) atomicOr(err, kErrNonFinite);
         } else {
-            const uint64_t key = link_key(c.seed, *sweep_ptr, x.lex, MU);
             q4 r;
             int att = 0;
-            const bool ok = kp ? sample_kp(alpha, key, max_attempts, r, att)
+            const bool ok = kp ? sample_kp(alpha, key, first, max_attempts, r, att)
                                : sample_reference(alpha, key, max_attempts, r, att);
             attempts_used = leader ? (unsigned)att : 0u;
             if (!ok) {
@@ -314,7 +343,7 @@ k_su2_heatbath_group(const ChainInfo *__restrict__ chains, const Tile *__restric
                     normalize_scaled<4>(comp, vhat.c);
                     next = qmul(r, qdag(vhat));
                 }
-                if (leader) store_q(links, c, s, MU, next);
+                if (leader) store_q(links, c, s, mu, next);
             }
         }
     }
@@ -323,10 +352,9 @@ k_su2_heatbath_group(const ChainInfo *__restrict__ chains, const Tile *__restric
         atomicAdd(proposals + block.chain, (unsigned long long)warp_sum);
 }
 
-template <int MU>
 __global__ void __launch_bounds__(T)
 k_su2_overrelax_group(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles,
-                const __grid_constant__ ChainInfo one, double2 *__restrict__ links, int parity, unsigned *__restrict__ err) {
+                const __grid_constant__ ChainInfo one, double2 *__restrict__ links, int parity, int mu, unsigned *__restrict__ err) {
     const ItemChain block = block_of(chains, tiles, one, blockIdx.x / kGroup, T);
     const ChainInfo &c = block.c;
     const int64_t t = block.start + (int64_t)(blockIdx.x % kGroup) * kGroupLinks + threadIdx.x / kGroup;
@@ -334,8 +362,12 @@ k_su2_overrelax_group(const ChainInfo *__restrict__ chains, const Tile *__restri
     const bool active = t < c.half;
     const int64_t s = (int64_t)parity * c.half + (active ? t : 0);
     const Coord x = decode_storage(c, s);
+    TermLinks l;
+    if (active && (threadIdx.x & (kGroup - 1)) < 6)
+        l = su2_term_links(links, c, site_of(c, x), parity, mu, threadIdx.x & (kGroup - 1));
+    const q4 u = load_q_rw(links, c, s, mu);
     double comp[4];
-    su2_staple_group<MU>(links, c, x, parity, active, comp);
+    su2_staple_group(l, active, comp);
     if (!active) return;
     const double norm = staple_norm(comp);
     if (!isfinite(norm)) {
@@ -346,8 +378,8 @@ k_su2_overrelax_group(const ChainInfo *__restrict__ chains, const Tile *__restri
     q4 vhat;
     normalize_scaled<4>(comp, vhat.c);
     const q4 nd = qdag(vhat);
-    const q4 next = qmul(qmul(nd, qdag(load_q_rw(links, c, s, MU))), nd);
-    if (leader) store_q(links, c, s, MU, next);
+    const q4 next = qmul(qmul(nd, qdag(u)), nd);
+    if (leader) store_q(links, c, s, mu, next);
 }
 
 // Plaquette half real trace per site, (mu, nu) order as the reference.
@@ -542,12 +574,8 @@ cudaError_t launch_su2_heatbath(ym_ensemble *e, int parity, int mu, int max_atte
     const dim3 b(T);
     if (su2_grouped(e)) {
         const dim3 g((unsigned)(e->n_half_tiles * kGroup));
-        switch (mu) {
-        case 0: k_su2_heatbath_group<0><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, max_attempts, kp, sweep_index(e), e->d_accepts, e->d_error); break;
-        case 1: k_su2_heatbath_group<1><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, max_attempts, kp, sweep_index(e), e->d_accepts, e->d_error); break;
-        case 2: k_su2_heatbath_group<2><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, max_attempts, kp, sweep_index(e), e->d_accepts, e->d_error); break;
-        default: k_su2_heatbath_group<3><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, max_attempts, kp, sweep_index(e), e->d_accepts, e->d_error); break;
-        }
+        k_su2_heatbath_group<<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, mu, max_attempts, kp, sweep_index(e),
+                                                     e->d_accepts, e->d_error);
         return cudaGetLastError();
     }
     const dim3 g((unsigned)e->n_half_tiles);
@@ -567,12 +595,7 @@ cudaError_t launch_su2_overrelax(ym_ensemble *e, int parity, int mu) {
     const dim3 b(T);
     if (su2_grouped(e)) {
         const dim3 g((unsigned)(e->n_half_tiles * kGroup));
-        switch (mu) {
-        case 0: k_su2_overrelax_group<0><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, e->d_error); break;
-        case 1: k_su2_overrelax_group<1><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, e->d_error); break;
-        case 2: k_su2_overrelax_group<2><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, e->d_error); break;
-        default: k_su2_overrelax_group<3><<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, e->d_error); break;
-        }
+        k_su2_overrelax_group<<<g, b, 0, e->stream>>>(ch, tl, one, e->d_links, parity, mu, e->d_error);
         return cudaGetLastError();
     }
     const dim3 g((unsigned)e->n_half_tiles);
