@@ -31,12 +31,13 @@ def _compare(make, cadence, single, stride, n=2):
 
 @pytest.mark.parametrize("chains", [1, 3])
 @pytest.mark.parametrize("stride", [1, 31, 32, 33, 64])
-def test_su3_cadence(chains, stride):
+@pytest.mark.parametrize("path", ["tiled", "resident"])
+def test_su3_cadence(chains, stride, path):
     import ymgpu
 
     def make():
         ens = ymgpu.Ensemble([[4, 4, 4, 4]] * chains, 6.0, list(range(5, 5 + chains)))
-        ens.sweep_path = "tiled"
+        ens.sweep_path = path
         return ens
     _compare(make, lambda e, n, s: e.measured_sweeps(0.3, n, s, "ordered"),
              lambda e: e.metropolis_sweeps(0.3, 1, "ordered"), stride)

@@ -888,7 +888,6 @@ int32_t ym_su3_measured_sweeps(ym_ensemble *e, double angle, int32_t generator_m
     if (st) return st;
     if (n_measurements == 0) return YM_OK;
     YM_CUDA(ensure_series(e, n_measurements));
-    YM_CUDA(cudaMemsetAsync(e->d_series_row, 0, sizeof(uint64_t), e->stream));
     const bool fused = sweeps_per_measurement > 0 && fused_plaquette(e, generator_mode);
     auto step = [&]() -> cudaError_t {
         const ym::SweepSlotScope scope(e);
@@ -928,6 +927,7 @@ int32_t ym_su3_measured_sweeps(ym_ensemble *e, double angle, int32_t generator_m
             e->resident_choice = 1;
         if (e->resident_choice < 0 && n_measurements >= 2 && n_measurements * sweeps_per_measurement >= 2 * kTuneSweeps) {
             float t_tiled = 0.f, t_res = 0.f;
+            YM_CUDA(cudaMemsetAsync(e->d_series_row, 0, sizeof(uint64_t), e->stream));
             YM_CUDA(step_graph());
             YM_CUDA(time_on_stream(e, [&] { return cudaGraphLaunch(e->measure_graph, e->stream); }, &t_tiled));
             YM_CUDA(time_on_stream(e, [&] {
@@ -948,7 +948,10 @@ int32_t ym_su3_measured_sweeps(ym_ensemble *e, double angle, int32_t generator_m
             YM_CUDA(cudaStreamSynchronize(e->stream));
         }
     }
-    if (m < n_measurements) YM_CUDA(step_graph());
+    if (m < n_measurements) {
+        if (m == 0) YM_CUDA(cudaMemsetAsync(e->d_series_row, 0, sizeof(uint64_t), e->stream));
+        YM_CUDA(step_graph());
+    }
     for (; m < n_measurements; ++m) YM_CUDA(cudaGraphLaunch(e->measure_graph, e->stream));
     YM_CUDA(cudaMemcpyAsync(series, e->d_series, (size_t)(n_measurements * e->n_chains) * sizeof(double),
                             cudaMemcpyDeviceToHost, e->stream));

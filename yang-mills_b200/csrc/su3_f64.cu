@@ -102,24 +102,17 @@ struct RowEnd {
 // 4 x 16^4 421 -> 413 (its launches are not in a graph).
 __device__ __forceinline__ void end_row(const RowEnd &end, int chain, double value) {
     if (!end.series || threadIdx.x >= 32) return;
-    unsigned long long *ticket = reinterpret_cast<unsigned long long *>(end.sweep + kSweepSlots);
     uint64_t row = 0;
-    int last = 1;
+    int last = 0;
     if (threadIdx.x == 0) {
         row = *end.row;
         end.series[row * gridDim.x + chain] = value;
-        if (gridDim.x > 1) {
-            __threadfence();
-            last = atomicAdd(ticket, 1ull) == gridDim.x - 1;
-        }
+        last = last_block(end.sweep + kSweepSlots);
     }
     if (!__shfl_sync(0xffffffffu, last, 0)) return;
     static_assert(kSweepSlots == 32, "one entry per lane");
     end.sweep[threadIdx.x] += end.sweeps;
-    if (threadIdx.x == 0) {
-        *end.row = row + 1;
-        *ticket = 0;
-    }
+    if (threadIdx.x == 0) *end.row = row + 1;
 }
 
 static RowEnd row_end(ym_ensemble *e, double *series) {

@@ -131,7 +131,7 @@ enum ResidentForm {
 template <int K, bool DRAWN, int FORM>
 __global__ void __launch_bounds__(kResidentThreads, 1)
 k_su3_resident(const ChainInfo *__restrict__ chains, double2 *__restrict__ links, double angle,
-               const uint64_t *__restrict__ sweep_ptr, int64_t n_meas, int64_t sweeps_per_meas,
+               uint64_t *sweep_ptr, int64_t n_meas, int64_t sweeps_per_meas,
                double *__restrict__ series, int64_t n_chains, unsigned long long *__restrict__ accepts) {
     using namespace tiled_exact;
     extern __shared__ __align__(16) double2 sl[];
@@ -235,6 +235,11 @@ k_su3_resident(const ChainInfo *__restrict__ chains, double2 *__restrict__ links
     for (int i = threadIdx.x; i < n; i += kResidentThreads) links[c.offset + i] = sl[i];
     const unsigned sum = __reduce_add_sync(0xffffffffu, accepted);
     if ((threadIdx.x & 31) == 0 && sum) atomicAdd(accepts + chain, (unsigned long long)sum);
+    __syncthreads();   // every thread has read the sweep counter
+    if (threadIdx.x < 32) {
+        const int last = threadIdx.x == 0 ? last_block(sweep_ptr + kSweepSlots) : 0;
+        if (__shfl_sync(0xffffffffu, last, 0)) sweep_ptr[threadIdx.x] += (uint64_t)(n_meas * sweeps_per_meas);
+    }
 }
 
 // (kSweepSlots threads)
@@ -291,21 +296,17 @@ static cudaError_t resident_launch(ym_ensemble *e, double angle, int64_t n_meas,
     const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
     kernel<<<(unsigned)e->n_chains, kResidentThreads, smem, e->stream>>>(
-        e->d_chains, e->d_links, angle, sweep_index(e), n_meas, sweeps_per_meas, series, e->n_chains, e->d_accepts);
+        e->d_chains, e->d_links, angle, e->d_sweep, n_meas, sweeps_per_meas, series, e->n_chains, e->d_accepts);
     return cudaGetLastError();
 }
 
 cudaError_t launch_su3_resident(ym_ensemble *e, double angle, int uniform, int64_t n_meas,
                                 int64_t sweeps_per_meas, double *series) {
     const bool small = angle <= tiled_exact::kShortRotation;
-    const cudaError_t err =
-        uniform ? (small ? resident_launch<11, true>(e, angle, n_meas, sweeps_per_meas, series)
-                         : resident_launch<14, true>(e, angle, n_meas, sweeps_per_meas, series))
-                : (small ? resident_launch<11, false>(e, angle, n_meas, sweeps_per_meas, series)
-                         : resident_launch<14, false>(e, angle, n_meas, sweeps_per_meas, series));
-    if (err != cudaSuccess) return err;
-    k_advance_sweep<<<1, kSweepSlots, 0, e->stream>>>(e->d_sweep, (uint64_t)(n_meas * sweeps_per_meas));
-    return cudaGetLastError();
+    return uniform ? (small ? resident_launch<11, true>(e, angle, n_meas, sweeps_per_meas, series)
+                            : resident_launch<14, true>(e, angle, n_meas, sweeps_per_meas, series))
+                   : (small ? resident_launch<11, false>(e, angle, n_meas, sweeps_per_meas, series)
+                            : resident_launch<14, false>(e, angle, n_meas, sweeps_per_meas, series));
 }
 
 cudaError_t launch_counted_sweeps(ym_ensemble *e) {

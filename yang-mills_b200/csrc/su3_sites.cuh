@@ -15,6 +15,17 @@ __device__ __forceinline__ m3 link_at(const double2 *links, const ChainInfo &c, 
     return RESIDENT ? load_su3_rw(links, c, s, mu) : load_su3(links, c, s, mu);
 }
 
+// One thread of each block of a launch: whether its block is the last to come
+// here (no block waits).  What a block has read or written before is done
+// with; the ticket is zero again afterwards.
+__device__ __forceinline__ bool last_block(uint64_t *ticket) {
+    if (gridDim.x == 1) return true;
+    __threadfence();
+    if (atomicAdd(reinterpret_cast<unsigned long long *>(ticket), 1ull) != gridDim.x - 1) return false;
+    *ticket = 0;
+    return true;
+}
+
 // Thread's share of the sum of at(b) .. at(e - 1), entries threadIdx.x,
 // threadIdx.x + blockDim.x, ... of the range in a fixed order.  The chain of
 // dependent loads bounds these sums (a few blocks, no more work per SM than
