@@ -108,39 +108,37 @@ __device__ __forceinline__ void wilson_site(const double2 *links, const ChainInf
                                             int rmax, int tmax, double2 *qs, double (*vs)[T]) {
     {   // D_T, stored as Q_{0,T}
         Walker w = w0;
-        m3 d;
+        m3 d, next = link_of(links, c, w, NU);
 #pragma unroll 1
         for (int t = 0; t < tmax; ++t) {
-            {
-                const m3 u = link_of(links, c, w, NU);
-                d = t == 0 ? u : mul_fma(d, u);
-                q_put(qs, t, d);
-                step_walker(c, w, NU);
-            }
+            const m3 u = next;
+            step_walker(c, w, NU);
+            if (t + 1 < tmax) next = link_of(links, c, w, NU);
+            d = t == 0 ? u : mul_fma(d, u);
+            q_put(qs, t, d);
         }
     }
     Walker wa = w0;   // x + (R-1) mu
     m3 a;
 #pragma unroll 1
     for (int r = 0; r < rmax; ++r) {
-        {
-            const m3 ua = link_of(links, c, wa, MU);
-            a = r == 0 ? ua : mul_fma(a, ua);
-            Walker wq = wa;          // x + (R-1) mu, walked along nu with T
-            step_walker(c, wa, MU);  // x + R mu
-            Walker wp = wa;
-            m3 p = a;
+        const m3 ua = link_of(links, c, wa, MU);
+        Walker wq = wa;          // x + (R-1) mu, walked along nu with T
+        step_walker(c, wa, MU);  // x + R mu
+        Walker wp = wa;
+        m3 up = link_of(links, c, wp, NU);
+        a = r == 0 ? ua : mul_fma(a, ua);
+        m3 p = a;
 #pragma unroll 1
-            for (int t = 0; t < tmax; ++t) {
-                {
-                    p = mul_fma(p, link_of(links, c, wp, NU));
-                    step_walker(c, wp, NU);
-                    step_walker(c, wq, NU);
-                    const m3 q = mul_fma(q_get(qs, t), link_of(links, c, wq, MU));
-                    q_put(qs, t, q);
-                    vs[r * kMaxRT + t][threadIdx.x] = retrace_mul_adj(p, q) * (1.0 / 3.0);
-                }
-            }
+        for (int t = 0; t < tmax; ++t) {
+            step_walker(c, wq, NU);
+            const m3 uq = link_of(links, c, wq, MU);
+            p = mul_fma(p, up);
+            step_walker(c, wp, NU);
+            if (t + 1 < tmax) up = link_of(links, c, wp, NU);
+            const m3 q = mul_fma(q_get(qs, t), uq);
+            q_put(qs, t, q);
+            vs[r * kMaxRT + t][threadIdx.x] = retrace_mul_adj(p, q) * (1.0 / 3.0);
         }
     }
 }
