@@ -43,24 +43,6 @@ __device__ __forceinline__ Walker walker_of(const Coord &x) {
     return w;
 }
 
-// Block sum of 16 values per thread into out[16] (thread 0 writes).
-__device__ __forceinline__ void block_sum16(double v[16], double *out) {
-    __shared__ double red[16][T / 32];
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-        double a = v[k];
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) a += __shfl_down_sync(0xffffffffu, a, off);
-        if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = a;
-    }
-    __syncthreads();
-    if (threadIdx.x < 16) {
-        double a = red[threadIdx.x][0];
-        for (int w = 1; w < T / 32; ++w) a += red[threadIdx.x][w];
-        out[threadIdx.x] = a;
-    }
-}
-
 // Wilson loops: grid (site tiles, 6 planes).  Each thread: one site x, one
 // plane (mu < nu), R along mu, T along nu, every (R, T) <= (rmax, tmax).
 // The rectangle's holonomy (R forward mu, T forward nu, R back, T back) is
@@ -70,8 +52,12 @@ __device__ __forceinline__ void block_sum16(double v[16], double *out) {
 // each multiplied left to right in traversal order (fma chains); P grows in T from the
 // mu-line A_R, Q grows in R (Q_{0,T} = the nu-line D_T), so all sixteen loops
 // take 38 products instead of 160.  The four Q_{R-1,T} wait in shared memory
-// between R steps, and the sixteen loop values are written straight to the
-// thread's shared-memory column (fewer registers than an indexed array).  Re (1/3) Tr(P Q^dag) differs from the single-chain
+// between R steps; each loop value is summed over its warp as it is made, so
+// that nothing else takes shared memory from L1.  What bounds it: the links
+// come from L2 (13 TB/s at 24^3 x 48) under the chain of products; the next
+// nu link is loaded a step ahead.  24^3 x 48: values in a shared-memory column
+// and no load ahead 2.31 ms, load ahead 2.26, warp sums 2.22; 16^4 0.247 to
+// 0.235.  Re (1/3) Tr(P Q^dag) differs from the single-chain
 // product only by rounding (<= 1e-12 relative on lattice means).
 // partial[(tile * 6 + plane) * 16 + (R-1)*4 + (T-1)] = tile sum.
 constexpr size_t kWilsonSmem = (size_t)kMaxRT * 9 * T * sizeof(double2);
@@ -105,7 +91,7 @@ __device__ __forceinline__ m3 q_get(const double2 *qs, int t) {
 
 template <int MU, int NU>
 __device__ __forceinline__ void wilson_site(const double2 *links, const ChainInfo &c, const Walker &w0,
-                                            int rmax, int tmax, double2 *qs, double (*vs)[T]) {
+                                            int rmax, int tmax, double2 *qs, double (*sums)[16], bool live) {
     {   // D_T, stored as Q_{0,T}
         Walker w = w0;
         m3 d, next = link_of(links, c, w, NU);
@@ -138,37 +124,42 @@ __device__ __forceinline__ void wilson_site(const double2 *links, const ChainInf
             if (t + 1 < tmax) up = link_of(links, c, wp, NU);
             const m3 q = mul_fma(q_get(qs, t), uq);
             q_put(qs, t, q);
-            vs[r * kMaxRT + t][threadIdx.x] = retrace_mul_adj(p, q) * (1.0 / 3.0);
+            double v = retrace_mul_adj(p, q) * (1.0 / 3.0);
+            if (!live) v = 0.0;
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+            if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5][r * kMaxRT + t] = v;
         }
     }
 }
 
-__global__ void __launch_bounds__(T)
+__global__ void __launch_bounds__(T, 2)
 k_wilson_loops(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles,
                const double2 *__restrict__ links, int rmax, int tmax, double *__restrict__ partial) {
     extern __shared__ __align__(16) double2 qs[];
-    __shared__ double vs[16][T];
+    __shared__ double sums[T / 32][16];
     const int plane = blockIdx.y;
     const Tile tile = tiles[blockIdx.x];
     const ChainInfo c = chains[tile.chain];
     const int64_t s = tile.start + threadIdx.x;
-#pragma unroll
-    for (int k = 0; k < 16; ++k) vs[k][threadIdx.x] = 0.0;
-    if (s < c.volume) {
-        const Walker w0 = walker_of(decode_storage(c, s));
-        switch (plane) {
-            case 0: wilson_site<0, 1>(links, c, w0, rmax, tmax, qs, vs); break;
-            case 1: wilson_site<0, 2>(links, c, w0, rmax, tmax, qs, vs); break;
-            case 2: wilson_site<0, 3>(links, c, w0, rmax, tmax, qs, vs); break;
-            case 3: wilson_site<1, 2>(links, c, w0, rmax, tmax, qs, vs); break;
-            case 4: wilson_site<1, 3>(links, c, w0, rmax, tmax, qs, vs); break;
-            default: wilson_site<2, 3>(links, c, w0, rmax, tmax, qs, vs); break;
-        }
+    if (threadIdx.x < T / 32 * 16) sums[threadIdx.x / 16][threadIdx.x % 16] = 0.0;
+    __syncthreads();
+    const bool live = s < c.volume;
+    const Walker w0 = walker_of(decode_storage(c, live ? s : 0));
+    switch (plane) {
+        case 0: wilson_site<0, 1>(links, c, w0, rmax, tmax, qs, sums, live); break;
+        case 1: wilson_site<0, 2>(links, c, w0, rmax, tmax, qs, sums, live); break;
+        case 2: wilson_site<0, 3>(links, c, w0, rmax, tmax, qs, sums, live); break;
+        case 3: wilson_site<1, 2>(links, c, w0, rmax, tmax, qs, sums, live); break;
+        case 4: wilson_site<1, 3>(links, c, w0, rmax, tmax, qs, sums, live); break;
+        default: wilson_site<2, 3>(links, c, w0, rmax, tmax, qs, sums, live); break;
     }
-    double v[16];
-#pragma unroll
-    for (int k = 0; k < 16; ++k) v[k] = vs[k][threadIdx.x];
-    block_sum16(v, partial + ((int64_t)blockIdx.x * 6 + plane) * 16);
+    __syncthreads();
+    if (threadIdx.x < 16) {
+        double a = sums[0][threadIdx.x];
+        for (int w = 1; w < T / 32; ++w) a += sums[w][threadIdx.x];
+        partial[((int64_t)blockIdx.x * 6 + plane) * 16 + threadIdx.x] = a;
+    }
 }
 
 // One block per (chain, value k): the chain's tile partials
