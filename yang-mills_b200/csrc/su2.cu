@@ -365,7 +365,10 @@ k_su2_overrelax_group(const ChainInfo *__restrict__ chains, const Tile *__restri
     TermLinks l;
     if (active && (threadIdx.x & (kGroup - 1)) < 6)
         l = su2_term_links(links, c, site_of(c, x), parity, mu, threadIdx.x & (kGroup - 1));
-    const q4 u = load_q_rw(links, c, s, mu);
+    // (an idle group has no link of its own: its slot is another group's,
+    // which may be storing to it)
+    q4 u{{0.0, 0.0, 0.0, 0.0}};
+    if (active) u = load_q_rw(links, c, s, mu);
     double comp[4];
     su2_staple_group(l, active, comp);
     if (!active) return;
