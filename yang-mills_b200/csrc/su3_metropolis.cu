@@ -278,6 +278,30 @@ bool resident_fits(const ym_ensemble *e) {
     return resident_smem_bytes(e) + kResidentFixed <= (size_t)optin_smem();
 }
 
+// The dynamic shared memory limit of the three forms, set once per device to
+// all a block may have.  It belongs to the kernel, not to the handle: set to
+// each launch's own size, another thread's launch of a smaller handle could
+// lower it between this thread's setting and its launch, which then fails.
+template <int K, bool DRAWN>
+static cudaError_t configure_resident() {
+    static thread_local int configured_device = -1;
+    int dev = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess || configured_device == dev) return err;
+    const void *forms[3] = {(const void *)k_su3_resident<K, DRAWN, kLocal>,
+                            (const void *)k_su3_resident<K, DRAWN, kShared>,
+                            (const void *)k_su3_resident<K, DRAWN, kTable>};
+    for (const void *f : forms) {
+        cudaFuncAttributes at;
+        if ((err = cudaFuncGetAttributes(&at, f)) != cudaSuccess) return err;
+        err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   optin_smem() - (int)at.sharedSizeBytes);
+        if (err != cudaSuccess) return err;
+    }
+    configured_device = dev;
+    return cudaSuccess;
+}
+
 template <int K, bool DRAWN>
 static cudaError_t resident_launch(ym_ensemble *e, double angle, int64_t n_meas, int64_t sweeps_per_meas,
                                    double *series) {
@@ -293,8 +317,7 @@ static cudaError_t resident_launch(ym_ensemble *e, double angle, int64_t n_meas,
         kernel = k_su3_resident<K, DRAWN, kShared>;
         smem = links + kResidentAccumulator;
     }
-    const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) return err;
+    if (const cudaError_t err = configure_resident<K, DRAWN>()) return err;
     kernel<<<(unsigned)e->n_chains, kResidentThreads, smem, e->stream>>>(
         e->d_chains, e->d_links, angle, e->d_sweep, n_meas, sweeps_per_meas, series, e->n_chains, e->d_accepts);
     return cudaGetLastError();
