@@ -444,6 +444,7 @@ int32_t ym_ensemble_create(const ym_ensemble_desc *desc, ym_ensemble **out) {
         e->chain_links.push_back(links);
         e->total_links += links;
         if (links > e->max_chain_links) e->max_chain_links = links;
+        if (sites / n[3] > e->max_slice_sites) e->max_slice_sites = sites / n[3];
     }
     // total_elems counts 16-byte units of link storage
     e->total_elems = e->precision == YM_PREC_F32_TWO_ROW ? (offset + 1) / 2 : offset;

@@ -173,7 +173,7 @@ __global__ void k_tile_mean(const double *__restrict__ partial, const int32_t *_
                             double *__restrict__ out) {
     const int chain = blockIdx.x, k = blockIdx.y;
     const int b = first[chain], e = first[chain + 1];
-    double v = strided_sum(b, e, [&](int i) { return partial[(int64_t)i * width + k]; });
+    double v = strided_sum(b, e, blockDim.x, [&](int i) { return partial[(int64_t)i * width + k]; });
     v = block_reduce<false>(v);
     if (threadIdx.x == 0) {
         const ChainInfo &c = chains[chain];
@@ -332,12 +332,13 @@ __global__ void k_operator_reduce(const ChainInfo *__restrict__ chains, const in
     const uint32_t vs = (uint32_t)c.n[0] * n1 * n2;
     const double2 *vals = site_vals + c.offset / 36;
     double p = 0.0, r = 0.0;
+    const uint32_t width = reduce_width(vs);
     // four sites in flight
-    for (uint32_t i0 = threadIdx.x; i0 < vs; i0 += 4 * blockDim.x) {
+    for (uint32_t i0 = threadIdx.x < width ? threadIdx.x : vs; i0 < vs; i0 += 4 * width) {
         double2 v[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const uint32_t i = i0 + j * blockDim.x;
+            const uint32_t i = i0 + j * width;
             const uint32_t row = i / n2, x0 = row / n1;
             const int par = ((i - row * n2) + (row - x0 * n1) + x0 + t) & 1;
             v[j] = make_double2(0.0, 0.0);
@@ -406,10 +407,7 @@ cudaError_t launch_operator_basis(ym_ensemble *e, double2 *d_site_vals, const in
                                   double *d_rect, const double2 *links) {
     k_operator_sites<<<(unsigned)e->n_site_tiles, T, 0, e->stream>>>(e->d_chains, e->d_site_tiles,
                                                                     links ? links : e->d_links, d_site_vals);
-    // a round of a block takes four sites per thread; slices of more than
-    // 1024 sites get blocks of 1024 threads
-    const int threads = (int64_t)e->n_site_tiles * T > 1024 * n_slices ? 1024 : 256;
-    k_operator_reduce<<<(unsigned)n_slices, threads, 0, e->stream>>>(e->d_chains, d_slice_chain, d_slice_t,
+    k_operator_reduce<<<(unsigned)n_slices, reduce_width(e->max_slice_sites), 0, e->stream>>>(e->d_chains, d_slice_chain, d_slice_t,
                                                                 d_site_vals, d_plaq, d_rect);
     return cudaGetLastError();
 }

@@ -130,7 +130,7 @@ __global__ void k_chain_reduce_sweep(const double *__restrict__ tr_partial, int6
                                      double *__restrict__ out, RowEnd end) {
     const int chain = blockIdx.x;
     const int b = cta_range[2 * chain] * kSweepWarps, e = cta_range[2 * chain + 1] * kSweepWarps;
-    double v = strided_sum(b, e, [&](int i) {
+    double v = strided_sum(b, e, blockDim.x, [&](int i) {
         return (tr_partial[i] + tr_partial[warps + i]) + tr_partial[2 * warps + i];
     });
     v = block_reduce<false>(v);
@@ -168,7 +168,7 @@ __global__ void k_chain_reduce(const double *__restrict__ partial, const int32_t
         for (int i = b + threadIdx.x; i < e; i += blockDim.x)
             v = (i == b + (int)threadIdx.x) ? partial[i] : fmax(v, partial[i]);
     } else {
-        v = strided_sum(b, e, [&](int i) { return partial[i]; });
+        v = strided_sum(b, e, reduce_width(e - b), [&](int i) { return partial[i]; });
     }
     v = mode ? block_reduce<true>(v) : block_reduce<false>(v);
     if (!mode) v /= per_site * (double)chains[chain].volume;
@@ -446,9 +446,8 @@ cudaError_t launch_store_rows(cudaStream_t st, const double *src, int64_t n, dou
     return cudaGetLastError();
 }
 
-// Threads of a k_chain_reduce block: 256 take 1024 tiles in one round of
-// strided_sum; chains of more tiles get 1024 (5184 tiles: 14 -> 5 us).
-static int reduce_threads(const ym_ensemble *e) { return (int64_t)e->n_site_tiles > 1024 * (int64_t)e->n_chains ? 1024 : 256; }
+// Threads of a k_chain_reduce block: the widest chain's.
+static int reduce_threads(const ym_ensemble *e) { return reduce_width((e->max_chain_links / 4 + kSiteThreads - 1) / kSiteThreads); }
 
 cudaError_t launch_chain_reduce(ym_ensemble *e, const double *partial, double *out, int mode,
                                 double per_site, double *series) {

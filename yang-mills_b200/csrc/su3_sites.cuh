@@ -26,21 +26,29 @@ __device__ __forceinline__ bool last_block(uint64_t *ticket) {
     return true;
 }
 
+// The width, in threads, of a reduction over n entries: 256 take 1024 entries
+// in one round of strided_sum, more entries get 1024 (5184 tiles: 14 -> 5 us).
+// It is each chain's (or slice's) own, whatever the block's size, so that the
+// order of a sum, and its bits, do not depend on what else the handle holds.
+__host__ __device__ constexpr int reduce_width(int64_t n) { return n > 1024 ? 1024 : 256; }
+
 // Thread's share of the sum of at(b) .. at(e - 1), entries threadIdx.x,
-// threadIdx.x + blockDim.x, ... of the range in a fixed order.  The chain of
+// threadIdx.x + width, ... of the range in a fixed order (threads from width
+// on have none).  The chain of
 // dependent loads bounds these sums (a few blocks, no more work per SM than
 // that), so four entries are in flight: 5184 tiles 14 -> 5 us (1024 threads,
 // 256 before), 32^4's 12288 shares of three planes 14 -> 12, the operators of
 // 2560 slices of 64 to 512 sites 19 -> 13.
 template <class At>
-__device__ __forceinline__ double strided_sum(int b, int e, At at) {
+__device__ __forceinline__ double strided_sum(int b, int e, int width, At at) {
     double a[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int i = b + threadIdx.x; i < e; i += 4 * blockDim.x)
+    if ((int)threadIdx.x < width)
+        for (int i = b + threadIdx.x; i < e; i += 4 * width)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int k = i + j * blockDim.x;
-            if (k < e) a[j] += at(k);
-        }
+            for (int j = 0; j < 4; ++j) {
+                const int k = i + j * width;
+                if (k < e) a[j] += at(k);
+            }
     return (a[0] + a[1]) + (a[2] + a[3]);
 }
 

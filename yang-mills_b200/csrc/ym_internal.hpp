@@ -53,6 +53,7 @@ struct ym_ensemble {
     std::vector<int64_t> chain_links;      // links per chain
     int64_t total_links = 0;
     int64_t max_chain_links = 0;
+    int64_t max_slice_sites = 0;           // of one time slice
     int64_t total_elems = 0;               // double2 elements of link storage
 
     ym::ChainInfo *d_chains = nullptr;
