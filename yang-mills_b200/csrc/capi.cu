@@ -891,7 +891,7 @@ int32_t ym_su3_measured_sweeps(ym_ensemble *e, double angle, int32_t generator_m
     YM_CUDA(ensure_series(e, n_measurements));
     const bool fused = sweeps_per_measurement > 0 && fused_plaquette(e, generator_mode);
     auto step = [&]() -> cudaError_t {
-        const ym::SweepSlotScope scope(e);
+        const ym::CapturedSweeps scope(e);
         for (int64_t k = 0; k < sweeps_per_measurement; ++k) {
             cudaError_t err = cadence_sweep(e, angle, generator_mode, fused && k == sweeps_per_measurement - 1);
             if (err != cudaSuccess) return err;
@@ -1022,7 +1022,7 @@ int32_t ym_su3_measured_run(ym_ensemble *e, ym_ensemble *view, const ym_measured
     const double angle = run->proposal_angle;
     const bool fused = fused_plaquette(e, mode);
     auto block = [&]() -> cudaError_t {
-        const ym::SweepSlotScope scope(e);
+        const ym::CapturedSweeps scope(e);
         for (int64_t k = 0; k < spb; ++k) {
             cudaError_t err = cadence_sweep(e, angle, mode, fused);
             if (err == cudaSuccess) err = cadence_plaquette(e, fused);
@@ -1761,7 +1761,7 @@ int32_t ym_su2_measured_sweeps(ym_ensemble *e, int64_t max_attempts_per_link, in
     // one measurement: the sweeps of ym_su2_markov_sweeps, then the average
     // plaquette of every chain into the next row of the device series
     auto step = [&]() -> cudaError_t {
-        const ym::SweepSlotScope scope(e);
+        const ym::CapturedSweeps scope(e);
         cudaError_t err = cudaSuccess;
         for (int64_t k = 0; k < sweeps_per_measurement && err == cudaSuccess; ++k) {
             for (int parity = 0; parity < 2 && err == cudaSuccess; ++parity)

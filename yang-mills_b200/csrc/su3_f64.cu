@@ -116,9 +116,14 @@ __device__ __forceinline__ void end_row(const RowEnd &end, int chain, double val
 }
 
 static RowEnd row_end(ym_ensemble *e, double *series) {
-    const RowEnd end{series, e->d_series_row, e->d_sweep, (uint64_t)e->sweep_slot};
-    if (series) e->sweep_slot = 0;
-    return end;
+    return RowEnd{series, e->d_series_row, e->d_sweep, (uint64_t)e->sweep_slot};
+}
+
+// The launch that ends the row has been made: it counts the deferred sweeps.
+static cudaError_t row_ended(ym_ensemble *e, double *series) {
+    const cudaError_t err = cudaGetLastError();
+    if (series && err == cudaSuccess) e->sweep_slot = 0;
+    return err;
 }
 
 // One 1024-thread block per chain: the plaquette shares the last three
@@ -453,7 +458,7 @@ cudaError_t launch_chain_reduce(ym_ensemble *e, const double *partial, double *o
                                 double per_site, double *series) {
     k_chain_reduce<<<(unsigned)e->n_chains, reduce_threads(e), 0, e->stream>>>(
         partial, e->d_site_tile_first, e->d_chains, out, mode, per_site, row_end(e, series));
-    return cudaGetLastError();
+    return row_ended(e, series);
 }
 
 cudaError_t launch_su3_plaquette(ym_ensemble *e, double *series) {
@@ -470,7 +475,7 @@ cudaError_t launch_su3_plaquette(ym_ensemble *e, double *series) {
         e->d_chains, e->d_site_tiles, e->d_links, e->d_partial);
     k_chain_reduce<<<(unsigned)e->n_chains, reduce_threads(e), 0, e->stream>>>(
         e->d_partial, e->d_site_tile_first, e->d_chains, e->d_result, 0, 6.0, row_end(e, series));
-    return cudaGetLastError();
+    return row_ended(e, series);
 }
 
 cudaError_t launch_su3_plaquette_from_sweep(ym_ensemble *e, const double *tr_partial, double *series) {
@@ -478,7 +483,7 @@ cudaError_t launch_su3_plaquette_from_sweep(ym_ensemble *e, const double *tr_par
     if (!L.d_chain_ctas) return cudaErrorInvalidValue;
     k_chain_reduce_sweep<<<(unsigned)e->n_chains, 1024, 0, e->stream>>>(tr_partial, L.ctas * kSweepWarps, L.d_chain_ctas,
                                                                          e->d_chains, e->d_result, row_end(e, series));
-    return cudaGetLastError();
+    return row_ended(e, series);
 }
 
 cudaError_t launch_su3_residuals(ym_ensemble *e) {

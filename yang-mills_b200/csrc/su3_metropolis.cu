@@ -335,13 +335,16 @@ cudaError_t launch_su3_resident(ym_ensemble *e, double angle, int uniform, int64
 cudaError_t launch_counted_sweeps(ym_ensemble *e) {
     if (e->sweep_slot == 0) return cudaSuccess;
     k_advance_sweep<<<1, kSweepSlots, 0, e->stream>>>(e->d_sweep, (uint64_t)e->sweep_slot);
-    e->sweep_slot = 0;
-    return cudaGetLastError();
+    const cudaError_t err = cudaGetLastError();
+    if (err == cudaSuccess) e->sweep_slot = 0;
+    return err;
 }
 
 cudaError_t launch_advance_sweep(ym_ensemble *e) {
     ++e->sweep_slot;
-    return launch_counted_sweeps(e);
+    const cudaError_t err = launch_counted_sweeps(e);
+    if (err != cudaSuccess) --e->sweep_slot;
+    return err;
 }
 
 }  // namespace ym

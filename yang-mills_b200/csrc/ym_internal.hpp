@@ -241,11 +241,22 @@ inline cudaError_t count_sweep(ym_ensemble *e) {
     ++e->sweep_slot;
     return cudaSuccess;
 }
-// Sweeps that an abandoned cadence deferred are not carried into the next.
+// Around sweeps that are launched as they are counted: when a later launch
+// fails, those already launched still go onto the device's counter, so that
+// the next call does not draw their stream words again.
 struct SweepSlotScope {
     ym_ensemble *e;
     explicit SweepSlotScope(ym_ensemble *e_) : e(e_) { e->sweep_slot = 0; }
-    ~SweepSlotScope() { e->sweep_slot = 0; }
+    ~SweepSlotScope() {
+        launch_counted_sweeps(e);
+        e->sweep_slot = 0;
+    }
+};
+// Around a captured cadence: the sweeps of a capture that failed never ran.
+struct CapturedSweeps {
+    ym_ensemble *e;
+    explicit CapturedSweeps(ym_ensemble *e_) : e(e_) { e->sweep_slot = 0; }
+    ~CapturedSweeps() { e->sweep_slot = 0; }
 };
 // Chain-resident sweeps (su3_metropolis.cu): every chain small enough that
 // its links fit in one CTA's shared memory.  series (device, may be null)
