@@ -636,7 +636,17 @@ __global__ void k_lp_adam(const double *__restrict__ groups, int64_t n_groups, i
 // blockIdx.x + gridDim.x, ...  Every tile's three MMA groups are waited for
 // before its hits, so the shared-memory operand tiles and the accumulator
 // columns are free again when the next tile writes them.
-template <int MU>
+//
+// REG: the hits in registers, not on rows in memory.  With at most two tiles
+// per SM a sub-sweep is one or two visits' latency, and the hits' row reads
+// and lambda8's branch lie on it; with more, issue bounds it and the memory
+// form has fewer instructions.  Per sweep, registers against memory: 8^4 155
+// against 162 us, 12^4 157 against 171, 151 tiles 172.7 against 173.2, 256
+// tiles (16^4) 176 against 188, 288 tiles 185 against 189; 411 tiles (18^4)
+// 223 against 206, 4 x 16^4 430 against 413.
+constexpr int kRegTilesPerSm = 2;
+
+template <int MU, bool REG>
 __global__ void __launch_bounds__(kRows, 4)
 k_lp_sweep(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles, int64_t n_tiles,
            float2 *__restrict__ links, int parity, const uint4 *__restrict__ image,
@@ -680,17 +690,21 @@ k_lp_sweep(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles,
             proposal_from(y, draw.cum, scale);
             m3f u = load_f(links, c, s, MU);
             const uint64_t key = link_key(c.seed, sweep, x.lex, MU);
-            // the staple and the rows in the activation tiles' memory, free
-            // since the last MMA group was waited for
-            float2 (*own)[kRows] = reinterpret_cast<float2 (*)[kRows]>(sm + L::H1);
-            const StapleColF<kRows> sa{own};
-            const RowCol<kRows> rows{own + 9};
-            put_staple(sa, a);
+            if (REG) {
+                accepted = visit_learned_reg(u, a, c.beta / 3.0, draw, scale, key);
+            } else {
+                // the staple and the rows in the activation tiles' memory, free
+                // since the last MMA group was waited for
+                float2 (*own)[kRows] = reinterpret_cast<float2 (*)[kRows]>(sm + L::H1);
+                const StapleColF<kRows> sa{own};
+                const RowCol<kRows> rows{own + 9};
+                put_staple(sa, a);
 #pragma unroll
-            for (int i = 0; i < 3; ++i) rows.put_row(i, u.e[i]);
-            accepted = visit_drawn_f(rows, sa, c.beta / 3.0, (double)scale, key, draw);
+                for (int i = 0; i < 3; ++i) rows.put_row(i, u.e[i]);
+                accepted = visit_drawn_f(rows, sa, c.beta / 3.0, (double)scale, key, draw);
 #pragma unroll
-            for (int i = 0; i < 2; ++i) rows.row(i, u.e[i]);
+                for (int i = 0; i < 2; ++i) rows.row(i, u.e[i]);
+            }
             store_f(links, c, s, MU, u);
         }
         const unsigned warp_sum = __reduce_add_sync(0xffffffffu, accepted);
@@ -787,38 +801,45 @@ cudaError_t launch_lp_adam(ym_proposal_model *m, int64_t n_tiles, int64_t n_vali
     return cudaGetLastError();
 }
 
+template <int MU>
+static cudaError_t allow_lp_sweep() {
+    const cudaError_t err = lp::allow_smem(lp::k_lp_sweep<MU, false>, lp::FwdLayout::BYTES);
+    return err == cudaSuccess ? lp::allow_smem(lp::k_lp_sweep<MU, true>, lp::FwdLayout::BYTES) : err;
+}
+
+template <int MU>
+static cudaError_t lp_sweep_launch(ym_ensemble *e, ym_proposal_model *m, int parity, int sms) {
+    const int64_t n = e->n_half_tiles;
+    // four CTAs per SM: registers, shared memory and 4 x 64 TMEM columns
+    const unsigned grid = (unsigned)(n < 4 * sms ? n : 4 * sms);
+    const auto kernel = n <= lp::kRegTilesPerSm * sms ? lp::k_lp_sweep<MU, true> : lp::k_lp_sweep<MU, false>;
+    kernel<<<grid, lp::kRows, lp::FwdLayout::BYTES, e->stream>>>(
+        e->d_chains, e->d_half_tiles, n, reinterpret_cast<float2 *>(e->d_links), parity,
+        reinterpret_cast<const uint4 *>(m->d_image), m->d_params, sweep_index(e), e->d_accepts, m->d_error);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_lp_sweep(ym_ensemble *e, ym_proposal_model *m, int parity, int mu) {
-    static thread_local int configured_device = -1;
+    static thread_local int configured_device = -1, sms = 148;
     int dev = 0;
     cudaGetDevice(&dev);
     if (configured_device != dev) {
-        cudaError_t err = lp::allow_smem(lp::k_lp_sweep<0>, lp::FwdLayout::BYTES);
-        if (err == cudaSuccess) err = lp::allow_smem(lp::k_lp_sweep<1>, lp::FwdLayout::BYTES);
-        if (err == cudaSuccess) err = lp::allow_smem(lp::k_lp_sweep<2>, lp::FwdLayout::BYTES);
-        if (err == cudaSuccess) err = lp::allow_smem(lp::k_lp_sweep<3>, lp::FwdLayout::BYTES);
+        cudaError_t err = allow_lp_sweep<0>();
+        if (err == cudaSuccess) err = allow_lp_sweep<1>();
+        if (err == cudaSuccess) err = allow_lp_sweep<2>();
+        if (err == cudaSuccess) err = allow_lp_sweep<3>();
         if (err != cudaSuccess) return err;
+        sms = 148;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         configured_device = dev;
     }
     if (e->n_half_tiles == 0) return cudaSuccess;
-    static thread_local int resident_ctas = 0, resident_device = -1;
-    if (resident_device != dev) {   // 4 CTAs per SM: registers, shared memory and 4 x 64 TMEM columns
-        int sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        resident_ctas = 4 * sms;
-        resident_device = dev;
-    }
-    const int64_t n = e->n_half_tiles;
-    const dim3 grid((unsigned)(n < resident_ctas ? n : resident_ctas));
-    float2 *links = reinterpret_cast<float2 *>(e->d_links);
-    const uint4 *img = reinterpret_cast<const uint4 *>(m->d_image);
-    const uint32_t sm = lp::FwdLayout::BYTES;
     switch (mu) {
-        case 0: lp::k_lp_sweep<0><<<grid, lp::kRows, sm, e->stream>>>(e->d_chains, e->d_half_tiles, n, links, parity, img, m->d_params, sweep_index(e), e->d_accepts, m->d_error); break;
-        case 1: lp::k_lp_sweep<1><<<grid, lp::kRows, sm, e->stream>>>(e->d_chains, e->d_half_tiles, n, links, parity, img, m->d_params, sweep_index(e), e->d_accepts, m->d_error); break;
-        case 2: lp::k_lp_sweep<2><<<grid, lp::kRows, sm, e->stream>>>(e->d_chains, e->d_half_tiles, n, links, parity, img, m->d_params, sweep_index(e), e->d_accepts, m->d_error); break;
-        default: lp::k_lp_sweep<3><<<grid, lp::kRows, sm, e->stream>>>(e->d_chains, e->d_half_tiles, n, links, parity, img, m->d_params, sweep_index(e), e->d_accepts, m->d_error); break;
+        case 0: return lp_sweep_launch<0>(e, m, parity, sms);
+        case 1: return lp_sweep_launch<1>(e, m, parity, sms);
+        case 2: return lp_sweep_launch<2>(e, m, parity, sms);
+        default: return lp_sweep_launch<3>(e, m, parity, sms);
     }
-    return cudaGetLastError();
 }
 
 }  // namespace ym

@@ -607,6 +607,116 @@ struct DrawLearned {
     }
 };
 
+// ---- learned hits of small handles ------------------------------------------
+// The link and the staple in registers, one hit after the other: fewer waits
+// between a hit's generator and its decision than visit_drawn_f's rows in
+// memory, at more instructions (k_lp_sweep's rule).
+__device__ __forceinline__ bool accept64(double old_tr, double new_tr, double beta3, double unif) {
+    const double m = fmax(beta3 * (old_tr - new_tr), 0.0);
+    return (m == 0.0) ? true : (unif < exp(-m));
+}
+
+// Re of a row of X times a column of A, in binary64 (the retr_row64 chain
+// with the column passed by value, for rows chosen at run time).
+__device__ __forceinline__ double retr_col64(const cf *x, cf c0, cf c1, cf c2) {
+    double acc = (double)x[0].re * (double)c0.re;
+    acc = fma(-(double)x[0].im, (double)c0.im, acc);
+    acc = fma((double)x[1].re, (double)c1.re, acc);
+    acc = fma(-(double)x[1].im, (double)c1.im, acc);
+    acc = fma((double)x[2].re, (double)c2.re, acc);
+    acc = fma(-(double)x[2].im, (double)c2.im, acc);
+    return acc;
+}
+
+__device__ __forceinline__ cf csel(bool p, cf a, cf b) { return cf{p ? a.re : b.re, p ? a.im : b.im}; }
+
+// One hit of a generator chosen per thread, without divergent control
+// flow.  exp(i theta T^g) acts on rows (i, j) as the 2x2 matrix
+// [[r00, r01], [r10, r11]] and multiplies the remaining row k by ek:
+//   sigma_1 type (g = 0, 3, 5): [[c, i s], [i s, c]]
+//   sigma_2 type (g = 1, 4, 6): [[c, s], [-s, c]]
+//   sigma_3      (g = 2):       diag(c + i s, c - i s)
+//   lambda_8     (g = 7):       rows 0, 1 times e^{i phi}, row 2 times e^{-2 i phi}
+// with c = cos(theta/2), s = sin(theta/2), phi = theta/(2 sqrt 3).  Rows are
+// picked with selects, so threads with different generators stay converged,
+// and every link's third row is formed, so no branch delays the decision.
+__device__ __forceinline__ void hit_any_f(m3f &u, const m3f &a, double rr[3], double &old_tr, int g,
+                                          float theta, double beta3, double unif,
+                                          unsigned &accepted) {
+    const bool diag = g == 7;
+    float s1, c1;
+    cos_sin_f(diag ? theta * 0.28867513459481287f : 0.5f * theta, c1, s1);
+    // e^{-2 i phi} of lambda_8 from the same pair by the double-angle
+    // identities (one cos/sin pair per hit instead of two)
+    const float c2 = fmaf(c1, c1, -s1 * s1), s2 = -2.f * s1 * c1;
+    const int kind = diag ? 3 : ((g == 2) ? 2 : ((g == 1 || g == 4 || g == 6) ? 1 : 0));
+    const cf zero = cfm(0.f, 0.f);
+    const cf r00 = (kind == 0 || kind == 1) ? cfm(c1, 0.f) : cfm(c1, s1);
+    const cf r11 = (kind == 0 || kind == 1) ? cfm(c1, 0.f) : cfm(c1, kind == 2 ? -s1 : s1);
+    const cf r01 = kind == 0 ? cfm(0.f, s1) : (kind == 1 ? cfm(s1, 0.f) : zero);
+    const cf r10 = kind == 0 ? cfm(0.f, s1) : (kind == 1 ? cfm(-s1, 0.f) : zero);
+    const cf ek = diag ? cfm(c2, s2) : cfm(1.f, 0.f);
+    const int i = (g <= 4 || diag) ? 0 : 1;
+    const int j = (g <= 2 || diag) ? 1 : 2;
+    const int k = 3 - i - j;
+    cf ri[3], rj[3], rk[3], ni[3], nj[3], nk[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        ri[c] = csel(i == 0, u.e[0][c], u.e[1][c]);
+        rj[c] = csel(j == 1, u.e[1][c], u.e[2][c]);
+        rk[c] = csel(k == 2, u.e[2][c], csel(k == 1, u.e[1][c], u.e[0][c]));
+        ni[c] = cfadd(cfmul(r00, ri[c]), cfmul(r01, rj[c]));
+        nj[c] = cfadd(cfmul(r10, ri[c]), cfmul(r11, rj[c]));
+        nk[c] = cfmul(ek, rk[c]);
+    }
+    cf ci[3], cj[3], ck[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        ci[r] = csel(i == 0, a.e[r][0], a.e[r][1]);
+        cj[r] = csel(j == 1, a.e[r][1], a.e[r][2]);
+        ck[r] = csel(k == 2, a.e[r][2], csel(k == 1, a.e[r][1], a.e[r][0]));
+    }
+    const double qi = retr_col64(ni, ci[0], ci[1], ci[2]);
+    const double qj = retr_col64(nj, cj[0], cj[1], cj[2]);
+    const double qk = retr_col64(nk, ck[0], ck[1], ck[2]);
+    const double q0 = i == 0 ? qi : qk;
+    const double q1 = i == 1 ? qi : (j == 1 ? qj : qk);
+    const double q2 = j == 2 ? qj : qk;
+    const double new_tr = (q0 + q1) + q2;
+    const bool acc = accept64(old_tr, new_tr, beta3, unif);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const cf n0 = csel(i == 0, ni[c], nk[c]);
+        const cf n1 = csel(i == 1, ni[c], csel(j == 1, nj[c], nk[c]));
+        const cf n2 = csel(j == 2, nj[c], nk[c]);
+        u.e[0][c] = csel(acc, n0, u.e[0][c]);
+        u.e[1][c] = csel(acc, n1, u.e[1][c]);
+        u.e[2][c] = csel(acc, n2, u.e[2][c]);
+    }
+    rr[0] = acc ? q0 : rr[0];
+    rr[1] = acc ? q1 : rr[1];
+    rr[2] = acc ? q2 : rr[2];
+    old_tr = acc ? new_tr : old_tr;
+    accepted += acc ? 1u : 0u;
+}
+
+// One learned visit with everything in registers (visit_drawn_f's bits).
+__device__ __forceinline__ unsigned visit_learned_reg(m3f &u, const m3f &a, double beta3, const DrawLearned &draw,
+                                                      float scale, uint64_t key) {
+    double rr[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) rr[i] = retr_col64(u.e[i], a.e[0][i], a.e[1][i], a.e[2][i]);
+    double old_tr = (rr[0] + rr[1]) + rr[2];
+    unsigned accepted = 0;
+#pragma unroll 1
+    for (int h = 0; h < 8; ++h) {
+        const uint64_t w = splitmix_at(key, (uint64_t)(2 * h));
+        hit_any_f(u, a, rr, old_tr, draw(w), (float)grid_angle(w, (double)scale), beta3,
+                  unit_from(splitmix_at(key, (uint64_t)(2 * h + 1))), accepted);
+    }
+    return accepted;
+}
+
 // Uniformly drawn generators: bits 52..54.
 struct DrawUniform {
     __device__ __forceinline__ int operator()(uint64_t w) const { return (int)((w >> 52) & 7); }
