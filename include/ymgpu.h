@@ -68,7 +68,9 @@ typedef struct {
     const double *beta;           /* n_chains couplings (may differ) */
     const uint64_t *chain_seed;   /* n_chains stream seeds */
     int32_t lift_reference_caps;  /* 0: reject lattices above the reference's
-                                     link caps (2^18 SU(3), 2^20 SU(2)) */
+                                     link caps (2^18 SU(3), 2^20 SU(2)); else
+                                     below 2^31 sites per chain
+                                     (YM_ERR_ALLOCATION_FAILED from there on) */
     int32_t device;               /* CUDA device ordinal */
 } ym_ensemble_desc;
 

@@ -433,6 +433,9 @@ int32_t ym_ensemble_create(const ym_ensemble_desc *desc, ym_ensemble **out) {
         const int64_t links = sites * 4;
         const int64_t cap = e->group == YM_GROUP_SU3 ? kMaxSu3Links : kMaxSu2Links;
         if (!desc->lift_reference_caps && links > cap) { delete e; return YM_ERR_LATTICE_TOO_LARGE; }
+        // the kernels' site indices have 32 bits; no device holds such a
+        // lattice (its host-layout staging alone takes 1.2 TB)
+        if (sites > INT32_MAX) { delete e; return YM_ERR_ALLOCATION_FAILED; }
         c.eo = (n[3] % 2 == 0) ? 1 : 0;
         c.volume = sites;
         c.half = c.eo ? sites / 2 : sites;

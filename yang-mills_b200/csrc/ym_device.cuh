@@ -396,7 +396,7 @@ __device__ __forceinline__ Nb step_any(const ChainInfo &c, const int32_t *x, int
 
 // A link's site within its chain and the steps to its neighbours, in
 // lexicographic positions.  Sweeps need even extents, so every step changes
-// the parity; 32 bits hold any site (a lattice of 2^31 sites takes 1.2 TB).
+// the parity; 32 bits hold any site (ym_ensemble_create refuses 2^31).
 struct Site {
     int32_t lex, half;
     int32_t fwd[4], bwd[4];
