@@ -206,7 +206,8 @@ __device__ __forceinline__ void proposal_from(const float y[16], float cum[7], f
 // ReTr(R_g(theta) M) and d/dtheta (closed forms of the header's definition)
 // from the angle's sines and cosines: (s, c) of theta/2 for the SU(2)
 // subgroups; for lambda8 (s, c) of k theta and (s2, c2) of 2 k theta, k =
-// 1/(2 sqrt 3).
+// 1/(2 sqrt 3).  Products and sums are fused as written here, not by the
+// compiler, so that they round alike for every caller and both signs.
 constexpr float kLambda8 = 0.28867513459481287f;
 
 __device__ __forceinline__ void retr_rotated(int g, const float *m, float tr, float s, float c, float s2, float cs2,
@@ -221,13 +222,14 @@ __device__ __forceinline__ void retr_rotated(int g, const float *m, float tr, fl
         if (kind == 0) c2 = -(m[2 * (3 * i + j) + 1] + m[2 * (3 * j + i) + 1]);
         else if (kind == 1) c2 = m[2 * (3 * j + i)] - m[2 * (3 * i + j)];
         else c2 = m[2 * (4 * j) + 1] - m[2 * (4 * i) + 1];
-        f = (tr - c1) + c1 * c + c2 * s;
-        df = 0.5f * (-c1 * s + c2 * c);
+        f = fmaf(c2, s, fmaf(c1, c, tr - c1));
+        df = 0.5f * fmaf(c2, c, -__fmul_rn(c1, s));
     } else {
         const float k = kLambda8;
         const float mr = m[0] + m[8], mi = m[1] + m[9];
-        f = c * mr - s * mi + cs2 * m[16] + s2 * m[17];
-        df = k * (-s * mr - c * mi) + 2.f * k * (-s2 * m[16] + cs2 * m[17]);
+        f = fmaf(s2, m[17], fmaf(cs2, m[16], fmaf(c, mr, -__fmul_rn(s, mi))));
+        const float d1 = fmaf(-s, mr, -__fmul_rn(c, mi)), d2 = fmaf(cs2, m[17], -__fmul_rn(s2, m[16]));
+        df = fmaf(k, d1, __fmul_rn(2.f * k, d2));
     }
 }
 
@@ -275,16 +277,14 @@ __device__ __forceinline__ float objective_row(const float y[16], const float *m
 #pragma unroll
             for (int sg = -1; sg <= 1; sg += 2) {
                 const float dth = sg * gk;
-                float f, df, s1 = sg * sn[q], c1 = cs[q], s2 = sg * sn2[q], c2 = cs2[q];
-                // the compiler must not share products between the two signs:
-                // which product it then fuses would change the rounding
-                asm volatile("" : "+f"(s1), "+f"(c1), "+f"(s2), "+f"(c2));
-                retr_rotated(a, m, tr, s1, c1, s2, c2, f, df);
+                float f, df;
+                retr_rotated(a, m, tr, sg * sn[q], cs[q], sg * sn2[q], cs2[q], f, df);
                 const float ds = b3 * (tr - f), dds = -b3 * df;
                 const float al = ds > 0.f ? expf(-ds) : 1.f;
                 const float dal = ds > 0.f ? -al * dds : 0.f;
-                j += al * ds * ds;
-                dj += (dal * ds * ds + 2.f * al * ds * dds) * dth;
+                const float lin = __fmul_rn(2.f * al, ds), quad = __fmul_rn(__fmul_rn(dal, ds), ds);
+                j = fmaf(__fmul_rn(al, ds), ds, j);
+                dj = fmaf(fmaf(lin, dds, quad), dth, dj);
             }
         }
         J[a] = j / (2.f * K);
