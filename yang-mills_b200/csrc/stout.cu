@@ -25,10 +25,6 @@ namespace {
 
 constexpr int T = kSiteThreads;
 
-#ifndef YM_STOUT_BLOCKS
-#define YM_STOUT_BLOCKS 4
-#endif
-
 // A Hermitian 3x3 matrix: its real diagonal and the upper triangle.
 struct herm3 {
     double d[3];
@@ -192,7 +188,7 @@ __device__ __forceinline__ void add_product_adj(m3 &acc, const m3 &p, const m3 &
 // on 24^3 x 48: the three directions of 32 sites in one block (so that their
 // loads might meet in L1) 385 us, factors staged by cp.async 353 (three
 // blocks 331, but 1 % slower on the uneven batch).
-__global__ void __launch_bounds__(T, YM_STOUT_BLOCKS)
+__global__ void __launch_bounds__(T, 4)
 k_stout_level(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles,
               const double2 *__restrict__ in, double2 *__restrict__ out, double rho,
               unsigned *__restrict__ err, int reverse) {

@@ -17,19 +17,7 @@ constexpr unsigned kErrProjection = 4u;
 constexpr unsigned kErrGroup = 8u;
 constexpr unsigned kErrNonFiniteStaple = 16u;
 
-__device__ __forceinline__ double cabs(cplx z) { return hypot(z.re, z.im); }
-
 __device__ __forceinline__ double norm2(cplx z) { return z.re * z.re + z.im * z.im; }
-
-// max |m_ij|, compared through squared magnitudes (one sqrt at the end)
-__device__ __forceinline__ double max_abs(const m3 &m) {
-    double r = 0.0;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) r = fmax(r, norm2(m.e[i][j]));
-    return sqrt(r);
-}
 
 __device__ __forceinline__ bool finite3(const m3 &m) {
 #pragma unroll
@@ -38,24 +26,6 @@ __device__ __forceinline__ bool finite3(const m3 &m) {
         for (int j = 0; j < 3; ++j)
             if (!isfinite(m.e[i][j].re) || !isfinite(m.e[i][j].im)) return false;
     return true;
-}
-
-__device__ __forceinline__ m3 sub3(const m3 &a, const m3 &b) {
-    m3 o;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) o.e[i][j] = csub(a.e[i][j], b.e[i][j]);
-    return o;
-}
-
-__device__ __forceinline__ m3 scale_c(const m3 &a, cplx f) {
-    m3 o;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) o.e[i][j] = cmul(a.e[i][j], f);
-    return o;
 }
 
 __device__ __forceinline__ m3 scale_r(const m3 &a, double f) {

@@ -27,10 +27,6 @@ namespace {
 constexpr int T = kSweepThreads;
 using namespace f32;
 
-#ifndef YM_F32_MIN_BLOCKS
-#define YM_F32_MIN_BLOCKS 4
-#endif
-
 // Shared memory of a block: two sets of three staged factors.
 constexpr size_t kRingF = (size_t)36 * T * sizeof(float2);
 
@@ -46,7 +42,7 @@ constexpr size_t kRingF = (size_t)36 * T * sizeof(float2);
 // drawn 1093, 4 x 16^4 drawn 315 us: the static split of 1.7 tiles per block
 // leaves SMs idle), as were three or five blocks per SM.
 template <bool DRAWN>
-__global__ void __launch_bounds__(T, YM_F32_MIN_BLOCKS)
+__global__ void __launch_bounds__(T, 4)
 k_f32_metropolis(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles,
                  const __grid_constant__ ChainInfo one, float2 *__restrict__ links, int parity, int mu, double angle,
                  const uint64_t *__restrict__ sweep_ptr, unsigned long long *__restrict__ accepts,

@@ -81,21 +81,6 @@ __device__ __forceinline__ m3 adj_mul(const m3 &a, const m3 &b) {
     return o;
 }
 
-// a^dagger * b^dagger
-__device__ __forceinline__ m3 adj_mul_adj(const m3 &a, const m3 &b) {
-    m3 o;
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            cplx v = cmul(cconj(a.e[0][r]), cconj(b.e[c][0]));
-            v = cadd(v, cmul(cconj(a.e[1][r]), cconj(b.e[c][1])));
-            v = cadd(v, cmul(cconj(a.e[2][r]), cconj(b.e[c][2])));
-            o.e[r][c] = v;
-        }
-    return o;
-}
-
 __device__ __forceinline__ m3 adj(const m3 &a) {
     m3 o;
 #pragma unroll
@@ -103,13 +88,6 @@ __device__ __forceinline__ m3 adj(const m3 &a) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) o.e[r][c] = cconj(a.e[c][r]);
     return o;
-}
-
-__device__ __forceinline__ void add_into(m3 &acc, const m3 &b) {
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) acc.e[r][c] = cadd(acc.e[r][c], b.e[r][c]);
 }
 
 __device__ __forceinline__ m3 identity3() {
@@ -133,15 +111,6 @@ __device__ __forceinline__ double retrace_mul_adj(const m3 &p, const m3 &b) {
         d[r] = v.re;
     }
     return (d[0] + d[1]) + d[2];
-}
-
-// Row contribution to Re Tr(X A): (t_i0 + t_i1) + t_i2,
-// t_ik = X_ik.re*A_ki.re - X_ik.im*A_ki.im.
-__device__ __forceinline__ double retr_row(const cplx *xrow, const m3 &a, int i) {
-    double t0 = xrow[0].re * a.e[0][i].re - xrow[0].im * a.e[0][i].im;
-    double t1 = xrow[1].re * a.e[1][i].re - xrow[1].im * a.e[1][i].im;
-    double t2 = xrow[2].re * a.e[2][i].re - xrow[2].im * a.e[2][i].im;
-    return (t0 + t1) + t2;
 }
 
 // ---------------------------------------------------------------- fused forms
