@@ -816,7 +816,7 @@ static void drop_run_graph(ym_ensemble *e) {
 // The run_chain cadence's plaquette after a sweep.  For binary64 handles
 // with ordered hits, one chain per sub-sweep CTA and chains too large for
 // the chain-resident kernel, the sweep's last three sub-sweeps (parity 1,
-// directions 1, 2, 3) also sum, per CTA, (1/3) Re Tr(U' A_p) of their links,
+// directions 1, 2, 3) also sum, per warp, (1/3) Re Tr(U' A_p) of their links,
 // A_p the staple terms of the lower directions: all those links are final
 // then, and each plaquette of plane (nu, mu) holds exactly one odd-site
 // mu-link, so the three sums are the six planes' plaquettes and no

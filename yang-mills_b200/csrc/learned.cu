@@ -320,6 +320,9 @@ __device__ __forceinline__ void teardown_block(uint32_t tmem, uint32_t ncols) {
 
 constexpr size_t kRecordBytes = 36 * kRows * sizeof(float2);   // two sets of three staged factors
 
+// The records of half a lattice's links.  The staple's factors are staged two
+// terms ahead and rows written in 16- and 8-byte pieces: 17.2 -> 11.3 us at
+// 16^4.
 __global__ void __launch_bounds__(kRows)
 k_lp_records(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles,
              const float2 *__restrict__ links, int parity, int mu, float *__restrict__ feat,
@@ -402,12 +405,10 @@ k_lp_forward(const float *__restrict__ feat, int64_t n, const uint4 *__restrict_
     teardown_block(tmem, 64);
 }
 
-// (records: the staple's factors staged two terms ahead and rows written in
-// 16- and 8-byte pieces, 17.2 -> 11.3 us at 16^4; this kernel: the nodes'
-// sines and cosines computed once for the seven subgroup generators and both
-// signs instead of 64 times, 43.6 -> 31.3 us)
 // One tile of the objective gradient.  partial[tile][p] receives the tile's
 // sum over rows of d(-E)/d param p; partial[tile][YM_LP_PARAMS] the sum of E.
+// The nodes' sines and cosines are computed once for the seven subgroup
+// generators and both signs, not 64 times: 43.6 -> 31.3 us at 16^4.
 __global__ void __launch_bounds__(kRows)
 k_lp_grad(const float *__restrict__ feat, const float *__restrict__ mrec,
           const float *__restrict__ b3rec, int64_t n, const uint4 *__restrict__ image,

@@ -7,7 +7,9 @@
 // t_k = (t_{k-1} * h) * fl(1/k) (h the scaled coefficient entry) and the
 // zero entries only add exact zeros.  Evaluating that recurrence reproduces
 // the reference rotation's non-zero entries bit for bit at a fraction of the
-// dense cost.  Include only from translation units built with -fmad=false.
+// dense cost.  The rotations belong to translation units built with
+// -fmad=false; the accept decision (neg_log_unit, accept_log, next_word) has
+// no product that could be fused and serves the others too.
 #pragma once
 
 #include "ym_device.cuh"

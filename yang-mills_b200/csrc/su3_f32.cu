@@ -8,8 +8,9 @@
 //
 // Arithmetic of the sub-sweep (fast mode; fused multiply-adds allowed):
 // the staple sum and the candidate rows are binary32; the action change
-// dS = (beta/3)(ReTr(U A) - ReTr(U' A)) and the accept test
-// u < exp(-max(dS, 0)) are evaluated in binary64 from the stored values.  The
+// dS = (beta/3)(ReTr(U A) - ReTr(U' A)) is evaluated in binary64 from the
+// stored values, and the accept test u < exp(-max(dS, 0)) decided as binary64
+// decides it (accept_log: binary32 away from equality, binary64 near it).  The
 // update rule, stream words and generator order are the FP64 path's.  The
 // plaquette and every conversion to FP64 are binary64 products of the
 // stored values; k_f32_reunitarize restores unitarity in binary64

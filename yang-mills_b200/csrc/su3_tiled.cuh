@@ -230,7 +230,8 @@ struct Row {
     double rr;
 };
 
-// Candidate entries of an SU(2)-subgroup hit on rows x, y (hit_block's).
+// Candidate entries of an SU(2)-subgroup hit on rows x, y: Mat3::mul's values,
+// two rounded products and their sum per entry.
 template <int KIND>
 __device__ __forceinline__ void block_candidate(const Row &x, const Row &y, double c, double s, cplx n0[3],
                                                 cplx n1[3]) {
@@ -480,8 +481,9 @@ __device__ __forceinline__ unsigned visit_drawn(const U &u, const A &a, double b
 // while term k multiplies.  Two
 // 128-thread CTAs per SM fit (registers and 108 KB of staging each); after
 // the staple the accumulator is written once to the second set's memory for
-// the hits.  The products and their order are staple_pipelined's, so A has
-// the same bits.
+// the hits.  Terms run over the directions nu other than mu in ascending
+// order, forward before backward, each product as fma chains (pair_product,
+// add_third): the chain-resident kernel's order, so A has the same bits there.
 //
 // What bounds it: latency, at two warps per scheduler.  Two things cut it.
 // (1) The CTAs are persistent, and the next item's first term loads into the
@@ -740,9 +742,9 @@ void metro_launch_ring(ym_ensemble *e, int parity, int mu, double angle, int rev
         reverse, nullptr);
 }
 
-// The last sub-sweep of a sweep (parity 1, direction 3, ordered hits) with
-// its plaquette share (MEASURE): the handle's layout must put one chain in
-// each CTA (128-site items).
+// One of a sweep's last three sub-sweeps (parity 1, mu = 1, 2 or 3, ordered
+// hits) with its plaquette shares (MEASURE): the handle's layout must put one
+// chain in each CTA (128-site items).
 template <int K>
 void metro_launch_measure(ym_ensemble *e, int mu, double angle, double *tr_partial) {
     const SweepLayout &L = e->layouts[e->sweep_layout];
@@ -797,8 +799,9 @@ cudaError_t tiled_launch(ym_ensemble *e, int parity, int mu, double angle, int u
 }
 
 // tiled_launch(e, 1, mu, angle, ordered hits), mu = 1, 2 or 3, that also
-// writes each CTA's plaquette share of the planes (nu, mu), nu < mu, to
-// tr_partial[cta] (the handle's layout must hold one chain per CTA).
+// writes each warp's plaquette share of the planes (nu, mu), nu < mu, to
+// tr_partial[cta * kSweepWarps + warp] (the handle's layout must hold one
+// chain per CTA).
 cudaError_t tiled_launch_measure(ym_ensemble *e, int mu, double angle, double *tr_partial) {
     if (cudaError_t err = configure_kernels()) return err;
     if (angle <= kShortRotation) metro_launch_measure<11>(e, mu, angle, tr_partial);

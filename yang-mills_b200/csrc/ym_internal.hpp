@@ -222,13 +222,14 @@ cudaError_t launch_su3_metropolis(ym_ensemble *e, int parity, int mu, double ang
 // launch_su3_metropolis dispatches to it when e->fast_sweeps is set.
 cudaError_t launch_su3_metropolis_fast(ym_ensemble *e, int parity, int mu, double angle, int uniform);
 // Sub-sweep (parity 1, mu), mu = 1, 2 or 3, with ordered hits, also writing
-// each CTA's share of the plaquettes in planes (nu, mu), nu < mu, to
-// tr_partial[cta]; the handle's layout must hold one chain per CTA.
+// each warp's share of the plaquettes in planes (nu, mu), nu < mu, to
+// tr_partial[cta * kSweepWarps + warp]; the handle's layout must hold one
+// chain per CTA.
 cudaError_t launch_su3_metropolis_measure(ym_ensemble *e, int mu, double angle, double *tr_partial);
 cudaError_t launch_su3_metropolis_measure_fast(ym_ensemble *e, int mu, double angle, double *tr_partial);
 // After a sweep whose last three sub-sweeps measured into tr_partial
-// (three arrays of the layout's CTA count): each chain's average plaquette
-// into d_result.  (series: see launch_chain_reduce.)
+// (three arrays of kSweepWarps times the layout's CTA count): each chain's
+// average plaquette into d_result.  (series: see launch_chain_reduce.)
 cudaError_t launch_su3_plaquette_from_sweep(ym_ensemble *e, const double *tr_partial, double *series = nullptr);
 // The deferred sweeps onto the device's sweep counter.
 cudaError_t launch_counted_sweeps(ym_ensemble *e);
