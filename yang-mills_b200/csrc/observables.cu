@@ -299,8 +299,9 @@ __device__ __forceinline__ void plane_loops(const double2 *links, const ChainInf
 // 1x1 spatial orientations (0,1),(0,2),(1,2) and the six 2x1 orientations
 // (0,1),(0,2),(1,0),(1,2),(2,0),(2,1) (glueball_operators.rs:24-26), summed
 // in that order.
-// (250 registers, two blocks per SM: 0.52 ms at 32^4; capped at three
-// blocks, 168 registers with spills, 0.66 ms)
+// (250 registers, two blocks per SM: 0.44 ms at 32^4 with its reduction;
+// capped at three blocks, 168 registers with spills, 0.66 ms when this form
+// took 0.52)
 __global__ void __launch_bounds__(T)
 k_operator_sites(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles,
                  const double2 *__restrict__ links, double2 *__restrict__ site_vals) {
