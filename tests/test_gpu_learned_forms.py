@@ -1,7 +1,7 @@
 """Learned sub-sweeps run their hits in registers on handles of at most two
-tiles per SM and on rows in shared memory on larger ones: a chain's links and
-accept counts are the same in both, at exactly that size, one tile past it
-and far past it, with ragged last tiles."""
+tiles per SM, or of more than four and at most five, and on rows in shared
+memory otherwise: a chain's links and accept counts are the same in both, at
+those sizes, just past them and far past them, with ragged last tiles."""
 import numpy as np
 import pytest
 
@@ -23,10 +23,11 @@ def _sweep(extents, copies, n=2):
 @pytest.mark.parametrize("extents", [[4, 4, 4, 4], [4, 4, 4, 6], [6, 6, 6, 10]])
 def test_a_chain_is_the_same_in_both_forms(extents):
     import torch
-    limit = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
     tiles = -(-(int(np.prod(extents)) // 2) // 128)
     links, accepted = _sweep(extents, 1)
-    for copies in (limit // tiles, limit // tiles + 1, 4 * limit // tiles):
-        got, count = _sweep(extents, copies)
-        assert np.array_equal(got, links)
-        assert count == accepted
+    for full in (2, 4, 5, 8):
+        for copies in (full * sms // tiles, full * sms // tiles + 1):
+            got, count = _sweep(extents, copies)
+            assert np.array_equal(got, links)
+            assert count == accepted

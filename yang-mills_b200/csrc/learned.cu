@@ -642,14 +642,22 @@ __global__ void k_lp_adam(const double *__restrict__ groups, int64_t n_groups, i
 // REG: the hits in registers, not on rows in memory.  With at most two tiles
 // per SM a sub-sweep is one or two visits' latency, and the hits' row reads
 // and lambda8's branch lie on it; with more, issue bounds it and the memory
-// form has fewer instructions.  Per sweep, registers against memory: 8^4 155
-// against 162 us, 12^4 157 against 171, 151 tiles 172.7 against 173.2, 256
-// tiles (16^4) 176 against 188, 288 tiles 185 against 189; 411 tiles (18^4)
-// 223 against 206, 4 x 16^4 430 against 413.
-constexpr int kRegTilesPerSm = 2;
+// form has fewer instructions, until a second wave of at most one tile per SM
+// adds a visit's latency to the first wave of four.  Per sweep, registers
+// against memory: 8^4 155 against 162 us, 12^4 157 against 171, 151 tiles
+// 172.7 against 173.2, 256 tiles (16^4) 176 against 188, 288 tiles 185 against
+// 189; 411 tiles (18^4) 223 against 206, 500 tiles 272 against 259; 625 tiles
+// (20^4) 326 against 337, 688 tiles 335 against 342; 756 tiles 366 against
+// 358, 1296 tiles (24^4, a third wave of 112) 553 against 547, 4 x 16^4 430
+// against 413.
+constexpr int kSweepCtas = 4;   // per SM: registers, shared memory and 4 x 64 TMEM columns
+
+static bool hits_in_registers(int64_t tiles, int64_t sms) {
+    return tiles <= 2 * sms || (tiles > kSweepCtas * sms && tiles <= (kSweepCtas + 1) * sms);
+}
 
 template <int MU, bool REG>
-__global__ void __launch_bounds__(kRows, 4)
+__global__ void __launch_bounds__(kRows, kSweepCtas)
 k_lp_sweep(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles, int64_t n_tiles,
            float2 *__restrict__ links, int parity, const uint4 *__restrict__ image,
            const float *__restrict__ params, const uint64_t *__restrict__ sweep_ptr,
@@ -812,9 +820,8 @@ static cudaError_t allow_lp_sweep() {
 template <int MU>
 static cudaError_t lp_sweep_launch(ym_ensemble *e, ym_proposal_model *m, int parity, int sms) {
     const int64_t n = e->n_half_tiles;
-    // four CTAs per SM: registers, shared memory and 4 x 64 TMEM columns
-    const unsigned grid = (unsigned)(n < 4 * sms ? n : 4 * sms);
-    const auto kernel = n <= lp::kRegTilesPerSm * sms ? lp::k_lp_sweep<MU, true> : lp::k_lp_sweep<MU, false>;
+    const unsigned grid = (unsigned)(n < lp::kSweepCtas * sms ? n : lp::kSweepCtas * sms);
+    const auto kernel = lp::hits_in_registers(n, sms) ? lp::k_lp_sweep<MU, true> : lp::k_lp_sweep<MU, false>;
     kernel<<<grid, lp::kRows, lp::FwdLayout::BYTES, e->stream>>>(
         e->d_chains, e->d_half_tiles, n, reinterpret_cast<float2 *>(e->d_links), parity,
         reinterpret_cast<const uint4 *>(m->d_image), m->d_params, sweep_index(e), e->d_accepts, m->d_error);
