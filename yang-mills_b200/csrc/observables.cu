@@ -61,6 +61,7 @@ __device__ __forceinline__ Walker walker_of(const Coord &x) {
 // product only by rounding (<= 1e-12 relative on lattice means).
 // partial[(tile * 6 + plane) * 16 + (R-1)*4 + (T-1)] = tile sum.
 constexpr size_t kWilsonSmem = (size_t)kMaxRT * 9 * T * sizeof(double2);
+constexpr size_t kWilsonColumn = (size_t)16 * T * sizeof(double);
 
 __device__ __forceinline__ void step_walker(const ChainInfo &c, Walker &w, int mu) {
     const Nb n = step(c, w.x, w.lex, w.par, mu, +1);
@@ -89,9 +90,30 @@ __device__ __forceinline__ m3 q_get(const double2 *qs, int t) {
     return q;
 }
 
-template <int MU, int NU>
+// Where a thread's loop values go; the sums have the same bits.  WarpSums: each
+// is summed over its warp as it is made, so threads past the chain's end walk
+// site 0 and count 0.  Column: each waits in the thread's column of shared
+// memory (which takes it from L1), the sixteen are summed side by side at the
+// end, and threads past the end do nothing.
+struct WarpSums {
+    double (*sums)[16];
+    bool live;
+    __device__ __forceinline__ void put(int k, double v) const {
+        if (!live) v = 0.0;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+        if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5][k] = v;
+    }
+};
+
+struct Column {
+    double (*values)[T];
+    __device__ __forceinline__ void put(int k, double v) const { values[k][threadIdx.x] = v; }
+};
+
+template <int MU, int NU, class Sink>
 __device__ __forceinline__ void wilson_site(const double2 *links, const ChainInfo &c, const Walker &w0,
-                                            int rmax, int tmax, double2 *qs, double (*sums)[16], bool live) {
+                                            int rmax, int tmax, double2 *qs, const Sink &sink) {
     {   // D_T, stored as Q_{0,T}
         Walker w = w0;
         m3 d, next = link_of(links, c, w, NU);
@@ -124,15 +146,25 @@ __device__ __forceinline__ void wilson_site(const double2 *links, const ChainInf
             if (t + 1 < tmax) up = link_of(links, c, wp, NU);
             const m3 q = mul_fma(q_get(qs, t), uq);
             q_put(qs, t, q);
-            double v = retrace_mul_adj(p, q) * (1.0 / 3.0);
-            if (!live) v = 0.0;
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-            if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5][r * kMaxRT + t] = v;
+            sink.put(r * kMaxRT + t, retrace_mul_adj(p, q) * (1.0 / 3.0));
         }
     }
 }
 
+template <class Sink>
+__device__ __forceinline__ void wilson_plane(int plane, const double2 *links, const ChainInfo &c, const Walker &w0,
+                                             int rmax, int tmax, double2 *qs, const Sink &sink) {
+    switch (plane) {
+        case 0: wilson_site<0, 1>(links, c, w0, rmax, tmax, qs, sink); break;
+        case 1: wilson_site<0, 2>(links, c, w0, rmax, tmax, qs, sink); break;
+        case 2: wilson_site<0, 3>(links, c, w0, rmax, tmax, qs, sink); break;
+        case 3: wilson_site<1, 2>(links, c, w0, rmax, tmax, qs, sink); break;
+        case 4: wilson_site<1, 3>(links, c, w0, rmax, tmax, qs, sink); break;
+        default: wilson_site<2, 3>(links, c, w0, rmax, tmax, qs, sink); break;
+    }
+}
+
+template <bool COLUMN>
 __global__ void __launch_bounds__(T, 2)
 k_wilson_loops(const ChainInfo *__restrict__ chains, const Tile *__restrict__ tiles,
                const double2 *__restrict__ links, int rmax, int tmax, double *__restrict__ partial) {
@@ -145,14 +177,24 @@ k_wilson_loops(const ChainInfo *__restrict__ chains, const Tile *__restrict__ ti
     if (threadIdx.x < T / 32 * 16) sums[threadIdx.x / 16][threadIdx.x % 16] = 0.0;
     __syncthreads();
     const bool live = s < c.volume;
-    const Walker w0 = walker_of(decode_storage(c, live ? s : 0));
-    switch (plane) {
-        case 0: wilson_site<0, 1>(links, c, w0, rmax, tmax, qs, sums, live); break;
-        case 1: wilson_site<0, 2>(links, c, w0, rmax, tmax, qs, sums, live); break;
-        case 2: wilson_site<0, 3>(links, c, w0, rmax, tmax, qs, sums, live); break;
-        case 3: wilson_site<1, 2>(links, c, w0, rmax, tmax, qs, sums, live); break;
-        case 4: wilson_site<1, 3>(links, c, w0, rmax, tmax, qs, sums, live); break;
-        default: wilson_site<2, 3>(links, c, w0, rmax, tmax, qs, sums, live); break;
+    if (COLUMN) {
+        double (*values)[T] = reinterpret_cast<double (*)[T]>(qs + kWilsonSmem / sizeof(double2));
+#pragma unroll
+        for (int k = 0; k < 16; ++k) values[k][threadIdx.x] = 0.0;
+        if (live) wilson_plane(plane, links, c, walker_of(decode_storage(c, s)), rmax, tmax, qs, Column{values});
+        __syncwarp();
+        double v[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = values[k][threadIdx.x];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+            for (int k = 0; k < 16; ++k) v[k] += __shfl_down_sync(0xffffffffu, v[k], off);
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+            if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5][k] = v[k];
+    } else {
+        wilson_plane(plane, links, c, walker_of(decode_storage(c, live ? s : 0)), rmax, tmax, qs, WarpSums{sums, live});
     }
     __syncthreads();
     if (threadIdx.x < 16) {
@@ -376,14 +418,25 @@ cudaError_t launch_wilson_loops(ym_ensemble *e, int rmax, int tmax, double *d_pa
     int dev = 0;
     cudaGetDevice(&dev);
     if (configured_device != dev) {
-        const cudaError_t err = cudaFuncSetAttribute(k_wilson_loops, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)kWilsonSmem);
+        cudaError_t err = cudaFuncSetAttribute(k_wilson_loops<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)kWilsonSmem);
+        if (err == cudaSuccess)
+            err = cudaFuncSetAttribute(k_wilson_loops<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(kWilsonSmem + kWilsonColumn));
         if (err != cudaSuccess) return err;
         configured_device = dev;
     }
     const dim3 g((unsigned)e->n_site_tiles, 6);
-    k_wilson_loops<<<g, T, kWilsonSmem, e->stream>>>(e->d_chains, e->d_site_tiles, e->d_links, rmax, tmax,
-                                                      d_partial);
+    // Columns where more than an eighth of the threads are past their chain's
+    // end (4 x 4 loops, warp sums against columns, per call: 3^4 41 against 37
+    // us, 3^3 x 5 43 against 38, 64 x 2^4 74 against 70; full tiles: 4^4 38
+    // against 41, 8 x 4^4 42 against 47, 18^4 371 against 382).
+    if (8 * (e->total_links / 4) < 7 * e->n_site_tiles * T)
+        k_wilson_loops<true><<<g, T, kWilsonSmem + kWilsonColumn, e->stream>>>(e->d_chains, e->d_site_tiles, e->d_links,
+                                                                              rmax, tmax, d_partial);
+    else
+        k_wilson_loops<false><<<g, T, kWilsonSmem, e->stream>>>(e->d_chains, e->d_site_tiles, e->d_links, rmax, tmax,
+                                                                d_partial);
     k_tile_mean<<<dim3((unsigned)e->n_chains, 96), 256, 0, e->stream>>>(d_partial, e->d_site_tile_first,
                                                                        e->d_chains, 96, -1, d_out);
     return cudaGetLastError();
